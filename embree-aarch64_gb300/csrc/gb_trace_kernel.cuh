@@ -6,8 +6,9 @@
 // (kernels/bvh/bvh_intersector1.cpp:30-195, bvh_intersector_hybrid.cpp:36-375)
 // with persistent CTAs: warps refill idle lanes with rays fetched by one
 // atomic, every lane walks the 8-wide quantised BVH with a short stack of node
-// groups (child base + hit bits) and postponed triangle groups, visiting
-// children in the order given by the ray's direction octant.
+// groups (child base + hit bits), visiting children in the order given by the
+// ray's direction octant, and the triangles of the leaves that a warp's rays
+// reach are tested in batches over all its lanes.
 //
 // Arithmetic that decides hits is the reference's, bit for bit:
 //   Moeller-Trumbore  kernels/geometry/triangle_intersector_moeller.h:62-104
@@ -161,12 +162,13 @@ constexpr float kSlabFloor = 0x1p-144f;      // 2^-144
 // |1/d| near 1e18) the products are NaN and fminf/fmaxf drop that plane, so
 // the box only grows.  Returns the node group of hit internal children (bit
 // 31 - j set when slot j ^ oct was hit, so the next child to visit is the
-// leading one; imask in bits 0..7) and the triangle group of hit leaves (up to
-// 32 triangle bits).  perm: the row of the ray's octant in the slot
-// permutation table (perm[m] has bit 7 - j set when m has bit j ^ oct).
+// leading one; imask in bits 0..7), the slots of the hit leaves, and the node's
+// triangle base and meta bytes, which say where those leaves' triangles are.
+// perm: the row of the ray's octant in the slot permutation table (perm[m] has
+// bit 7 - j set when m has bit j ^ oct).
 __device__ __forceinline__ void intersect_node(const WideNode* __restrict__ np, const TRay& r, const float tfar,
-                                               uint32_t& g_base, uint32_t& g_bits, uint32_t& t_base,
-                                               uint32_t& t_bits, const uint8_t* __restrict__ perm) {
+                                               uint32_t& g_base, uint32_t& g_bits, uint32_t& t_base, uint32_t& leaf,
+                                               uint2& meta, const uint8_t* __restrict__ perm, const uint32_t row) {
   const uint4* q = reinterpret_cast<const uint4*>(np);
   const uint4 n0 = __ldg(q + 0);
   const uint4 n1 = __ldg(q + 1);
@@ -235,19 +237,17 @@ __device__ __forceinline__ void intersect_node(const WideNode* __restrict__ np, 
   // internal children: bit 31 - j of the group is slot j ^ oct (near to far),
   // one lookup in the octant's row of the permutation table
   const uint32_t inner = perm[hit8 & imask];
-  // leaves that were hit: their triangle bits (count, offset in the meta byte)
-  uint32_t leaf = hit8 & ~imask & 0xFFu, tb = 0;
-  const uint64_t meta = (uint64_t)n1.z | ((uint64_t)n1.w << 32);
-  while (leaf) {
-    const int s = __ffs(leaf) - 1;
-    leaf &= leaf - 1u;
-    const uint32_t m = (uint32_t)(meta >> (8 * s)) & 0xFFu;
-    if (m & 0x80u) tb |= ((2u << ((m >> 5) & 3u)) - 1u) << (m & 31u);
-  }
+  leaf = hit8 & ~imask & 0xFFu;
+  meta = make_uint2(n1.z, n1.w);
   g_base = n1.x;
-  g_bits = (inner << 24) | imask;
+  g_bits = (inner << 24) | imask | row;
   t_base = n1.y;
-  t_bits = tb;
+}
+
+// Meta byte of slot s (0..7): triangle offset in bits 0..4, triangle count - 1
+// in bits 5..6, bit 7 clear for an empty slot.
+__device__ __forceinline__ uint32_t meta_of(const uint2 meta, const uint32_t s) {
+  return __byte_perm(meta.x, meta.y, s) & 0xFFu;
 }
 
 struct Ctx {
@@ -259,12 +259,16 @@ struct Ctx {
   uint32_t num_tris;
 };
 
-// Triangle work waits (its group is pushed) while fewer than this percentage of
-// the warp's active lanes have some.  0 disables postponing: with the default
-// leaves (1 triangle for volumetric scenes, 2 for flat ones) it measured 1-2 %
-// faster than 10 % (the best with 2-triangle leaves everywhere), and 20 % was
-// slower still.
-constexpr int kPostponePct = 0;
+// Batched queries look up each ray's batch when they fetch it, and their scenes
+// are small (8 node visits a ray), so fetching weighs more: a warp waits for this
+// many times the idle lanes of the launch shape.  128 scenes, 14.6M rays: 2.08 ms
+// with a factor of 1, 1.95 with 2, 1.93 with 3, 2.01 with 4.
+constexpr int kBatchedRefill = 3;
+
+// Leaves wait for their triangle tests in a ring per warp (k_trace below): up
+// to 31 waiting + 32 new.
+constexpr int kQueue = 64;
+
 constexpr uint32_t kTriGroup = 0x80000000u;  // stack entry flag: triangle group
 
 template <bool ALIGNED>
@@ -288,9 +292,29 @@ __device__ __forceinline__ void load_ray(const char* p, TRay& r, float& tfar) {
 // Persistent traversal.  Every lane owns one ray at a time; a warp refills
 // its idle lanes with one atomic once SH::kRefillIdle of them are idle.  Each
 // loop iteration an active lane (1) visits one node of its current group,
-// (2) tests its pending triangles -- unless few lanes of the warp have
-// triangle work, in which case the group is pushed and tested later -- and
-// (3) pops the stack when its group is exhausted.
+// (2) queues the triangles of the leaves it hit, and (3) pops the stack when
+// its group is exhausted.
+//
+// Triangle tests are not done by the lane that found the leaf: a node visit
+// yields a triangle on only a few lanes of a warp (4 tests per 37 node visits
+// on an incoherent soup), so testing them in place ran the test with 2-3 of 32
+// lanes.  Instead the warp's lanes append (triangle, owner lane) to a ring in
+// shared memory, and a batch of up to 32 entries is tested by all lanes at
+// once, each reading its entry's ray from the owner lane by shuffles.  A ray's
+// entries are tested in the order in which it found them, and two hits of one
+// ray in a batch are committed in that order, the later one tested again
+// against the lowered tfar, so the accepted hit is the one that testing in
+// place accepts, ties included.  Between finding a triangle and its batch a ray
+// visits nodes with an older, larger tfar: 1.5 % more visits on the soup, none
+// fewer.  A lane whose traversal is over waits for its last entry's batch before
+// it takes another ray.  The finished rays' results are written when the warp
+// refills (several lanes at a time), from the per-lane result words in shared
+// memory.  The ray's octant travels in the node group (bits 8..10), its direction
+// and tnear in shared memory: 56 registers hold the rest without spills (16 bytes
+// of spills cost 10 % on the soup).
+// Measured on a GB300 (whole calls, in place -> batched): 16M closest-hit rays on
+// the 4M soup 12.02 -> 11.54 ms, 16M shadow rays 7.73 -> 7.26 ms, 1M primary rays
+// on the 131k heightfield 161 -> 153 us, 1M rays in a robust scene 253 -> 242 us.
 //
 // SEEDED: the ray's stack starts as [root, seed3, seed2, seed1] with seed0 as
 // the current group, so the proposed subtrees are searched first and the whole
@@ -324,12 +348,13 @@ __device__ __forceinline__ void to_instance(const float* __restrict__ m, TRay& r
 
 // Launch shape (SH, one of kTraceShapes): threads per CTA, the resident CTAs
 // per SM whose register budget the plain variants are compiled for (9 x 128
-// threads: at most 56 registers a thread; 4 % faster than the 8 that 64
-// registers allow on the 4M soup), traversal stack entries kept in shared
-// memory, and the number of idle lanes at which a warp fetches new rays.  The
-// counting, seeded and instance variants keep their registers (under the same
-// bound they would spill 32-150 bytes), and so does the variant with per-ray
-// exclusion lists (EXCL: filter callbacks).
+// threads: at most 56 registers a thread, which they meet without spills),
+// traversal stack entries kept in shared memory, and the number of idle lanes at
+// which a warp fetches new rays.  The variants that would spill 20-50 bytes under
+// that budget (proposals, instances, exclusion lists, closest hit in robust
+// scenes) are compiled for 1,024 resident threads, 64 registers, at most: with
+// the 100 registers they take unbounded, 4 CTAs fit an SM (1M primary rays on 125
+// instances: 1005 us so, 861 us with 64 registers and batched writes).
 template <int THREADS, int CTAS, int SHARED_STACK, int REFILL>
 struct Shape {
   static constexpr int kThreads = THREADS, kCtas = CTAS, kSharedStack = SHARED_STACK, kRefillIdle = REFILL;
@@ -339,36 +364,60 @@ struct Shape {
 using DefaultShape = Shape<kTraceShapes[0].threads, kTraceShapes[0].ctas, kTraceShapes[0].shared_stack,
                            kTraceShapes[0].refill>;
 
+template <bool ANYHIT, bool COUNT, bool ROBUST, bool SEEDED, bool INST, bool EXCL, class SH>
+constexpr int min_ctas() {
+  if (COUNT) return 1;
+  const bool wide = SEEDED || INST || EXCL || (ROBUST && !ANYHIT);
+  return wide && SH::kCtas * SH::kThreads > 1024 ? 1024 / SH::kThreads : SH::kCtas;
+}
+
 template <bool ANYHIT, bool COUNT, bool ALIGNED, bool ROBUST, bool SEEDED, bool INST = false, bool EXCL = false,
           class SH = DefaultShape>
-__global__ void __launch_bounds__(SH::kThreads, (COUNT || SEEDED || INST || EXCL) ? 1 : SH::kCtas)
+__global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, SEEDED, INST, EXCL, SH>())
     k_trace(TraceParams P) {
   constexpr int kSharedStack = SH::kSharedStack;
+  constexpr int kWarps = SH::kThreads / 32;
   Ctx c{P.nodes, P.tris, P.err, P.max_iters, P.num_nodes, P.num_tris};
   uint32_t cur_inst = kInvalidID, hit_inst = kInvalidID;  // INST: instance being traversed / of the hit
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
   const uint32_t nrays = P.nrays_ptr ? *P.nrays_ptr : P.nrays;
-  // stack of node / triangle groups: the first kSharedStack entries live in
-  // shared memory ([entry][thread]: a warp's accesses are conflict-free), the
-  // deeper ones in local memory.  8 entries measured 2.6 % faster than an
-  // all-local stack (4: 2 % slower, 16: as 8 minus 0.5 %).
+  // stack of node groups (and, in scenes with instances, triangle groups): the
+  // first kSharedStack entries live in shared memory ([entry][thread]: a warp's
+  // accesses are conflict-free), the deeper ones in local memory.  8 entries
+  // measured 2.6 % faster than an all-local stack (4: 2 % slower, 16: as 8
+  // minus 0.5 %).
   uint2 stack[kStackSize];
   int sp = 0;
   __shared__ uint2 s_stack[kSharedStack][SH::kThreads];
+  // per lane: distance, u, v and triangle of its ray's nearest hit so far
+  // (any hit: the distance becomes -inf at a hit); SEEDED: the triangle of the
+  // last hit found in a proposed subtree
+  __shared__ float s_t[SH::kThreads], s_u[ANYHIT ? 1 : SH::kThreads], s_v[ANYHIT ? 1 : SH::kThreads];
+  __shared__ uint32_t s_tri[SH::kThreads], s_seed[SEEDED ? SH::kThreads : 1];
+  // per lane: ray direction and tnear, which only triangle tests read
+  __shared__ float4 s_dir[INST ? 1 : SH::kThreads];
+  // per warp: ring of leaves to test, as (first triangle, owner lane | bits 5..7
+  // of the leaf's meta byte | bit 8: found while seeding)
+  __shared__ uint2 s_queue[INST ? 1 : kWarps][kQueue];
   // slot permutation by octant: s_perm[o][m] has bit 7 - j set when m has bit
   // j ^ o (one shared-memory byte load per node instead of a three-stage swap
   // network: 1.4 % faster; the reversed order lets one count of leading zeros
   // find the next child: 0.5 %)
   __shared__ uint8_t s_perm[8][256];
   for (int i = threadIdx.x; i < 8 * 256; i += SH::kThreads) {
-    const uint32_t o = i >> 8, m = i & 255;
-    uint32_t v = 0;
-    for (int j = 0; j < 8; j++) v |= ((m >> (j ^ o)) & 1u) << (7 - j);
-    s_perm[o][m] = (uint8_t)v;
+    const uint32_t o = i >> 8;
+    uint32_t v = i & 255;  // bit j ^ o of the slot mask moves to bit j: swaps of 1, 2 and 4 bits
+    if (o & 1u) v = ((v & 0x55u) << 1) | ((v >> 1) & 0x55u);
+    if (o & 2u) v = ((v & 0x33u) << 2) | ((v >> 2) & 0x33u);
+    if (o & 4u) v = ((v & 0x0Fu) << 4) | (v >> 4);
+    s_perm[o][i & 255] = (uint8_t)(__brev(v) >> 24);
   }
+  s_tri[threadIdx.x] = kInvalidID;  // no result to write yet
+  __shared__ uint32_t s_batch[kWarps];  // batched queries: a batch that a ray of this warp was in
+  if (lane == 0) s_batch[warp] = 0;
   __syncthreads();
-  const int stk_tid = threadIdx.x;
+  const int stk_tid = threadIdx.x, w0 = threadIdx.x & ~31;
   auto push = [&](uint2 e) {
     if (sp < kSharedStack) s_stack[sp][stk_tid] = e; else stack[sp] = e;
     sp++;
@@ -378,43 +427,205 @@ __global__ void __launch_bounds__(SH::kThreads, (COUNT || SEEDED || INST || EXCL
     return sp < kSharedStack ? s_stack[sp][stk_tid] : stack[sp];
   };
   bool active = false, exhausted = false, seeding = false;
-  char* rec = nullptr;
+  uint32_t rid = 0;
   TRay r;
-  float t_best = 0.f, hu = 0.f, hv = 0.f;
-  uint32_t hit_tri = kInvalidID, seed_tri = kInvalidID, g_base = 0, g_bits = 0, t_base = 0, t_bits = 0, iters = 0;
+  r.org = r.dir = r.rdir = make_float3(0.f, 0.f, 0.f);
+  r.tnear = r.tnear_c = 0.f;
+  r.oct = 0;
+  float t_best = 0.f;
+  uint32_t g_base = 0, g_bits = 0, iters = 0;
   uint32_t ex_lo = 0, ex_hi = 0;  // EXCL: this ray's range of excluded triangles
+  uint32_t qhead = 0, qtail = 0;  // ring positions (uniform in the warp): tested up to qhead, queued up to qtail
   unsigned long long n_nodes = 0, n_tris = 0, n_rays = 0, n_prop = 0;
+
+  // one ray against triangle ti (record a, b, d); true when it is hit in range.
+  // Moeller: (A, B, C, D) = (U, V, T, |den|); Pluecker: (U, V, UVW, t).
+  auto test = [&](const float4 a, const float4 b, const float4 d, const float3 org, const float3 dir,
+                  const float tnear, const float tfar, float& A, float& B, float& C, float& D) -> bool {
+    const float3 p = make_float3(a.x, a.y, a.z), q = make_float3(b.x, b.y, b.z), s = make_float3(d.x, d.y, d.z);
+    return ROBUST ? pluecker(p, q, s, org, dir, tnear, tfar, A, B, C, D)
+                  : moeller(p, q, s, org, dir, tnear, tfar, A, B, C, D);
+  };
+  // records a hit of the ray of the thread `o` of this CTA
+  auto commit = [&](const int o, const uint32_t ti, const float A, const float B, const float C, const float D) {
+    if (ANYHIT) {
+      s_t[o] = -INFINITY;
+      s_tri[o] = ti;
+      return;
+    }
+    if (ROBUST) {
+      // PlueckerHitM::finalize: u,v = U,V * rcp(UVW), 0 when |UVW| < 1e-18
+      const float rcp = fabsf(C) < kMinRcpInput ? 0.0f : __frcp_rn(C);
+      s_t[o] = D;
+      s_u[o] = __fmul_rn(A, rcp);
+      s_v[o] = __fmul_rn(B, rcp);
+    } else {
+      const float rcp = __frcp_rn(D);
+      s_t[o] = __fmul_rn(C, rcp);
+      s_u[o] = __fmul_rn(A, rcp);
+      s_v[o] = __fmul_rn(B, rcp);
+    }
+    s_tri[o] = ti;
+  };
+  // tests the first 32 (or all) entries of the ring; the whole warp calls it.
+  // A lane tests its entry's triangles in order against the entry's own running
+  // distance; the nearest of them is then committed in queue order.
+  auto flush = [&]() {
+    __syncwarp();
+    const uint32_t n = min(qtail - qhead, 32u);
+    uint2 e = make_uint2(0u, (uint32_t)lane);
+    if ((uint32_t)lane < n) e = s_queue[warp][(qhead + lane) & (kQueue - 1)];
+    // the meta byte of an empty slot (bit 7 clear) holds no triangle: overflowed
+    // planes can make one count as hit
+    const bool have = (e.y & 128u) != 0u;
+    const int own = (int)(e.y & 31u);
+    const float3 org = make_float3(__shfl_sync(0xFFFFFFFFu, r.org.x, own), __shfl_sync(0xFFFFFFFFu, r.org.y, own),
+                                   __shfl_sync(0xFFFFFFFFu, r.org.z, own));
+    float tfar = __shfl_sync(0xFFFFFFFFu, t_best, own);
+    uint32_t xl = 0, xh = 0;
+    if (EXCL) {
+      xl = __shfl_sync(0xFFFFFFFFu, ex_lo, own);
+      xh = __shfl_sync(0xFFFFFFFFu, ex_hi, own);
+    }
+    bool hit = false;
+    uint32_t hit_ti = 0;
+    float A = 0.f, B = 0.f, C = 0.f, D = 0.f;
+    if (have) {
+      const float4 dn = s_dir[w0 + own];
+      const uint32_t end = e.x + ((e.y >> 5) & 3u);
+      if (end >= c.num_tris) {
+        atomicOr(c.err, kErrBuild);
+      } else {
+        for (uint32_t ti = e.x;; ti++) {
+          const float4* tp = reinterpret_cast<const float4*>(c.tris + ti);
+          const float4 a = __ldg(tp + 0), b = __ldg(tp + 1), d = __ldg(tp + 2);
+          bool skip = false;
+          if (EXCL) {  // a triangle whose hit a filter callback rejected
+            for (uint32_t x = xl; x < xh && !skip; x++) {
+              const uint2 y = __ldg(P.excl + x);
+              skip = y.x == __float_as_uint(a.w) && y.y == __float_as_uint(b.w);
+            }
+          }
+          if (!skip) {
+            if (COUNT) n_tris++;
+            float A1, B1, C1, D1;
+            if (test(a, b, d, org, make_float3(dn.x, dn.y, dn.z), dn.w, tfar, A1, B1, C1, D1)) {
+              hit = true;
+              hit_ti = ti;
+              A = A1; B = B1; C = C1; D = D1;
+              if (ANYHIT) break;
+              if (ti != end) tfar = ROBUST ? D : __fmul_rn(C, __frcp_rn(D));
+            }
+          }
+          if (ti == end) break;
+        }
+      }
+    }
+    if (ANYHIT) {
+      if (hit) {
+        commit(w0 + own, hit_ti, A, B, C, D);
+        if (SEEDED && (e.y & 256u)) s_seed[w0 + own] = hit_ti;
+      }
+      __syncwarp();
+    } else {
+      // a ray's hits are committed in queue order, each tested again against the
+      // distance that the ones before it left
+      uint32_t pend = __ballot_sync(0xFFFFFFFFu, hit);
+      while (pend) {
+        if (hit && lane == __ffs(__match_any_sync(pend, own)) - 1) {
+          commit(w0 + own, hit_ti, A, B, C, D);
+          if (SEEDED && (e.y & 256u)) s_seed[w0 + own] = hit_ti;
+          hit = false;
+        }
+        __syncwarp();
+        if (hit) {
+          const float tf = s_t[w0 + own];
+          hit = ROBUST ? D <= tf : C <= __fmul_rn(D, tf);
+        }
+        pend = __ballot_sync(0xFFFFFFFFu, hit);
+      }
+    }
+    qhead += n;
+    t_best = s_t[threadIdx.x];
+    if (ANYHIT && t_best == -INFINITY) {  // occluded: nothing left to search
+      active = false;
+      g_bits = 0;
+    }
+    __syncwarp();
+  };
   for (;;) {
-    // ---- refill idle lanes
-    const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !active);
-    if (!exhausted && __popc(idle) >= SH::kRefillIdle) {
+    // ---- write finished rays, refill idle lanes
+    uint32_t idle = __ballot_sync(0xFFFFFFFFu, !active);
+    const bool refill = idle == 0xFFFFFFFFu || (!exhausted && __popc(idle) >= SH::kRefillIdle * (P.batch_root ? kBatchedRefill : 1));
+    // waiting leaves (at most 31: one batch empties the ring) are tested before a
+    // refill and once there is one per active lane
+    if (!INST && qtail != qhead && (refill || qtail - qhead + __popc(idle) >= 32u)) {
+      flush();
+      if (ANYHIT) idle = __ballot_sync(0xFFFFFFFFu, !active);
+    }
+    if (refill) {
+      if (!active) {
+        const uint32_t hit_tri = s_tri[threadIdx.x];
+        if (hit_tri != kInvalidID) {
+          s_tri[threadIdx.x] = kInvalidID;
+          if (SEEDED && hit_tri == s_seed[threadIdx.x]) n_prop++;
+          char* rec = P.rays + (uint64_t)rid * P.stride;
+          if (ANYHIT) {
+            *reinterpret_cast<float*>(rec + 32) = -INFINITY;
+          } else {
+            const TriRecord* htris = (INST && hit_inst != kInvalidID) ? P.insts[hit_inst].tris : P.tris;
+            const uint32_t inst_id = (INST && hit_inst != kInvalidID) ? P.insts[hit_inst].geomID : kInvalidID;
+            const float4* tp = reinterpret_cast<const float4*>(htris + hit_tri);
+            const float4 a = __ldg(tp + 0), b = __ldg(tp + 1), d = __ldg(tp + 2);
+            const float3 Ng = ROBUST ? pluecker_normal(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z),
+                                                       make_float3(d.x, d.y, d.z), r.org)
+                                     : cross3(make_float3(d.x, d.y, d.z), make_float3(b.x, b.y, b.z));
+            const float hu = s_u[threadIdx.x], hv = s_v[threadIdx.x];
+            *reinterpret_cast<float*>(rec + 32) = s_t[threadIdx.x];
+            if (ALIGNED) {
+              *reinterpret_cast<float4*>(rec + 48) = make_float4(Ng.x, Ng.y, Ng.z, hu);
+              *reinterpret_cast<uint4*>(rec + 64) =
+                  make_uint4(__float_as_uint(hv), __float_as_uint(a.w), __float_as_uint(b.w), inst_id);
+            } else {
+              float* f = reinterpret_cast<float*>(rec + 48);
+              f[0] = Ng.x; f[1] = Ng.y; f[2] = Ng.z; f[3] = hu; f[4] = hv;
+              uint32_t* w = reinterpret_cast<uint32_t*>(rec + 68);
+              w[0] = __float_as_uint(a.w); w[1] = __float_as_uint(b.w); w[2] = inst_id;
+            }
+          }
+        }
+      }
+      if (exhausted) break;  // no ray left, no lane active
       const int leader = __ffs(idle) - 1;
       uint32_t base = 0;
       if (lane == leader) base = atomicAdd(P.ray_counter, (unsigned)__popc(idle));
       base = __shfl_sync(0xFFFFFFFFu, base, leader);
       if (base + __popc(idle) >= nrays) exhausted = true;
       if (!active) {
-        uint32_t rid = base + __popc(idle & lt_mask);
+        rid = base + __popc(idle & lt_mask);
         if (rid < nrays) {
           if (P.order) rid = __ldg(P.order + rid);  // the record this fetch slot traces
           if (EXCL) {
             ex_lo = __ldg(P.excl_off + rid);
             ex_hi = __ldg(P.excl_off + rid + 1);
           }
-          rec = P.rays + (uint64_t)rid * P.stride;
           float tfar;
-          load_ray<ALIGNED>(rec, r, tfar);
+          load_ray<ALIGNED>(P.rays + (uint64_t)rid * P.stride, r, tfar);
           // stream semantics: only tnear <= tfar rays are traced; any-hit also
           // skips already occluded rays (bvh_intersector_stream_filters.cpp:75)
           const bool valid = ANYHIT ? ((r.tnear <= tfar) && !(tfar < 0.0f)) : (r.tnear <= tfar);
           // batched queries: the ray's batch (binary search) gives its tree's root
           uint32_t root = 0;
           if (P.batch_root) {
-            uint32_t lo = 0, hi = P.nbatches;
+            // rays are fetched in order: most are in the batch of the last one
+            uint32_t lo = s_batch[warp], hi = P.nbatches;
+            if (__ldg(P.batch_start + lo) > rid) lo = 0;
+            else if (__ldg(P.batch_start + lo + 1) > rid) hi = lo + 1;
             while (hi - lo > 1) {
               const uint32_t mid = (lo + hi) >> 1;
               if (__ldg(P.batch_start + mid) <= rid) lo = mid; else hi = mid;
             }
+            s_batch[warp] = lo;
             root = __ldg(P.batch_root + lo);
           }
           if (INST) {  // a ray that ended inside an instance left the lane in its space
@@ -427,11 +638,12 @@ __global__ void __launch_bounds__(SH::kThreads, (COUNT || SEEDED || INST || EXCL
           }
           if (valid && root < c.num_nodes) {
             init_ray(r);
+            if (!INST) s_dir[threadIdx.x] = make_float4(r.dir.x, r.dir.y, r.dir.z, r.tnear);
             t_best = tfar;
-            hit_tri = kInvalidID;
+            s_t[threadIdx.x] = tfar;
+            s_tri[threadIdx.x] = kInvalidID;
             g_base = root;
-            g_bits = (0x80000000u >> r.oct) | 1u;  // virtual group: the root as internal slot 0
-            t_bits = 0;
+            g_bits = (0x80000000u >> r.oct) | (r.oct << 8) | 1u;  // virtual group: the root as internal slot 0
             sp = 0;
             iters = 0;
             active = true;
@@ -440,7 +652,7 @@ __global__ void __launch_bounds__(SH::kThreads, (COUNT || SEEDED || INST || EXCL
               const uint4 s4 = P.seeds[rid];
               const uint32_t sd[4] = {s4.x, s4.y, s4.z, s4.w};
               push(make_uint2(g_base, g_bits));
-              seed_tri = kInvalidID;
+              s_seed[threadIdx.x] = kInvalidID;
               seeding = false;
               for (int q = 3; q >= 0; q--) {
                 if (sd[q] == 0u || sd[q] >= c.num_nodes) continue;
@@ -455,167 +667,134 @@ __global__ void __launch_bounds__(SH::kThreads, (COUNT || SEEDED || INST || EXCL
         }
       }
     }
-    if (!__any_sync(0xFFFFFFFFu, active)) {
-      if (exhausted) break;
-      continue;
-    }
-    bool done = false, visited = false;
-    if (active && ++iters > c.max_iters) {
-      atomicOr(c.err, kErrIterationLimit);
-      active = false;
-    }
     // ---- (1) one node of the current group
-    if (active && t_bits == 0 && (g_bits & 0xFF000000u)) {
+    uint32_t leaf = 0, t_base = 0;
+    uint2 meta = make_uint2(0u, 0u);
+    if (active && (g_bits & 0xFF000000u)) {
       const uint32_t k = __clz(g_bits);  // visiting position of the next child (bit 31 - k)
       g_bits &= ~(0x80000000u >> k);
-      const uint32_t slot = k ^ r.oct;
+      const uint32_t row = g_bits & 0x700u;  // the ray's octant << 8
+      const uint32_t slot = k ^ (row >> 8);
       const uint32_t child = g_base + __popc(g_bits & ((1u << slot) - 1u) & 0xFFu);
-      if (g_bits & 0xFF000000u) {
-        if (sp < kStackSize) push(make_uint2(g_base, g_bits));
-        else { atomicOr(c.err, kErrStackOverflow); active = false; }
-      }
-      if (active && child >= c.num_nodes) { atomicOr(c.err, kErrBuild); active = false; }
-      if (active) {
+      const bool rest = (g_bits & 0xFF000000u) != 0u, room = !rest || sp < kStackSize;
+      if (room && child < c.num_nodes && ++iters <= c.max_iters) {
+        if (rest) push(make_uint2(g_base, g_bits));
         if (COUNT) n_nodes++;
-        intersect_node(c.nodes + child, r, t_best, g_base, g_bits, t_base, t_bits, s_perm[r.oct]);
-        visited = true;
-      }
-    }
-    // ---- (2) triangles, postponed while few lanes have any
-    if constexpr (kPostponePct > 0) {
-      const uint32_t want = __ballot_sync(0xFFFFFFFFu, active && t_bits != 0);
-      const uint32_t act = __ballot_sync(0xFFFFFFFFu, active);
-      if (visited && t_bits != 0 && __popc(want) * 100 < __popc(act) * kPostponePct) {
-        if (sp < kStackSize) {
-          push(make_uint2(t_base | kTriGroup, t_bits));
-          t_bits = 0;
-        }
-      }
-    }
-    while (active && t_bits) {
-      const uint32_t idx = __ffs(t_bits) - 1;
-      t_bits &= t_bits - 1;
-      const uint32_t ti = t_base + idx;
-      if (ti >= c.num_tris) { atomicOr(c.err, kErrBuild); active = false; break; }
-      const float4* tp = reinterpret_cast<const float4*>(c.tris + ti);
-      const float4 a = __ldg(tp + 0), b = __ldg(tp + 1), d = __ldg(tp + 2);
-      if (EXCL) {  // a triangle whose hit a filter callback rejected
-        bool skip = false;
-        for (uint32_t e = ex_lo; e < ex_hi && !skip; e++) {
-          const uint2 x = __ldg(P.excl + e);
-          skip = x.x == __float_as_uint(a.w) && x.y == __float_as_uint(b.w);
-        }
-        if (skip) continue;
-      }
-      if (INST && __float_as_uint(d.w) == kInstanceLeaf) {
-        const uint32_t ii = __float_as_uint(a.w);
-        if (cur_inst != kInvalidID) continue;  // nested instance: not traversed
-        if (ii >= P.ninsts) { atomicOr(c.err, kErrBuild); active = false; break; }
-        const InstDesc* in = P.insts + ii;
-        const uint32_t bn = in->num_nodes;
-        if (bn == 0) continue;  // empty instanced scene
-        if (sp + 3 > kStackSize) { atomicOr(c.err, kErrStackOverflow); active = false; break; }
-        // the node group of this visit (its hit internal children) and the rest of this
-        // leaf group resume after the instance
-        if (g_bits & 0xFF000000u) push(make_uint2(g_base, g_bits));
-        if (t_bits) push(make_uint2(t_base | kTriGroup, t_bits));
-        push(make_uint2(kInstMarker, 0u));
-        t_bits = 0;
-        cur_inst = ii;
-        c.nodes = in->nodes;
-        c.tris = in->tris;
-        c.num_nodes = bn;
-        c.num_tris = in->num_tris;
-        to_instance(in->w2l, r);
-        init_ray(r);
-        g_base = 0;
-        g_bits = (0x80000000u >> r.oct) | 1u;
-        break;
-      }
-      if (COUNT) n_tris++;
-      if (ROBUST) {
-        float U, V, UVW, t;
-        if (pluecker(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(d.x, d.y, d.z), r.org,
-                     r.dir, r.tnear, t_best, U, V, UVW, t)) {
-          hit_tri = ti;
-          if (INST) hit_inst = cur_inst;
-          if (SEEDED && seeding) seed_tri = ti;
-          if (ANYHIT) { done = true; t_bits = 0; break; }
-          // PlueckerHitM::finalize: u,v = U,V * rcp(UVW), 0 when |UVW| < 1e-18
-          const float rcp = fabsf(UVW) < kMinRcpInput ? 0.0f : __frcp_rn(UVW);
-          t_best = t;
-          hu = __fmul_rn(U, rcp);
-          hv = __fmul_rn(V, rcp);
-        }
+        intersect_node(c.nodes + child, r, t_best, g_base, g_bits, t_base, leaf, meta, &s_perm[0][0] + row, row);
       } else {
-        float U, V, T, absDen;
-        if (moeller(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), make_float3(d.x, d.y, d.z), r.org, r.dir,
-                    r.tnear, t_best, U, V, T, absDen)) {
-          hit_tri = ti;
-          if (INST) hit_inst = cur_inst;
-          if (SEEDED && seeding) seed_tri = ti;
-          if (ANYHIT) { done = true; t_bits = 0; break; }
-          const float rcp = __frcp_rn(absDen);
-          t_best = __fmul_rn(T, rcp);
-          hu = __fmul_rn(U, rcp);
-          hv = __fmul_rn(V, rcp);
-        }
+        atomicOr(c.err, !room ? kErrStackOverflow : child >= c.num_nodes ? kErrBuild : kErrIterationLimit);
+        active = false;
+        g_bits = 0;
       }
     }
-    // ---- (3) next group from the stack, or finish
-    if (active && !done && t_bits == 0 && !(g_bits & 0xFF000000u)) {
-      if (sp > 0) {
-        const uint2 e = pop();
-        if (INST && e.x == kInstMarker && e.y == 0u) {
-          // leaving the instance: world ray and top-level BVH again
-          float unused_tfar;
-          load_ray<ALIGNED>(rec, r, unused_tfar);
-          init_ray(r);
-          c.nodes = P.nodes;
-          c.tris = P.tris;
-          c.num_nodes = P.num_nodes;
-          c.num_tris = P.num_tris;
-          cur_inst = kInvalidID;
-          g_bits = 0;
-          t_bits = 0;
-        } else if ((INST || kPostponePct > 0) && (e.x & kTriGroup)) {
-          // triangle groups are pushed only by instance entries and by postponing
-          t_base = e.x & ~kTriGroup;
-          t_bits = e.y;
-          g_bits = 0;
+    if constexpr (!INST) {
+      // ---- (2) queue the leaves that were hit; a full batch is tested
+      for (uint32_t bal; (bal = __ballot_sync(0xFFFFFFFFu, leaf != 0u)) != 0u;) {
+        if (leaf) {
+          const uint32_t m = meta_of(meta, __ffs(leaf) - 1);
+          leaf &= leaf - 1u;
+          const uint32_t at = (qtail + __popc(bal & lt_mask)) & (kQueue - 1);
+          s_queue[warp][at] = make_uint2(t_base + (m & 31u), (uint32_t)lane | (m & 0xE0u) | (SEEDED && seeding ? 256u : 0u));
         }
-        else { g_base = e.x; g_bits = e.y; }
-        if (SEEDED && sp == 0) seeding = false;  // the root group: proposals are done
-      } else {
-        done = true;
+        qtail += __popc(bal);
+        if (qtail - qhead >= 32u) {
+          flush();
+          if (ANYHIT && !active) leaf = 0;
+        }
       }
-    }
-    if (active && done) {
-      active = false;
-      if (SEEDED && hit_tri != kInvalidID && hit_tri == seed_tri) n_prop++;
-      if (hit_tri != kInvalidID) {
-        if (ANYHIT) {
-          *reinterpret_cast<float*>(rec + 32) = -INFINITY;
-        } else {
-          const TriRecord* htris = (INST && hit_inst != kInvalidID) ? P.insts[hit_inst].tris : P.tris;
-          const uint32_t inst_id = (INST && hit_inst != kInvalidID) ? P.insts[hit_inst].geomID : kInvalidID;
-          const float4* tp = reinterpret_cast<const float4*>(htris + hit_tri);
+    } else {
+      // ---- (2) scenes with instances: each lane tests its own triangles, since
+      // entering an instance changes the lane's ray and BVH
+      uint32_t t_bits = 0;
+      while (leaf) {  // the triangle bits of the leaves that were hit
+        const uint32_t m = meta_of(meta, __ffs(leaf) - 1);
+        leaf &= leaf - 1u;
+        if (m & 0x80u) t_bits |= ((2u << ((m >> 5) & 3u)) - 1u) << (m & 31u);
+      }
+      bool popped = false;  // a triangle group came from the stack: test it too
+      do {
+        popped = false;
+        while (active && t_bits) {
+          const uint32_t idx = __ffs(t_bits) - 1;
+          t_bits &= t_bits - 1;
+          const uint32_t ti = t_base + idx;
+          if (ti >= c.num_tris) { atomicOr(c.err, kErrBuild); active = false; break; }
+          const float4* tp = reinterpret_cast<const float4*>(c.tris + ti);
           const float4 a = __ldg(tp + 0), b = __ldg(tp + 1), d = __ldg(tp + 2);
-          const float3 Ng = ROBUST ? pluecker_normal(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z),
-                                                     make_float3(d.x, d.y, d.z), r.org)
-                                   : cross3(make_float3(d.x, d.y, d.z), make_float3(b.x, b.y, b.z));
-          *reinterpret_cast<float*>(rec + 32) = t_best;
-          if (ALIGNED) {
-            *reinterpret_cast<float4*>(rec + 48) = make_float4(Ng.x, Ng.y, Ng.z, hu);
-            *reinterpret_cast<uint4*>(rec + 64) =
-                make_uint4(__float_as_uint(hv), __float_as_uint(a.w), __float_as_uint(b.w), inst_id);
-          } else {
-            float* f = reinterpret_cast<float*>(rec + 48);
-            f[0] = Ng.x; f[1] = Ng.y; f[2] = Ng.z; f[3] = hu; f[4] = hv;
-            uint32_t* w = reinterpret_cast<uint32_t*>(rec + 68);
-            w[0] = __float_as_uint(a.w); w[1] = __float_as_uint(b.w); w[2] = inst_id;
+          if (__float_as_uint(d.w) == kInstanceLeaf) {
+            const uint32_t ii = __float_as_uint(a.w);
+            if (cur_inst != kInvalidID) continue;  // nested instance: not traversed
+            if (ii >= P.ninsts) { atomicOr(c.err, kErrBuild); active = false; break; }
+            const InstDesc* in = P.insts + ii;
+            const uint32_t bn = in->num_nodes;
+            if (bn == 0) continue;  // empty instanced scene
+            if (sp + 3 > kStackSize) { atomicOr(c.err, kErrStackOverflow); active = false; break; }
+            // the node group of this visit (its hit internal children) and the rest of this
+            // leaf group resume after the instance
+            if (g_bits & 0xFF000000u) push(make_uint2(g_base, g_bits));
+            if (t_bits) push(make_uint2(t_base | kTriGroup, t_bits));
+            push(make_uint2(kInstMarker, 0u));
+            t_bits = 0;
+            cur_inst = ii;
+            c.nodes = in->nodes;
+            c.tris = in->tris;
+            c.num_nodes = bn;
+            c.num_tris = in->num_tris;
+            to_instance(in->w2l, r);
+            init_ray(r);
+            g_base = 0;
+            g_bits = (0x80000000u >> r.oct) | (r.oct << 8) | 1u;
+            break;
+          }
+          if (COUNT) n_tris++;
+          float A, B, C, D;
+          if (test(a, b, d, r.org, r.dir, r.tnear, t_best, A, B, C, D)) {
+            commit(threadIdx.x, ti, A, B, C, D);
+            t_best = s_t[threadIdx.x];
+            hit_inst = cur_inst;
+            if (ANYHIT) {
+              t_bits = 0;
+              g_bits = 0;
+              sp = 0;
+              break;
+            }
           }
         }
+        // back from an instance, or on to the rest of a leaf group
+        while (active && !(g_bits & 0xFF000000u) && sp > 0) {
+          const uint2 e = sp <= kSharedStack ? s_stack[sp - 1][stk_tid] : stack[sp - 1];
+          if (e.x == kInstMarker && e.y == 0u) {
+            // leaving the instance: world ray and top-level BVH again
+            sp--;
+            float unused_tfar;
+            load_ray<ALIGNED>(P.rays + (uint64_t)rid * P.stride, r, unused_tfar);
+            init_ray(r);
+            c.nodes = P.nodes;
+            c.tris = P.tris;
+            c.num_nodes = P.num_nodes;
+            c.num_tris = P.num_tris;
+            cur_inst = kInvalidID;
+          } else if (e.x & kTriGroup) {
+            sp--;
+            t_base = e.x & ~kTriGroup;
+            t_bits = e.y;
+            popped = true;
+            break;
+          } else {
+            break;
+          }
+        }
+      } while (popped);
+    }
+    // ---- (3) next group from the stack, or finish
+    if (active && !(g_bits & 0xFF000000u)) {
+      if (sp > 0) {
+        const uint2 e = pop();
+        g_base = e.x;
+        g_bits = e.y;
+        if (SEEDED && sp == 0) seeding = false;  // the root group: proposals are done
+      } else {
+        active = false;
       }
     }
   }
