@@ -1773,6 +1773,10 @@ __device__ __forceinline__ void collapse_emit_node(
   node.ey = (uint8_t)Ey;
   node.ez = (uint8_t)Ez;
   node.imask = 0;
+  node.sx = sx * 32768.0f;
+  node.sy = sy * 32768.0f;
+  node.sz = sz * 32768.0f;
+  node.pad = 0;
   node.child_base = next_base + off_int[k];
   node.tri_base = tri_next + off_tri[k];
   uint32_t int_rank = 0, tri_off = 0;
@@ -1997,7 +2001,7 @@ __device__ __forceinline__ void collapse_emit_group(
     if (i == 0) atomicOr(err, kErrBuild);
     return;
   }
-  // WideNode as five 16-byte words (gb_common.h layout)
+  // WideNode as six 16-byte words (gb_common.h layout)
   uint4* dst = reinterpret_cast<uint4*>(nodes + level_base + k);
   if (i == 0) {
     dst[0] = make_uint4(__float_as_uint(ulo.x), __float_as_uint(ulo.y), __float_as_uint(ulo.z),
@@ -2010,6 +2014,9 @@ __device__ __forceinline__ void collapse_emit_group(
     dst[3] = make_uint4(lz0, lz1, hx0, hx1);
   } else if (i == 4) {
     dst[4] = make_uint4(hy0, hy1, hz0, hz1);
+  } else if (i == 5) {
+    dst[5] = make_uint4(__float_as_uint(sx * 32768.0f), __float_as_uint(sy * 32768.0f),
+                        __float_as_uint(sz * 32768.0f), 0u);
   }
 }
 
@@ -3247,6 +3254,9 @@ __device__ __forceinline__ void refit_node(const float4* __restrict__ tri_box, u
   node.ex = (uint8_t)Ex;
   node.ey = (uint8_t)Ey;
   node.ez = (uint8_t)Ez;
+  node.sx = sx * 32768.0f;
+  node.sy = sy * 32768.0f;
+  node.sz = sz * 32768.0f;
   double sah = 0.0, sahx = 0.0;
   for (int s = 0; s < 8; s++) {
     if (node.meta[s] == 0) continue;

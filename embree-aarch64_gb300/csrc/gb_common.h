@@ -1,10 +1,10 @@
 // gb_common.h -- data layouts shared by the GPU builder, the traversal kernels
 // and the C-ABI host layer of the GB300 triangle ray-query library.
 //
-// HBM layout of one committed scene (all arrays 16-byte aligned):
-//   WideNode  nodes[num_nodes]   80 B each: 8-wide node, child boxes quantised
+// HBM layout of one committed scene (all arrays 32-byte aligned):
+//   WideNode  nodes[num_nodes]   96 B each: 8-wide node, child boxes quantised
 //                                to 8 bits per plane relative to a per-node
-//                                origin and power-of-two scale (5 x 16-B loads)
+//                                origin and power-of-two scale (3 x 32-B loads)
 //   TriRecord tris[num_tris]     48 B each: v0, e1 = v0-v1, e2 = v2-v0 (the
 //                                reference's Triangle4 lane contents,
 //                                kernels/geometry/triangle.h:40-41) + ids
@@ -28,7 +28,7 @@ constexpr int kLeafMaxLimit = 4;     // largest leaf the node encoding allows
 constexpr int kLeafMaxDefault = 0;
 constexpr int kStackSize = 64;       // traversal stack entries (node groups)
 
-// 80-byte wide node.
+// 96-byte wide node: an 80-byte record and, for the traversal, the scales as floats.
 //   meta[s]: 0 = empty slot; otherwise bit 7 is set and, for a leaf, bits
 //            5..6 hold (triangle count - 1) and bits 0..4 the first
 //            triangle's offset from tri_base (0..28).  An empty slot's box is
@@ -38,7 +38,7 @@ constexpr int kStackSize = 64;       // traversal stack entries (node groups)
 //   ex/ey/ez: IEEE-754 biased exponent of the per-axis scale 2^(e-127).
 //   decoded child box: lo = p + qlo * scale, hi = p + qhi * scale (the
 //   quantisation rounds outward, so the decoded box contains the child).
-struct alignas(16) WideNode {
+struct alignas(32) WideNode {
   float px, py, pz;
   uint8_t ex, ey, ez, imask;
   uint32_t child_base;
@@ -46,8 +46,11 @@ struct alignas(16) WideNode {
   uint8_t meta[8];
   uint8_t qlo_x[8], qlo_y[8], qlo_z[8];
   uint8_t qhi_x[8], qhi_y[8], qhi_z[8];
+  float sx, sy, sz;  // 2^15 * scale
+  uint32_t pad;
 };
-static_assert(sizeof(WideNode) == 80, "WideNode must be 80 bytes");
+static_assert(sizeof(WideNode) == 96, "WideNode must be three 32-byte words");
+constexpr size_t kNodeRecordBytes = 80;  // the part of a node that rtcgbGetSceneBVH copies out (all but sx .. pad)
 
 // 48-byte triangle record: (v0.xyz, primID), (e1.xyz, geomID), (e2.xyz, pad);
 // in robust scenes (v0.xyz, primID), (v1.xyz, geomID), (v2.xyz, pad), the

@@ -2074,7 +2074,9 @@ RTC_API unsigned int rtcgbGetSceneBVH(RTCScene hs, void* nodes, unsigned int max
   if (!s->committed) fail(RTC_ERROR_INVALID_OPERATION, "scene not committed");
   s->device->set_current();
   const unsigned nn = std::min(max_nodes, s->bvh.num_nodes), nt = std::min(max_tris, s->bvh.num_tris);
-  if (nodes && nn) cuda_ok(cudaMemcpy(nodes, s->bvh.nodes, (size_t)nn * sizeof(gb::WideNode), cudaMemcpyDeviceToHost), "copy nodes");
+  if (nodes && nn)
+    cuda_ok(cudaMemcpy2D(nodes, gb::kNodeRecordBytes, s->bvh.nodes, sizeof(gb::WideNode), gb::kNodeRecordBytes, nn,
+                         cudaMemcpyDeviceToHost), "copy nodes");
   if (tris && nt) cuda_ok(cudaMemcpy(tris, s->bvh.tris, (size_t)nt * sizeof(gb::TriRecord), cudaMemcpyDeviceToHost), "copy tris");
   if (num_tris) *num_tris = s->bvh.num_tris;
   return s->bvh.num_nodes;
