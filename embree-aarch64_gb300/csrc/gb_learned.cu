@@ -646,7 +646,6 @@ constexpr int kTcThreads = kTcScanThreads + 32;     // + the producer warp
 constexpr int kTcRays = 128;                        // UMMA M
 constexpr int kTcN = 256;                           // UMMA N: treelets per chunk
 constexpr int kTcK = kHidden + 16;                  // 64 weights + bias (hi, lo) + zero padding
-constexpr int kTcChunks = kTreelets / kTcN;         // 16
 constexpr uint32_t kTcChunkBytes = kTcN * kTcK * 2; // 40 KB
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kTcStages = 2;                   // weight chunks in flight
@@ -841,7 +840,7 @@ __global__ void __launch_bounds__(256) k_propose_hidden(const char* rays, uint64
 }
 
 __global__ void __launch_bounds__(kTcThreads, 1)
-    k_propose_tc(uint32_t M, const uint32_t* d_count, const uint16_t* __restrict__ H,
+    k_propose_tc(uint32_t M, const uint32_t* d_count, const uint32_t nchunks, const uint16_t* __restrict__ H,
                  const uint16_t* __restrict__ W4p, const uint32_t* __restrict__ node_of_treelet, uint4* seeds,
                  uint32_t* treelets, uint32_t* err) {
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
@@ -872,7 +871,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (d_count) M = min(M, *d_count);
   const uint32_t ntiles = (M + kTcRays - 1) / kTcRays;
   const uint32_t my_tiles = blockIdx.x < ntiles ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
-  const uint32_t total_chunks = my_tiles * kTcChunks;
+  const uint32_t total_chunks = my_tiles * nchunks;
   auto tile_src = [&](uint32_t k) { return H + (size_t)(blockIdx.x + k * gridDim.x) * kTcRays * kTcK; };
 
   // phases started on each barrier by the producer (bulk copies and MMA
@@ -887,11 +886,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       n_a[0]++;
       if (my_tiles > 1) bulk_load(S.a[1], tile_src(1), kTcTileBytes, &S.a_bar[1]), n_a[1]++;
       for (uint32_t q = 0; q < kTcStages && q < total_chunks; q++) {
-        bulk_load(S.w4[q], W4p + (size_t)(q % kTcChunks) * kTcN * kTcK, kTcChunkBytes, &S.tma_bar[q]);
+        bulk_load(S.w4[q], W4p + (size_t)(q % nchunks) * kTcN * kTcK, kTcChunkBytes, &S.tma_bar[q]);
         n_w[q]++;
       }
+      uint32_t k = 0, c = 0;  // tile and chunk of gc
       for (uint32_t gc = 0; gc < total_chunks && ok; gc++) {
-        const uint32_t k = gc / kTcChunks, c = gc % kTcChunks, s = gc & 1u, ab = k & 1u;
+        const uint32_t s = gc & 1u, ab = k & 1u;
         const uint32_t ws = gc % kTcStages;
         if (c == 0) ok = mbar_wait(&S.a_bar[ab], (k >> 1) & 1u);                       // A operand of tile k
         if (ok) ok = mbar_wait(&S.tma_bar[ws], (gc / kTcStages) & 1u);                 // weights of chunk gc
@@ -909,16 +909,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (gc >= 1 && gc - 1 + kTcStages < total_chunks) {
           if (!(ok = mbar_wait(&S.mma_bar[(gc - 1) & 1u], ((gc - 1) >> 1) & 1u))) break;
           const uint32_t nc = gc - 1 + kTcStages;
-          bulk_load(S.w4[nc % kTcStages], W4p + (size_t)(nc % kTcChunks) * kTcN * kTcK, kTcChunkBytes,
+          bulk_load(S.w4[nc % kTcStages], W4p + (size_t)(nc % nchunks) * kTcN * kTcK, kTcChunkBytes,
                     &S.tma_bar[nc % kTcStages]);
           n_w[nc % kTcStages]++;
         }
         // after the last MMA of tile k, its A buffer takes tile k + 2
-        if (c == kTcChunks - 1 && k + 2 < my_tiles) {
+        if (c == nchunks - 1 && k + 2 < my_tiles) {
           if (!(ok = mbar_wait(&S.mma_bar[s], (gc >> 1) & 1u))) break;
           bulk_load(S.a[ab], tile_src(k + 2), kTcTileBytes, &S.a_bar[ab]);
           n_a[ab]++;
         }
+        if (++c == nchunks) c = 0, k++;
       }
       if (!ok) {
         *(volatile uint32_t*)&S.fail = 1u;
@@ -936,7 +937,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
       for (int q = 0; q < 4; q++) { v[q] = -INFINITY; ix[q] = -1; }
       bool ok = true;
-      for (int c = 0; c < kTcChunks; c++, gc++) {
+      for (uint32_t c = 0; c < nchunks; c++, gc++) {
         const uint32_t s = gc & 1u;
         if (!mbar_wait(&S.mma_bar[s], (gc >> 1) & 1u)) { ok = false; break; }
         tc_fence_after();
@@ -948,7 +949,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&S.epi_bar[s]);  // this warp is done with accumulator s
-        const int col0 = c * kTcN + quarter * 64;
+        const int col0 = (int)c * kTcN + quarter * 64;
         float m0 = __uint_as_float(acc0[0]), m1 = __uint_as_float(acc1[0]);
 #pragma unroll
         for (int q = 1; q < 32; q++) {
@@ -1257,8 +1258,11 @@ cudaError_t Proposer::predict(const char* rays, uint64_t stride, uint32_t M, uin
     }
     k_propose_hidden<<<std::min<uint32_t>(ntiles, (uint32_t)num_sms() * 4), 256, sizeof(HidSmem), st>>>(
         rays, stride, M, d_count, grid, Pb_, P_, H_);
+    // only the chunks that hold treelets: the rest of the outputs carry a -inf bias
+    // and are never proposed (2M rays, 1,024 of 4,096 treelets: 2.68 -> 1.82 ms)
+    const uint32_t nchunks = std::max(1u, (num_treelets + kTcN - 1) / kTcN);
     k_propose_tc<<<std::min<uint32_t>(ntiles, (uint32_t)num_sms()), kTcThreads, sizeof(TcSmem), st>>>(
-        M, d_count, H_, W4p_, node_of_treelet_, seeds, treelets, err ? err : err_);
+        M, d_count, nchunks, H_, W4p_, node_of_treelet_, seeds, treelets, err ? err : err_);
     note_launches(2);
     return cudaGetLastError();
   }
