@@ -3174,14 +3174,11 @@ __device__ __forceinline__ bool refit_tri_vertices(const GeomDesc* __restrict__ 
   return vtx_ok(p0.x, p0.y, p0.z) && vtx_ok(p1.x, p1.y, p1.z) && vtx_ok(p2.x, p2.y, p2.z);
 }
 
-// Rewrites every triangle record from the current vertices and stores the
-// triangle's box (tri_box[2i] = lo, [2i + 1] = hi) for the node levels.
-__global__ void __launch_bounds__(256) k_refit_tris(const GeomDesc* __restrict__ geoms,
-                                                    const uint32_t* __restrict__ slot_of, uint32_t nslots,
-                                                    TriRecord* __restrict__ tris, uint32_t n, int robust,
-                                                    float4* __restrict__ tri_box, uint32_t* err) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// Rewrites triangle record i from the current vertices and stores the triangle's
+// box (tri_box[2i] = lo, [2i + 1] = hi) for the node levels.
+__device__ __forceinline__ void refit_tri(const GeomDesc* __restrict__ geoms, const uint32_t* __restrict__ slot_of,
+                                          uint32_t nslots, TriRecord* __restrict__ tris, uint32_t i, int robust,
+                                          float4* __restrict__ tri_box, uint32_t* err) {
   TriRecord rec = tris[i];
   float3 p0, p1, p2;
   if (!refit_tri_vertices(geoms, slot_of, nslots, rec, p0, p1, p2)) {
@@ -3200,175 +3197,159 @@ __global__ void __launch_bounds__(256) k_refit_tris(const GeomDesc* __restrict__
 }
 
 // Refits wide node k from its children's boxes (inner children: node_box of the
-// level below; leaf children: the boxes k_refit_tris stored for their
-// triangles, independent loads); returns the node's SAH terms on the decoded
-// and on the exact boxes.
-__device__ __forceinline__ void refit_node(const float4* __restrict__ tri_box, uint32_t num_tris,
-                                           WideNode* __restrict__ nodes, uint32_t num_nodes,
-                                           float* __restrict__ node_box, uint32_t k, uint32_t* err, double& sah_out,
-                                           double& sahx_out) {
-  WideNode node = nodes[k];
-  float3 clo[8], chi[8];
-  float3 ulo = make_float3(INFINITY, INFINITY, INFINITY), uhi = make_float3(-INFINITY, -INFINITY, -INFINITY);
-  uint32_t rank = 0;
-  for (int s = 0; s < 8; s++) {
-    clo[s] = make_float3(INFINITY, INFINITY, INFINITY);
-    chi[s] = make_float3(-INFINITY, -INFINITY, -INFINITY);
-    const uint32_t m = node.meta[s];
-    if (m == 0) continue;
-    if (node.imask >> s & 1u) {
-      const uint32_t c = node.child_base + rank++;
+// level below; leaf children: the boxes refit_tri stored for their triangles) and
+// adds the node's SAH terms on the decoded and on the exact boxes.  The 8 lanes of
+// a lane group share the node, lane i its slot i (all 8 call it with the same k;
+// gmask names them): the children's loads are one dependent step instead of eight,
+// and a level takes as long as its widest lane.  Boxes are read past L1, where
+// another CTA of the same launch may have written them.
+__device__ __forceinline__ void refit_node_group(const float4* tri_box, uint32_t num_tris,
+                                                 WideNode* __restrict__ nodes, uint32_t num_nodes, float* node_box,
+                                                 uint32_t k, uint32_t gmask, uint32_t* err, double& sah_out,
+                                                 double& sahx_out) {
+  const uint32_t s = threadIdx.x & 7u;
+  WideNode* node = nodes + k;
+  const uint32_t m = node->meta[s], imask = node->imask;
+  float3 lo = make_float3(INFINITY, INFINITY, INFINITY), hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
+  bool ok = true;
+  if (m != 0) {
+    if (imask >> s & 1u) {
+      const uint32_t c = node->child_base + __popc(imask & ((1u << s) - 1u));
       if (c >= num_nodes || c <= k) {
-        atomicOr(err, kErrBuild);
-        return;
+        ok = false;
+      } else {
+        const float* bx = node_box + 6 * (size_t)c;
+        lo = make_float3(__ldcg(bx + 0), __ldcg(bx + 1), __ldcg(bx + 2));
+        hi = make_float3(__ldcg(bx + 3), __ldcg(bx + 4), __ldcg(bx + 5));
       }
-      clo[s] = make_float3(node_box[6 * (size_t)c + 0], node_box[6 * (size_t)c + 1], node_box[6 * (size_t)c + 2]);
-      chi[s] = make_float3(node_box[6 * (size_t)c + 3], node_box[6 * (size_t)c + 4], node_box[6 * (size_t)c + 5]);
     } else {
-      const uint32_t cnt = ((m >> 5) & 3u) + 1u, first = node.tri_base + (m & 31u);
+      const uint32_t cnt = ((m >> 5) & 3u) + 1u, first = node->tri_base + (m & 31u);
       if (first + cnt > num_tris) {
-        atomicOr(err, kErrBuild);
-        return;
-      }
+        ok = false;
+      } else {
 #pragma unroll
-      for (uint32_t q = 0; q < 4; q++) {
-        if (q < cnt) {
-          const float4 a = tri_box[2 * (size_t)(first + q)], b = tri_box[2 * (size_t)(first + q) + 1];
-          clo[s] = f3min(clo[s], make_float3(a.x, a.y, a.z));
-          chi[s] = f3max(chi[s], make_float3(b.x, b.y, b.z));
+        for (uint32_t q = 0; q < 4; q++) {
+          if (q < cnt) {
+            const float4 a = __ldcg(tri_box + 2 * (size_t)(first + q)), b = __ldcg(tri_box + 2 * (size_t)(first + q) + 1);
+            lo = f3min(lo, make_float3(a.x, a.y, a.z));
+            hi = f3max(hi, make_float3(b.x, b.y, b.z));
+          }
         }
       }
     }
-    ulo = f3min(ulo, clo[s]);
-    uhi = f3max(uhi, chi[s]);
+  }
+  if (__any_sync(gmask, !ok)) {
+    if (s == 0) atomicOr(err, kErrBuild);
+    return;
+  }
+  float3 ulo = lo, uhi = hi;
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    ulo.x = fminf(ulo.x, __shfl_xor_sync(gmask, ulo.x, o, 8));
+    ulo.y = fminf(ulo.y, __shfl_xor_sync(gmask, ulo.y, o, 8));
+    ulo.z = fminf(ulo.z, __shfl_xor_sync(gmask, ulo.z, o, 8));
+    uhi.x = fmaxf(uhi.x, __shfl_xor_sync(gmask, uhi.x, o, 8));
+    uhi.y = fmaxf(uhi.y, __shfl_xor_sync(gmask, uhi.y, o, 8));
+    uhi.z = fmaxf(uhi.z, __shfl_xor_sync(gmask, uhi.z, o, 8));
   }
   const uint32_t Ex = exp_for(__fsub_ru(uhi.x, ulo.x));
   const uint32_t Ey = exp_for(__fsub_ru(uhi.y, ulo.y));
   const uint32_t Ez = exp_for(__fsub_ru(uhi.z, ulo.z));
   const float sx = __uint_as_float(Ex << 23), sy = __uint_as_float(Ey << 23), sz = __uint_as_float(Ez << 23);
-  const float ix = __uint_as_float((254u - Ex) << 23), iy = __uint_as_float((254u - Ey) << 23),
-              iz = __uint_as_float((254u - Ez) << 23);
-  node.px = ulo.x;
-  node.py = ulo.y;
-  node.pz = ulo.z;
-  node.ex = (uint8_t)Ex;
-  node.ey = (uint8_t)Ey;
-  node.ez = (uint8_t)Ez;
-  node.sx = sx * 32768.0f;
-  node.sy = sy * 32768.0f;
-  node.sz = sz * 32768.0f;
-  double sah = 0.0, sahx = 0.0;
-  for (int s = 0; s < 8; s++) {
-    if (node.meta[s] == 0) continue;
-    const float3 a = clo[s], b = chi[s];
-    sahx += (double)fmaxf(0.f, half_area(a, b));
-    const float qlx = fminf(fmaxf(floorf(__fsub_rd(a.x, ulo.x) * ix), 0.f), 255.f);
-    const float qly = fminf(fmaxf(floorf(__fsub_rd(a.y, ulo.y) * iy), 0.f), 255.f);
-    const float qlz = fminf(fmaxf(floorf(__fsub_rd(a.z, ulo.z) * iz), 0.f), 255.f);
-    const float qhx = fminf(fmaxf(ceilf(__fsub_ru(b.x, ulo.x) * ix), 0.f), 255.f);
-    const float qhy = fminf(fmaxf(ceilf(__fsub_ru(b.y, ulo.y) * iy), 0.f), 255.f);
-    const float qhz = fminf(fmaxf(ceilf(__fsub_ru(b.z, ulo.z) * iz), 0.f), 255.f);
-    node.qlo_x[s] = (uint8_t)qlx; node.qlo_y[s] = (uint8_t)qly; node.qlo_z[s] = (uint8_t)qlz;
-    node.qhi_x[s] = (uint8_t)qhx; node.qhi_y[s] = (uint8_t)qhy; node.qhi_z[s] = (uint8_t)qhz;
+  if (m != 0) {
+    const float ix = __uint_as_float((254u - Ex) << 23), iy = __uint_as_float((254u - Ey) << 23),
+                iz = __uint_as_float((254u - Ez) << 23);
+    const float qlx = fminf(fmaxf(floorf(__fsub_rd(lo.x, ulo.x) * ix), 0.f), 255.f);
+    const float qly = fminf(fmaxf(floorf(__fsub_rd(lo.y, ulo.y) * iy), 0.f), 255.f);
+    const float qlz = fminf(fmaxf(floorf(__fsub_rd(lo.z, ulo.z) * iz), 0.f), 255.f);
+    const float qhx = fminf(fmaxf(ceilf(__fsub_ru(hi.x, ulo.x) * ix), 0.f), 255.f);
+    const float qhy = fminf(fmaxf(ceilf(__fsub_ru(hi.y, ulo.y) * iy), 0.f), 255.f);
+    const float qhz = fminf(fmaxf(ceilf(__fsub_ru(hi.z, ulo.z) * iz), 0.f), 255.f);
+    node->qlo_x[s] = (uint8_t)qlx; node->qlo_y[s] = (uint8_t)qly; node->qlo_z[s] = (uint8_t)qlz;
+    node->qhi_x[s] = (uint8_t)qhx; node->qhi_y[s] = (uint8_t)qhy; node->qhi_z[s] = (uint8_t)qhz;
     const float3 dlo = make_float3(__fmaf_rd(qlx, sx, ulo.x), __fmaf_rd(qly, sy, ulo.y), __fmaf_rd(qlz, sz, ulo.z));
     const float3 dhi = make_float3(__fmaf_ru(qhx, sx, ulo.x), __fmaf_ru(qhy, sy, ulo.y), __fmaf_ru(qhz, sz, ulo.z));
-    sah += (double)fmaxf(0.f, half_area(dlo, dhi));  // leaves of <= 4 triangles: one block each
+    sah_out += (double)fmaxf(0.f, half_area(dlo, dhi));  // leaves of <= 4 triangles: one block each
+    sahx_out += (double)fmaxf(0.f, half_area(lo, hi));
   }
-  nodes[k] = node;
-  node_box[6 * (size_t)k + 0] = ulo.x; node_box[6 * (size_t)k + 1] = ulo.y; node_box[6 * (size_t)k + 2] = ulo.z;
-  node_box[6 * (size_t)k + 3] = uhi.x; node_box[6 * (size_t)k + 4] = uhi.y; node_box[6 * (size_t)k + 5] = uhi.z;
-  sah_out = sah;
-  sahx_out = sahx;
+  // frame and scales (16-byte words 0 and 5), then the node's box
+  if (s == 0)
+    reinterpret_cast<uint4*>(node)[0] = make_uint4(__float_as_uint(ulo.x), __float_as_uint(ulo.y), __float_as_uint(ulo.z),
+                                                   Ex | (Ey << 8) | (Ez << 16) | (imask << 24));
+  else if (s == 1)
+    reinterpret_cast<uint4*>(node)[5] = make_uint4(__float_as_uint(sx * 32768.0f), __float_as_uint(sy * 32768.0f),
+                                                   __float_as_uint(sz * 32768.0f), 0u);
+  else
+    node_box[6 * (size_t)k + s - 2] = s == 2 ? ulo.x : s == 3 ? ulo.y : s == 4 ? ulo.z : s == 5 ? uhi.x : s == 6 ? uhi.y : uhi.z;
 }
 
-// One node of the level [begin, end) per thread; SAH sums reduced per CTA.
-__global__ void __launch_bounds__(128) k_refit_level(const float4* __restrict__ tri_box, uint32_t num_tris,
-                                                     WideNode* __restrict__ nodes, uint32_t num_nodes,
-                                                     float* __restrict__ node_box, uint32_t begin, uint32_t end,
-                                                     double* sah_acc, uint32_t* err) {
-  const uint32_t k = begin + blockIdx.x * blockDim.x + threadIdx.x;
+// The breadth-first levels of a BVH whose levels fit (deeper ones are refitted by
+// one launch per level).
+struct RefitLevels {
+  uint32_t n;
+  uint32_t start[kColMaxLevels + 1];
+};
+
+// Levels of at most this many nodes are refitted by the first CTA alone, without a
+// grid barrier between two of them.
+constexpr uint32_t kRefitNarrow = 64;
+
+// The whole refit in one cooperative launch: the triangles, then the levels,
+// deepest first, a grid barrier between two levels.  A refit is a chain of about 14
+// levels that each take a few microseconds at most: as one launch per level with
+// one thread per node, its eight children's loads in sequence, the chain took
+// 0.44 ms on a 1M-triangle soup whatever the bandwidth (the whole refit 0.61 ms;
+// here 0.14 ms, of which the 176 MB of the triangle pass need 0.03).  *bar and *bar_err are
+// zero before the first launch and left ready for the next one (an error of the
+// triangles or nodes does not stop the refit, a barrier that fails does).
+__global__ void __launch_bounds__(256) k_refit_all(const GeomDesc* __restrict__ geoms,
+                                                   const uint32_t* __restrict__ slot_of, uint32_t nslots,
+                                                   TriRecord* __restrict__ tris, uint32_t num_tris, int robust,
+                                                   float4* tri_box, WideNode* __restrict__ nodes, uint32_t num_nodes,
+                                                   float* node_box, const RefitLevels lv, double* sah_acc,
+                                                   GridBarrier* bar, unsigned int* bar_err, uint32_t* err) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < num_tris; i += gridDim.x * blockDim.x)
+    refit_tri(geoms, slot_of, nslots, tris, i, robust, tri_box, err);
   double sah = 0.0, sahx = 0.0;
-  if (k < end && k < num_nodes) refit_node(tri_box, num_tris, nodes, num_nodes, node_box, k, err, sah, sahx);
+  const uint32_t gmask = 0xFFu << (threadIdx.x & 24u);
+  bool wide_below = true;
+  for (uint32_t l = lv.n; l-- > 0;) {
+    const uint32_t begin = lv.start[l], end = min(lv.start[l + 1], num_nodes);
+    const bool wide = end - begin > kRefitNarrow;
+    if (wide || wide_below) {
+      if (!grid_sync(bar, bar_err)) {
+        if (threadIdx.x == 0) atomicOr(err, kErrBuild);
+        break;
+      }
+    } else {
+      __syncthreads();
+    }
+    wide_below = wide;
+    if (!wide && blockIdx.x != 0) continue;
+    const uint32_t stride = (wide ? gridDim.x * blockDim.x : blockDim.x) >> 3;
+    for (uint32_t k = begin + ((wide ? blockIdx.x * blockDim.x + threadIdx.x : threadIdx.x) >> 3); k < end; k += stride)
+      refit_node_group(tri_box, num_tris, nodes, num_nodes, node_box, k, gmask, err, sah, sahx);
+  }
   block_add2(sah, sahx, sah_acc);
 }
 
-cudaError_t refit_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, DeviceBVH* bvh, BuildStats* stats,
-                      bool* fallback) {
-  *fallback = false;
-  if (bvh->num_nodes == 0 || bvh->level_start.size() < 2) {
-    *fallback = true;
-    return cudaSuccess;
-  }
-  cudaEvent_t ev0, ev1;
-  GB_CHECK(cudaEventCreate(&ev0));
-  GB_CHECK(cudaEventCreate(&ev1));
-  GB_CHECK(cudaEventRecord(ev0, st));
-  uint32_t nslots = 0;
-  for (int g = 0; g < ngeoms; g++) nslots = std::max(nslots, h_geoms[g].geomID + 1);
-  std::vector<uint32_t> slot_of(std::max(nslots, 1u), kInvalidID);
-  for (int g = 0; g < ngeoms; g++) slot_of[h_geoms[g].geomID] = (uint32_t)g;
-  GeomDesc* d_geoms = nullptr;
-  uint32_t *d_slot = nullptr, *d_err = nullptr;
-  float* node_box = nullptr;
-  float4* tri_box = nullptr;
-  double* d_sah = nullptr;
-  GB_CHECK(dalloc(&d_geoms, ngeoms, st));
-  GB_CHECK(dalloc(&tri_box, 2 * (size_t)bvh->num_tris, st));
-  GB_CHECK(dalloc(&d_slot, slot_of.size(), st));
-  GB_CHECK(dalloc(&d_err, 1, st));
-  GB_CHECK(dalloc(&node_box, (size_t)6 * bvh->num_nodes, st));
-  GB_CHECK(dalloc(&d_sah, 2, st));
-  GB_CHECK(cudaMemcpyAsync(d_geoms, h_geoms, sizeof(GeomDesc) * ngeoms, cudaMemcpyHostToDevice, st));
-  GB_CHECK(cudaMemcpyAsync(d_slot, slot_of.data(), sizeof(uint32_t) * slot_of.size(), cudaMemcpyHostToDevice, st));
-  GB_CHECK(cudaMemsetAsync(d_err, 0, sizeof(uint32_t), st));
-  GB_CHECK(cudaMemsetAsync(d_sah, 0, 2 * sizeof(double), st));
-  k_refit_tris<<<cdiv(bvh->num_tris, 256), 256, 0, st>>>(d_geoms, d_slot, (uint32_t)slot_of.size(), bvh->tris,
-                                                         bvh->num_tris, bvh->robust, tri_box, d_err);
-  note_launches(1);
-  for (size_t l = bvh->level_start.size() - 1; l-- > 0;) {
-    const uint32_t b = bvh->level_start[l], e = bvh->level_start[l + 1];
-    if (e <= b) continue;
-    k_refit_level<<<cdiv(e - b, 128), 128, 0, st>>>(tri_box, bvh->num_tris, bvh->nodes, bvh->num_nodes, node_box, b,
-                                                   e, d_sah, d_err);
-    note_launches(1);
-  }
-  GB_CHECK(cudaGetLastError());
-  uint32_t err = 0;
-  float root[6];
-  double sah_sum[2] = {0.0, 0.0};
-  GB_CHECK(cudaMemcpyAsync(&err, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  GB_CHECK(cudaMemcpyAsync(root, node_box, sizeof(root), cudaMemcpyDeviceToHost, st));
-  GB_CHECK(cudaMemcpyAsync(sah_sum, d_sah, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  GB_CHECK(cudaEventRecord(ev1, st));
-  cudaFreeAsync(d_geoms, st);
-  cudaFreeAsync(d_slot, st);
-  cudaFreeAsync(d_err, st);
-  cudaFreeAsync(node_box, st);
-  cudaFreeAsync(tri_box, st);
-  cudaFreeAsync(d_sah, st);
-  GB_CHECK(cudaStreamSynchronize(st));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ev0, ev1);
-  cudaEventDestroy(ev0);
-  cudaEventDestroy(ev1);
-  if (err) {  // a vertex became invalid or the records are inconsistent: rebuild
-    *fallback = true;
-    return cudaSuccess;
-  }
-  for (int d = 0; d < 3; d++) {
-    bvh->lo[d] = root[d];
-    bvh->hi[d] = root[3 + d];
-  }
-  const float gx = bvh->hi[0] - bvh->lo[0], gy = bvh->hi[1] - bvh->lo[1], gz = bvh->hi[2] - bvh->lo[2];
-  const double Aroot = std::max(0.0, (double)(gx * (gy + gz) + gy * gz));
-  stats->sah = Aroot > 0 ? (Aroot + sah_sum[0]) / Aroot : 0.0;
-  stats->sah_exact = Aroot > 0 ? (Aroot + sah_sum[1]) / Aroot : 0.0;
-  stats->build_ms = ms;
-  stats->num_nodes = bvh->num_nodes;
-  stats->num_prims = bvh->num_tris;
-  stats->depth = bvh->depth;
-  stats->refit = 1;
-  return cudaSuccess;
+// The same as separate launches, for BVHs of more levels than RefitLevels holds.
+__global__ void __launch_bounds__(256) k_refit_tris(const GeomDesc* __restrict__ geoms,
+                                                    const uint32_t* __restrict__ slot_of, uint32_t nslots,
+                                                    TriRecord* __restrict__ tris, uint32_t n, int robust,
+                                                    float4* __restrict__ tri_box, uint32_t* err) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) refit_tri(geoms, slot_of, nslots, tris, i, robust, tri_box, err);
+}
+__global__ void __launch_bounds__(128) k_refit_level(const float4* tri_box, uint32_t num_tris,
+                                                     WideNode* __restrict__ nodes, uint32_t num_nodes,
+                                                     float* node_box, uint32_t begin, uint32_t end, double* sah_acc,
+                                                     uint32_t* err) {
+  const uint32_t k = begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 3);
+  double sah = 0.0, sahx = 0.0;
+  if (k < end && k < num_nodes)
+    refit_node_group(tri_box, num_tris, nodes, num_nodes, node_box, k, 0xFFu << (threadIdx.x & 24u), err, sah, sahx);
+  block_add2(sah, sahx, sah_acc);
 }
 
 cudaError_t refit_prepare(const GeomDesc* h_geoms, int ngeoms, const DeviceBVH& bvh, RefitScratch* out,
@@ -3380,37 +3361,120 @@ cudaError_t refit_prepare(const GeomDesc* h_geoms, int ngeoms, const DeviceBVH& 
   std::vector<uint32_t> slot_of(std::max(nslots, 1u), kInvalidID);
   for (int g = 0; g < ngeoms; g++) slot_of[h_geoms[g].geomID] = (uint32_t)g;
   out->nslots = (uint32_t)slot_of.size();
-  GB_CHECK(cudaMalloc(&out->d_geoms, sizeof(GeomDesc) * std::max(ngeoms, 1)));
-  GB_CHECK(cudaMalloc(&out->d_slot, sizeof(uint32_t) * slot_of.size()));
-  GB_CHECK(cudaMalloc(&out->d_err, sizeof(uint32_t)));
-  GB_CHECK(cudaMalloc(&out->node_box, sizeof(float) * 6 * bvh.num_nodes));
-  GB_CHECK(cudaMalloc(&out->tri_box, sizeof(float4) * 2 * std::max<size_t>(bvh.num_tris, 1)));
-  GB_CHECK(cudaMalloc(&out->d_sah, 2 * sizeof(double)));
-  GB_CHECK(cudaMemcpyAsync(out->d_geoms, h_geoms, sizeof(GeomDesc) * ngeoms, cudaMemcpyHostToDevice, st));
-  GB_CHECK(cudaMemcpyAsync(out->d_slot, slot_of.data(), sizeof(uint32_t) * slot_of.size(), cudaMemcpyHostToDevice, st));
-  GB_CHECK(cudaMemsetAsync(out->d_err, 0, sizeof(uint32_t), st));
-  return cudaStreamSynchronize(st);
+  out->ngeoms = ngeoms;
+  int per_sm = 0;
+  GB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_refit_all, 256, 0));
+  // enough CTAs for the triangles and the widest level, at most 4 per SM (a grid
+  // barrier costs more with every CTA)
+  uint64_t work = bvh.num_tris;
+  for (size_t l = 0; l + 1 < bvh.level_start.size(); l++)
+    work = std::max<uint64_t>(work, 8ull * (bvh.level_start[l + 1] - bvh.level_start[l]));
+  out->grid = std::min<uint32_t>(cdiv(work, 256), (uint32_t)std::max(1, std::min(per_sm, 4)) * (uint32_t)num_sms_build());
+  cudaError_t e = cudaMalloc(&out->d_geoms, sizeof(GeomDesc) * std::max(ngeoms, 1));
+  if (e == cudaSuccess) e = cudaMalloc(&out->d_slot, sizeof(uint32_t) * slot_of.size());
+  if (e == cudaSuccess) e = cudaMalloc(&out->result, sizeof(RefitResult) + sizeof(float) * 6 * (size_t)bvh.num_nodes);
+  if (e == cudaSuccess) e = cudaMalloc(&out->tri_box, sizeof(float4) * 2 * std::max<size_t>(bvh.num_tris, 1));
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(out->d_geoms, h_geoms, sizeof(GeomDesc) * ngeoms, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(out->d_slot, slot_of.data(), sizeof(uint32_t) * slot_of.size(), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(out->result, 0, sizeof(RefitResult), st);
+  if (e == cudaSuccess) e = cudaEventCreate(&out->e0);
+  if (e == cudaSuccess) e = cudaEventCreate(&out->e1);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) refit_release(out);
+  return e;
 }
 
 cudaError_t refit_enqueue(const DeviceBVH& bvh, const RefitScratch& s, cudaStream_t st) {
-  GB_CHECK(cudaMemsetAsync(s.d_sah, 0, 2 * sizeof(double), st));
+  RefitResult* r = s.result;
+  float* node_box = reinterpret_cast<float*>(r + 1);
+  GB_CHECK(cudaMemsetAsync(r->sah, 0, sizeof(r->sah), st));
+  const size_t nlevels = bvh.level_start.size() - 1;
+  if (nlevels <= (size_t)kColMaxLevels) {
+    RefitLevels lv{};
+    lv.n = (uint32_t)nlevels;
+    std::copy(bvh.level_start.begin(), bvh.level_start.end(), lv.start);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s.grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GB_CHECK(cudaLaunchKernelEx(&cfg, k_refit_all, (const GeomDesc*)s.d_geoms, (const uint32_t*)s.d_slot, s.nslots,
+                                bvh.tris, bvh.num_tris, bvh.robust, s.tri_box, bvh.nodes, bvh.num_nodes, node_box, lv,
+                                r->sah, reinterpret_cast<GridBarrier*>(r->bar), &r->bar[2], &r->err));
+    note_launches(1);
+    return cudaGetLastError();
+  }
   k_refit_tris<<<cdiv(bvh.num_tris, 256), 256, 0, st>>>(s.d_geoms, s.d_slot, s.nslots, bvh.tris, bvh.num_tris,
-                                                        bvh.robust, s.tri_box, s.d_err);
+                                                        bvh.robust, s.tri_box, &r->err);
   note_launches(1);
-  for (size_t l = bvh.level_start.size() - 1; l-- > 0;) {
+  for (size_t l = nlevels; l-- > 0;) {
     const uint32_t b = bvh.level_start[l], e = bvh.level_start[l + 1];
     if (e <= b) continue;
-    k_refit_level<<<cdiv(e - b, 128), 128, 0, st>>>(s.tri_box, bvh.num_tris, bvh.nodes, bvh.num_nodes, s.node_box, b,
-                                                   e, s.d_sah, s.d_err);
+    k_refit_level<<<cdiv(8ull * (e - b), 128), 128, 0, st>>>(s.tri_box, bvh.num_tris, bvh.nodes, bvh.num_nodes,
+                                                             node_box, b, e, r->sah, &r->err);
     note_launches(1);
   }
   return cudaGetLastError();
 }
 
+// The scratch of a scene's refits is kept in *s between commits: it is made for the
+// BVH of the last build (released when the scene is built again).
+cudaError_t refit_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, DeviceBVH* bvh, BuildStats* stats,
+                      bool* fallback, RefitScratch* s) {
+  *fallback = false;
+  if (bvh->num_nodes == 0 || bvh->level_start.size() < 2) {
+    *fallback = true;
+    return cudaSuccess;
+  }
+  if (!s->result) GB_CHECK(refit_prepare(h_geoms, ngeoms, *bvh, s, st));
+  if (s->ngeoms != ngeoms) return cudaErrorInvalidValue;
+  // buffers may have moved since the last commit
+  GB_CHECK(cudaMemcpyAsync(s->d_geoms, h_geoms, sizeof(GeomDesc) * ngeoms, cudaMemcpyHostToDevice, st));
+  GB_CHECK(cudaMemsetAsync(&s->result->err, 0, sizeof(uint32_t), st));
+  GB_CHECK(cudaEventRecord(s->e0, st));
+  GB_CHECK(refit_enqueue(*bvh, *s, st));
+  GB_CHECK(cudaEventRecord(s->e1, st));
+  struct {
+    RefitResult r;
+    float root[6];
+  } out;
+  static_assert(sizeof(out.r) + sizeof(out.root) <= sizeof(out), "result and root box in one copy");
+  GB_CHECK(cudaMemcpyAsync(&out, s->result, sizeof(out.r) + sizeof(out.root), cudaMemcpyDeviceToHost, st));
+  GB_CHECK(cudaStreamSynchronize(st));
+  float ms = 0;
+  cudaEventElapsedTime(&ms, s->e0, s->e1);
+  if (out.r.err) {  // a vertex became invalid or the records are inconsistent: rebuild
+    *fallback = true;
+    return cudaSuccess;
+  }
+  for (int d = 0; d < 3; d++) {
+    bvh->lo[d] = out.root[d];
+    bvh->hi[d] = out.root[3 + d];
+  }
+  const float gx = bvh->hi[0] - bvh->lo[0], gy = bvh->hi[1] - bvh->lo[1], gz = bvh->hi[2] - bvh->lo[2];
+  const double Aroot = std::max(0.0, (double)(gx * (gy + gz) + gy * gz));
+  stats->sah = Aroot > 0 ? (Aroot + out.r.sah[0]) / Aroot : 0.0;
+  stats->sah_exact = Aroot > 0 ? (Aroot + out.r.sah[1]) / Aroot : 0.0;
+  stats->build_ms = ms;
+  stats->num_nodes = bvh->num_nodes;
+  stats->num_prims = bvh->num_tris;
+  stats->depth = bvh->depth;
+  stats->refit = 1;
+  return cudaSuccess;
+}
+
 void refit_release(RefitScratch* s) {
-  void* ptrs[] = {s->d_geoms, s->d_slot, s->d_err, s->node_box, s->tri_box, s->d_sah};
+  void* ptrs[] = {s->d_geoms, s->d_slot, s->result, s->tri_box};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (s->e0) cudaEventDestroy(s->e0);
+  if (s->e1) cudaEventDestroy(s->e1);
   *s = RefitScratch{};
 }
 

@@ -13,30 +13,38 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
                       BuildStats* stats);
 void free_bvh(DeviceBVH* b);
 
-// Refits `bvh` in place to the geometries' current vertex positions (same
-// topology: the geometries, their triangles and indices are those of the
-// build).  Sets *fallback when a refit is impossible (e.g. a vertex became
-// invalid); the caller then rebuilds.  Synchronises `st`.
-cudaError_t refit_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, DeviceBVH* bvh, BuildStats* stats,
-                      bool* fallback);
-
 // Refit split for work captured in CUDA graphs: refit_prepare uploads the
 // geometry table once (synchronous); refit_enqueue only launches the refit
-// kernels on `st` (no allocation, no synchronisation; errors accumulate in
-// d_err until the caller reads it).  The BVH's host-side bounds are not updated.
+// kernel on `st` (no allocation, no synchronisation; errors accumulate in
+// result->err until the caller clears it).  The BVH's host-side bounds are not
+// updated.  A scratch belongs to the BVH it was prepared for.
+struct RefitResult {
+  double sah[2];         // SAH sums on the decoded and on the exact boxes
+  uint32_t err;          // kErr* bits
+  unsigned int bar[3];   // grid barrier (count, generation) and its own error word
+};
 struct RefitScratch {
   GeomDesc* d_geoms = nullptr;
   uint32_t* d_slot = nullptr;
   uint32_t nslots = 0;
-  uint32_t* d_err = nullptr;
-  float* node_box = nullptr;
-  float4* tri_box = nullptr;  // per-triangle boxes written by the triangle pass
-  double* d_sah = nullptr;  // SAH sums on the decoded and on the exact boxes
+  int ngeoms = 0;
+  uint32_t grid = 0;              // CTAs of the cooperative launch
+  RefitResult* result = nullptr;  // followed by the nodes' boxes (6 floats each)
+  float4* tri_box = nullptr;      // per-triangle boxes written by the triangle pass
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
 };
 cudaError_t refit_prepare(const GeomDesc* h_geoms, int ngeoms, const DeviceBVH& bvh, RefitScratch* out,
                           cudaStream_t st);
 cudaError_t refit_enqueue(const DeviceBVH& bvh, const RefitScratch& s, cudaStream_t st);
 void refit_release(RefitScratch* s);
+
+// Refits `bvh` in place to the geometries' current vertex positions (same
+// topology: the geometries, their triangles and indices are those of the
+// build).  Sets *fallback when a refit is impossible (e.g. a vertex became
+// invalid); the caller then rebuilds.  *scratch is prepared at the first refit of
+// a BVH and kept by the caller for the next ones.  Synchronises `st`.
+cudaError_t refit_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, DeviceBVH* bvh, BuildStats* stats,
+                      bool* fallback, RefitScratch* scratch);
 
 // A build that runs without host reads, so that it can be captured into a
 // CUDA graph and replayed: every buffer is allocated up front, and the loops

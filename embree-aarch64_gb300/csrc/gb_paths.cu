@@ -228,7 +228,7 @@ struct FrameBody {
                                                         anim.nverts, rest, frame, anim.amplitude, anim.seed);
       nk++;
       GB_TRY(refit_enqueue(*bvh, *refit, st));
-      nk += (unsigned)bvh->level_start.size();  // tris + one per level (upper bound)
+      nk++;  // one cooperative launch (BVHs of more than 64 levels: one per level)
     }
     GB_TRY(cudaMemsetAsync(counts, 0, (kMaxBounces + 1) * sizeof(uint32_t), st));
     GB_TRY(cudaMemsetAsync(scratch + 1, 0, 9 * sizeof(uint32_t), st));  // error flags and counters
@@ -314,7 +314,7 @@ cudaError_t PathTracer::render(uint32_t frame, bool learned, cudaStream_t st, Fr
   uint32_t* h = h_frame_ + 1;  // pinned: [0..8] counts, [9..24] scratch, [25] refit errors
   GB_TRY(cudaMemcpyAsync(h, counts_, (kMaxBounces + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   GB_TRY(cudaMemcpyAsync(h + 9, scratch_, 10 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  if (animated_) GB_TRY(cudaMemcpyAsync(h + 19, refit_->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  if (animated_) GB_TRY(cudaMemcpyAsync(h + 19, &refit_->result->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   GB_TRY(cudaStreamSynchronize(st));
   float ms = 0;
   cudaEventElapsedTime(&ms, ev_[0], ev_[1]);

@@ -525,6 +525,7 @@ struct Scene : RefCounted {
   // host-driven build and, once the scene was built twice with that layout, the graph
   std::vector<uint64_t> layout_key;
   gb::CachedBuild* gcache = nullptr;
+  gb::RefitScratch refit;     // refits of the current BVH (made at the first one)
   uint64_t build_serial = 0;  // counts full builds (a refit keeps the BVH's structure)
   std::vector<gb::GeomDesc> descs;  // geometry table of the committed BVH (device buffers)
   bool batched = false;             // rtcgbSetSceneBatched: one tree per geometry
@@ -554,6 +555,7 @@ struct Scene : RefCounted {
     drop_instances();
     if (d_roots) cudaFree(d_roots);
     gb::free_bvh(&bvh);
+    gb::refit_release(&refit);
     gb::cached_build_release(gcache);
     device->dec();
   }
@@ -700,7 +702,8 @@ struct Scene : RefCounted {
     if (committed && all_refit && bvh.num_nodes > 0 && sig == built_sig && robust == built_robust) {
       gb::BuildStats bs = stats;
       bool fallback = false;
-      cuda_ok(gb::refit_bvh(descs.data(), (int)descs.size(), st, &bvh, &bs, &fallback), "rtcCommitScene (refit)");
+      cuda_ok(gb::refit_bvh(descs.data(), (int)descs.size(), st, &bvh, &bs, &fallback, &refit),
+              "rtcCommitScene (refit)");
       if (!fallback) {
         stats = bs;
         this->descs = descs;
@@ -713,6 +716,7 @@ struct Scene : RefCounted {
     // estimated device bytes of the build (scratch + result)
     device->memory((ssize_t)(total * 256 + 4096), false);
     gb::free_bvh(&bvh);
+    gb::refit_release(&refit);
     committed = false;
     gb::BuildStats bs;
     gb::BuildOptions opt = device->build_opt;
