@@ -55,6 +55,7 @@ cudaError_t refit_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, Devi
 // levels (the replay checks that they still suffice and flags it otherwise).
 // The BVH stays in the build's own node and triangle arrays (sized for the
 // maximum), with the roots of the segments in seg_index.
+struct GraphBuildOut;
 struct GraphBuildPlan {
   uint32_t valid_tris = 0;   // valid triangles of the ordinary build
   uint32_t roots = 0;        // non-empty segments (1 without segments)
@@ -82,7 +83,8 @@ struct GraphBuild {
   TriRecord* tris = nullptr;
   uint32_t *items[2] = {nullptr, nullptr}, *kids = nullptr, *nint = nullptr, *ntri = nullptr, *leaf_root = nullptr;
   double* d_sah = nullptr;
-  uint32_t *d_leaves = nullptr, *cstate = nullptr, *seg_index = nullptr, *status = nullptr;
+  uint32_t *d_leaves = nullptr, *cstate = nullptr, *seg_index = nullptr;
+  GraphBuildOut* out = nullptr;                         // results (page-locked host memory)
   uint32_t col_grid = 0;                                // CTAs of the cooperative collapse
   uint32_t *col_sums = nullptr, *col_bar = nullptr;     // its per-CTA sums and grid barrier
   TriRecord* prec = nullptr;                            // leaf records in primitive order
@@ -124,6 +126,7 @@ struct CachedBuild {
 cudaError_t cached_build_create(const GeomDesc* h_geoms, int ngeoms, const BuildOptions& opt,
                                 const GraphBuildPlan& plan, cudaStream_t st, CachedBuild** out);
 // Replays it for the geometries `h_geoms` (same layout; buffers may have moved).
+// *out refers to the build's own arrays until the next replay or release.
 // cudaErrorNotReady: the replayed build does not match the plan (e.g. a different
 // number of valid triangles); the caller builds the ordinary way.
 cudaError_t cached_build_run(CachedBuild* c, const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, DeviceBVH* out,

@@ -106,6 +106,7 @@ constexpr uint32_t kInstanceLeaf = 1u;
 struct DeviceBVH {
   WideNode* nodes = nullptr;
   TriRecord* tris = nullptr;
+  bool borrowed = false;     // nodes and tris belong to the scene's captured build
   uint32_t num_nodes = 0;
   uint32_t num_tris = 0;     // valid primitives in the BVH
   uint32_t depth = 0;        // wide levels

@@ -52,7 +52,14 @@ struct TraceParams {
   const uint32_t* excl_off;
   const uint2* excl;
   int shape;                  // index into kTraceShapes (0: default)
+  // optional: the last CTA copies the state words (ray_counter[0..9]: fetch counter,
+  // error flags, counters) to host_state, page-locked host memory, and zeroes them
+  // and *done, so that the next launch on the same state needs no memset and the
+  // host no copy.  All zero before the launch.
+  unsigned int* done;
+  unsigned int* host_state;
 };
+constexpr int kStateWords = 10;  // fetch counter, error flags, TraceCounters
 
 // Launches the persistent closest-hit (anyhit = false) or any-hit kernel.
 // P.shape selects the launch shape of the plain kernels on 16-byte aligned

@@ -823,6 +823,17 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
       atomicAdd(&P.counters->rays, n_rays);
     }
   }
+  if (P.done) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(P.done, 1u) == gridDim.x - 1) {
+        __threadfence();
+        for (int i = 0; i < kStateWords; i++) P.host_state[i] = atomicExch(P.ray_counter + i, 0u);
+        *P.done = 0u;
+      }
+    }
+  }
 }
 
 

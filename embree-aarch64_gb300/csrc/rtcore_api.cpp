@@ -399,7 +399,8 @@ struct ThreadCtx {
   bool user_set = false;
   char* dbuf = nullptr;
   size_t cap = 0;
-  unsigned int* dscratch = nullptr;     // [0] ray counter, [1] error flags, [2..] counters
+  unsigned int* dscratch = nullptr;     // [0] ray counter, [1] error flags, [2..9] counters, [12] finished CTAs
+  bool scratch_zero = false;            // the scratch is all zero (left so by the last launch)
   unsigned int* hscratch = nullptr;     // pinned mirror
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
   static constexpr int kMaxChunks = 32;
@@ -421,6 +422,7 @@ struct ThreadCtx {
     if (device == dev && dscratch) return;
     device = dev;
     cuda_ok(cudaMalloc((void**)&dscratch, 64), "cudaMalloc scratch");
+    scratch_zero = false;
     cuda_ok(cudaMallocHost((void**)&hscratch, 64), "cudaMallocHost");
     cuda_ok(cudaEventCreate(&e0), "event");
     cuda_ok(cudaEventCreate(&e1), "event");
@@ -931,6 +933,7 @@ void run_filtered(Scene* scene, const RTCIntersectContext* uctx, void* rays, uns
     P.robust = bvh.robust;
     P.excl_off = reinterpret_cast<const uint32_t*>(d + b_work);
     P.excl = reinterpret_cast<const uint2*>(d + b_work + b_off);
+    c.scratch_zero = false;
     cuda_ok(cudaMemsetAsync(c.dscratch, 0, 64, st), "memset");
     cuda_ok(cudaEventRecord(c.e1, st), "event");
     cuda_ok(gb::launch_trace(P, false, false, st), "traversal launch");
@@ -1089,9 +1092,16 @@ void run_query(Scene* scene, void* rays, unsigned M, size_t stride, bool anyhit,
     P.batch_root = scene->d_roots;
     P.nbatches = batch->nbatches;
   }
-  cuda_ok(cudaEventRecord(c.e0, st), "event");
-  cuda_ok(cudaMemsetAsync(c.dscratch, 0, 64, st), "memset");
-  unsigned launches = 1;
+  // device rays and host rays traced in place: the kernel itself reports its state
+  // and leaves the scratch zero, so the call is one launch between two events
+  const bool reports = on_device || direct;
+  if (!reports) cuda_ok(cudaEventRecord(c.e0, st), "event");
+  unsigned launches = 0;
+  if (!reports || !c.scratch_zero) {
+    cuda_ok(cudaMemsetAsync(c.dscratch, 0, 64, st), "memset");
+    launches++;
+  }
+  c.scratch_zero = false;
   const uint32_t kChunk = 1u << 21;  // rays per pipeline stage
   // ray reordering (gpu.reorder=1): fetch order by direction octant and origin Morton code
   auto reorder = [&](gb::TraceParams& Pq) {
@@ -1121,9 +1131,11 @@ void run_query(Scene* scene, void* rays, unsigned M, size_t stride, bool anyhit,
     prop = nullptr;
     prop_lock = std::unique_lock<std::mutex>();
   }
-  if (on_device || direct) {
+  if (reports) {
     P.rays = (char*)rays;
     P.nrays = M;
+    P.done = c.dscratch + 12;
+    P.host_state = c.hscratch;
     cuda_ok(cudaEventRecord(c.e1, st), "event");
     reorder(P);
     propose(P);
@@ -1184,12 +1196,16 @@ void run_query(Scene* scene, void* rays, unsigned M, size_t stride, bool anyhit,
     c.last.d2h_bytes = span;
   }
   gb::note_launches(launches);
-  cuda_ok(cudaMemcpyAsync(c.hscratch, c.dscratch, 64, cudaMemcpyDeviceToHost, st), "D2H status");
-  cuda_ok(cudaEventRecord(c.e3, st), "event");
+  if (!reports) {
+    cuda_ok(cudaMemcpyAsync(c.hscratch, c.dscratch, 64, cudaMemcpyDeviceToHost, st), "D2H status");
+    cuda_ok(cudaEventRecord(c.e3, st), "event");
+  }
   cuda_ok(cudaStreamSynchronize(st), "traversal");
+  c.scratch_zero = reports;
   float k_ms = 0, t_ms = 0;
   cudaEventElapsedTime(&k_ms, c.e1, c.e2);
-  cudaEventElapsedTime(&t_ms, c.e0, c.e3);
+  if (reports) t_ms = k_ms;
+  else cudaEventElapsedTime(&t_ms, c.e0, c.e3);
   c.last.kernel_ms = k_ms;
   c.last.total_ms = t_ms;
   const gb::TraceCounters* tc = reinterpret_cast<const gb::TraceCounters*>(c.hscratch + 2);
@@ -2390,6 +2406,7 @@ RTC_API void rtcgbProposerPredict(RTCGBProposer hp, const struct RTCRay* rays, u
   DevSpan in(rays, (size_t)(M - 1) * byteStride + sizeof(RTCRay), st, true);
   DevSpan out(treelets, (size_t)M * 16, st, false);
   t_ctx.ensure(p->scene->device->cuda_device);
+  t_ctx.scratch_zero = false;
   cuda_ok(cudaMemsetAsync(t_ctx.dscratch + 1, 0, sizeof(uint32_t), st), "memset");
   cuda_ok(p->net.predict(in.d, byteStride, M, nullptr, (uint32_t*)out.d, st, nullptr, t_ctx.dscratch + 1),
           "proposer inference");
