@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
@@ -770,39 +771,31 @@ __device__ __forceinline__ void dp_node(float4* cost, uint2* choice, uint32_t n,
 // Grid barrier of the cooperative build kernels (all CTAs resident).
 struct GridBarrier {
   unsigned int count;
-  unsigned int gen;
 };
 
-// Barrier over all CTAs of a cooperative launch; every thread calls it.  A CTA
-// that waits for more than kLbSpinLimit re-reads (a CTA missing) sets kErrBuild
-// in *err; a CTA that finds *err set does not wait.  Returns false once *err
-// is set, so the grid leaves its loop.
+// Barrier over all CTAs of a cooperative launch; every thread calls it.  b->count
+// is zero before the launch (a barrier adds gridDim.x to it).  A CTA that waits for
+// more than kLbSpinLimit re-reads (a CTA missing) sets kErrBuild in *err; false
+// once *err is set, so the grid leaves its loop.  A build waits at about 70 of
+// these and a refit at 12, so their latency counts: one arriving atomic and reads of
+// the same word between two acquire-release fences take 1.5 us over 456 CTAs;
+// a separate generation word, sequentially consistent fences and sleeping between
+// the reads took 2.3 us.
 __device__ __forceinline__ bool grid_sync(GridBarrier* b, unsigned int* err) {
   __shared__ bool s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    bool ok = lb_load(err) == 0u;
-    if (ok) {
-      const unsigned int g = lb_load(&b->gen);
-      __threadfence();
-      if (atomicAdd(&b->count, 1u) == gridDim.x - 1) {
-        lb_store(&b->count, 0u);
-        __threadfence();
-        atomicAdd(&b->gen, 1u);
-      } else {
-        uint32_t it = 0;
-        while (lb_load(&b->gen) == g && it < kLbSpinLimit) {
-          __nanosleep(64);
-          it++;
-        }
-        if (it == kLbSpinLimit) {
-          atomicOr(err, kErrBuild);
-          ok = false;
-        }
-      }
-      __threadfence();
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    const unsigned int ticket = atomicAdd(&b->count, 1u);
+    const unsigned int target = (ticket / gridDim.x + 1u) * gridDim.x;
+    uint32_t it = 0, e = lb_load(err);
+    while (lb_load(&b->count) < target && e == 0u && it < kLbSpinLimit) {
+      e = lb_load(err);
+      it++;
     }
-    s_ok = ok;
+    if (it == kLbSpinLimit) atomicOr(err, kErrBuild);
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    s_ok = e == 0u && it < kLbSpinLimit;
   }
   __syncthreads();
   return s_ok;
@@ -1527,6 +1520,96 @@ __device__ int gather_children(const BinTree& t, uint32_t b, uint32_t kids[8]) {
   return nk;
 }
 
+// The same by 8 lanes: lane group lane & ~7 of the warp handles binary node b (all
+// 32 lanes call it; `have` is the group's).  An entry (n, i) -- node n may take up to
+// i slots -- lives in the lane where its slots begin; a split keeps the right child
+// there and sends the left child to the lane behind the right child's slots, so
+// the children come out in the order of the serial form (right subtrees first)
+// and a wide node takes as many dependent reads as its binary subtree is deep,
+// not as it has nodes.  A live lane returns its child in `kid`; live: the group's live lanes.
+__device__ __forceinline__ void gather_group(const BinTree& t, uint32_t b, bool have, uint32_t& kid, uint32_t& live) {
+  const uint32_t s = threadIdx.x & 7u, gshift = threadIdx.x & 24u;
+  uint32_t n = kInvalidID, i = 0;
+  if (have) {
+    if (bt_leaf(t, b)) {
+      if (s == 0) n = b, i = 1;
+    } else {
+      const uint32_t k8 = min(max(t.choice[b].x & 0xFFu, 1u), 7u);  // split of D(b, 8)
+      const uint32_t l = bt_left(t, b), r = bt_right(t, b);
+      if (s == 0) n = r, i = 8u - k8;
+      if (s == 8u - k8) n = l, i = k8;
+    }
+  }
+  for (;;) {
+    bool split = false;
+    uint32_t k = 0, left = 0, right = 0;
+    if (i > 1u) {
+      if (bt_leaf(t, n)) {
+        i = 1;
+      } else {
+        const uint2 ch = t.choice[n];
+        left = bt_left(t, n);
+        right = bt_right(t, n);
+        for (; i > 1u; i--) {
+          k = ((i - 1u < 4u ? ch.x : ch.y) >> (8u * ((i - 1u) & 3u))) & 0xFFu;
+          if (k != 0u) break;
+        }
+        split = i > 1u;
+        k = min(k, i - 1u);
+      }
+    }
+    live = __ballot_sync(0xFFFFFFFFu, i > 0u) >> gshift & 0xFFu;
+    if (!__any_sync(0xFFFFFFFFu, split)) break;
+    const uint32_t dst = split ? s + i - k : 8u;
+    const uint32_t below = live & ((1u << s) - 1u);
+    const int src = below ? 31 - __clz(below) : 0;  // the entry whose slots this lane may lie in
+    const uint32_t d2 = __shfl_sync(0xFFFFFFFFu, dst, src, 8), k2 = __shfl_sync(0xFFFFFFFFu, k, src, 8);
+    const uint32_t l2 = __shfl_sync(0xFFFFFFFFu, left, src, 8);
+    if (split) {
+      n = right;
+      i -= k;
+    } else if (i == 0u && below && d2 == s) {
+      n = l2;
+      i = k2;
+    }
+  }
+  kid = n;
+}
+
+// Children and counts of item k of a level (all 32 lanes call it): kids[8k ..] =
+// its children, *ni internal ones, *nt triangles in leaf children.
+__device__ __forceinline__ void collapse_count_group(const BinTree& t, const uint32_t* __restrict__ items, uint32_t k,
+                                                     bool have, uint32_t* __restrict__ kids, uint32_t* ni,
+                                                     uint32_t* nt) {
+  const uint32_t s = threadIdx.x & 7u, gshift = threadIdx.x & 24u;
+  uint32_t kid = kInvalidID, live = 0;
+  if (t.choice) {
+    gather_group(t, have ? items[k] : 0u, have, kid, live);
+  } else {  // greedy: one lane gathers
+    uint32_t kk[8];
+    const int nk = have && s == 0u ? gather_children(t, items[k], kk) : 0;
+    live = (1u << __shfl_sync(0xFFFFFFFFu, nk, 0, 8)) - 1u;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const uint32_t c = __shfl_sync(0xFFFFFFFFu, j < nk ? kk[j] : kInvalidID, 0, 8);
+      if ((uint32_t)j == s) kid = c;
+    }
+  }
+  const uint32_t nk = __popc(live);
+  const bool mine = live >> s & 1u;
+  uint32_t cnt = mine ? bt_cnt(t, kid) : 0u;
+  const bool inner = cnt > t.leaf_max;
+  *ni = __popc(__ballot_sync(0xFFFFFFFFu, inner) >> gshift & 0xFFu);
+  if (inner) cnt = 0;
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o, 8);
+  *nt = cnt;
+  if (have) {
+    if (mine) kids[8 * (size_t)k + __popc(live & ((1u << s) - 1u))] = kid;
+    if (s >= nk) kids[8 * (size_t)k + s] = 0xFFFFFFFFu;
+  }
+}
+
 // The collapse runs level by level from a state in device memory, so levels
 // can be enqueued (or captured) before their sizes are known: [kColN] items of
 // the current level, [kColBase] its first wide node, [kColTri] its first
@@ -1612,22 +1695,14 @@ __global__ void __launch_bounds__(128) k_collapse_count(BinTree t, const ColItem
                                                         uint32_t* __restrict__ ntri) {
   const uint32_t nitems = cstate[kColN];
   const uint32_t* __restrict__ items = ci.items[cstate[kColDepth] & 1u];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nitems; k += gridDim.x * blockDim.x) {
-    uint32_t kids[8];
-    const int nk = gather_children(t, items[k], kids);
-    uint32_t ni = 0, nt = 0;
-    for (int i = 0; i < 8; i++) {
-      if (i < nk) {
-        const uint32_t c = kids[i];
-        const uint32_t cnt = bt_cnt(t, c);
-        if (cnt > t.leaf_max) ni++; else nt += cnt;
-        kids_out[8 * (size_t)k + i] = c;
-      } else {
-        kids_out[8 * (size_t)k + i] = 0xFFFFFFFFu;
-      }
+  for (uint32_t k0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 3; k0 < nitems; k0 += (gridDim.x * blockDim.x) >> 3) {
+    const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
+    uint32_t ni, nt;
+    collapse_count_group(t, items, k, k < nitems, kids_out, &ni, &nt);
+    if (k < nitems && (threadIdx.x & 7u) == 0u) {
+      nint[k] = ni;
+      ntri[k] = nt;
     }
-    nint[k] = ni;
-    ntri[k] = nt;
   }
 }
 
@@ -1693,205 +1768,63 @@ __device__ __forceinline__ void write_tri(const GeomDesc* __restrict__ geoms, co
   dst->c = make_float4(e2.x, e2.y, e2.z, 0.f);
 }
 
-// Writes wide node k of the level and the triangle records of its leaves;
-// adds the node's SAH terms and leaf count to sah_out / nleaf_out.
+// Shared memory of the lane groups that emit wide nodes: the slot auction and the
+// node's words.
+template <int GROUPS>
+struct EmitSmem {
+  unsigned long long key[GROUPS][8];
+  alignas(16) uint32_t node[GROUPS][sizeof(WideNode) / 4];
+};
 
-// The wide node of item k by one thread: wide levels (more items than there
-// are lane groups to share them) are throughput-bound, and this form does the
-// least work per node; collapse_emit_group gives the same node.
-__device__ __forceinline__ void collapse_emit_node(
-    const BinTree& t, const uint32_t* __restrict__ kids_in, uint32_t k, const uint32_t* __restrict__ off_int,
-    const uint32_t* __restrict__ off_tri, uint32_t level_base, uint32_t next_base, uint32_t tri_next,
-    WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root, uint32_t* __restrict__ next_items,
-    uint32_t node_cap, uint32_t tri_cap, uint32_t* err, double& sah_out, double& sahx_out, uint32_t& nleaf_out) {
-  // all loops over the 8 children are unrolled, so the per-child values stay
-  // in registers (no local-memory arrays)
-  uint32_t kids[8];
-  int nk = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    kids[i] = kids_in[8 * (size_t)k + i];
-    if (kids[i] != 0xFFFFFFFFu) nk = i + 1;
-  }
-  // union box and quantisation frame
-  float3 klo[8], khi[8];
-  float3 ulo = make_float3(INFINITY, INFINITY, INFINITY), uhi = make_float3(-INFINITY, -INFINITY, -INFINITY);
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    klo[i] = khi[i] = make_float3(0.f, 0.f, 0.f);
-    if (i < nk) {
-      klo[i] = bt_lo(t, kids[i]);
-      khi[i] = bt_hi(t, kids[i]);
-      ulo = f3min(ulo, klo[i]);
-      uhi = f3max(uhi, khi[i]);
-    }
-  }
-  const uint32_t Ex = exp_for(__fsub_ru(uhi.x, ulo.x));
-  const uint32_t Ey = exp_for(__fsub_ru(uhi.y, ulo.y));
-  const uint32_t Ez = exp_for(__fsub_ru(uhi.z, ulo.z));
-  const float sx = __uint_as_float(Ex << 23), sy = __uint_as_float(Ey << 23), sz = __uint_as_float(Ez << 23);
-  const float ix = __uint_as_float((254u - Ex) << 23), iy = __uint_as_float((254u - Ey) << 23),
-              iz = __uint_as_float((254u - Ez) << 23);
-  // slot assignment: slot s prefers children far along the octant direction
-  // with sign bits s (bit set = negative axis), so that visiting slots in
-  // ascending order of (slot ^ ray octant) is roughly near-to-far.
-  const float3 pc = make_float3((ulo.x + uhi.x) * 0.5f, (ulo.y + uhi.y) * 0.5f, (ulo.z + uhi.z) * 0.5f);
-  float dx[8], dy[8], dz[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    dx[i] = (klo[i].x + khi[i].x) * 0.5f - pc.x;
-    dy[i] = (klo[i].y + khi[i].y) * 0.5f - pc.y;
-    dz[i] = (klo[i].z + khi[i].z) * 0.5f - pc.z;
-  }
-  // greedy: repeatedly the cheapest (child, free slot) pair, cost = the child's
-  // offset from the node centre along the slot's octant direction
-  uint32_t used = 0, assigned = 0;
-  uint32_t kid_at = 0xFFFFFFFFu;  // 4 bits per slot: child index, 0xF = empty
-  for (int it = 0; it < nk; it++) {
-    float bc = INFINITY;
-    int bi = -1, bs = -1;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      if (i >= nk || (assigned >> i & 1)) continue;
-#pragma unroll
-      for (int s = 0; s < 8; s++) {
-        if (used >> s & 1) continue;
-        const float c = ((s & 1) ? -dx[i] : dx[i]) + ((s & 2) ? -dy[i] : dy[i]) + ((s & 4) ? -dz[i] : dz[i]);
-        if (bi < 0 || c < bc) { bc = c; bi = i; bs = s; }
-      }
-    }
-    assigned |= 1u << bi;
-    used |= 1u << bs;
-    kid_at = (kid_at & ~(0xFu << (4 * bs))) | ((uint32_t)bi << (4 * bs));
-  }
-
-  WideNode node;
-  node.px = ulo.x;
-  node.py = ulo.y;
-  node.pz = ulo.z;
-  node.ex = (uint8_t)Ex;
-  node.ey = (uint8_t)Ey;
-  node.ez = (uint8_t)Ez;
-  node.imask = 0;
-  node.sx = sx * 32768.0f;
-  node.sy = sy * 32768.0f;
-  node.sz = sz * 32768.0f;
-  node.pad = 0;
-  node.child_base = next_base + off_int[k];
-  node.tri_base = tri_next + off_tri[k];
-  uint32_t int_rank = 0, tri_off = 0;
-  double sah = 0.0, sahx = 0.0;  // on the decoded (quantised) and on the exact boxes
-  uint32_t nleaf = 0;
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    const uint32_t i = (kid_at >> (4 * s)) & 0xFu;
-    if (i == 0xFu) {
-      node.meta[s] = 0;
-      node.qlo_x[s] = node.qlo_y[s] = node.qlo_z[s] = 255;
-      node.qhi_x[s] = node.qhi_y[s] = node.qhi_z[s] = 0;
-      continue;
-    }
-    uint32_t c = 0;
-    float3 a = make_float3(0.f, 0.f, 0.f), b = a;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      if ((uint32_t)j == i) {
-        c = kids[j];
-        a = klo[j];
-        b = khi[j];
-      }
-    }
-    const float qlx = fminf(fmaxf(floorf(__fsub_rd(a.x, ulo.x) * ix), 0.f), 255.f);
-    const float qly = fminf(fmaxf(floorf(__fsub_rd(a.y, ulo.y) * iy), 0.f), 255.f);
-    const float qlz = fminf(fmaxf(floorf(__fsub_rd(a.z, ulo.z) * iz), 0.f), 255.f);
-    const float qhx = fminf(fmaxf(ceilf(__fsub_ru(b.x, ulo.x) * ix), 0.f), 255.f);
-    const float qhy = fminf(fmaxf(ceilf(__fsub_ru(b.y, ulo.y) * iy), 0.f), 255.f);
-    const float qhz = fminf(fmaxf(ceilf(__fsub_ru(b.z, ulo.z) * iz), 0.f), 255.f);
-    node.qlo_x[s] = (uint8_t)qlx; node.qlo_y[s] = (uint8_t)qly; node.qlo_z[s] = (uint8_t)qlz;
-    node.qhi_x[s] = (uint8_t)qhx; node.qhi_y[s] = (uint8_t)qhy; node.qhi_z[s] = (uint8_t)qhz;
-    // decoded (outward-rounded) box, as traversal sees it
-    const float3 dlo = make_float3(__fmaf_rd(qlx, sx, ulo.x), __fmaf_rd(qly, sy, ulo.y), __fmaf_rd(qlz, sz, ulo.z));
-    const float3 dhi = make_float3(__fmaf_ru(qhx, sx, ulo.x), __fmaf_ru(qhy, sy, ulo.y), __fmaf_ru(qhz, sz, ulo.z));
-    const double A = (double)fmaxf(0.f, half_area(dlo, dhi));
-    const double Ax = (double)fmaxf(0.f, half_area(a, b));
-    const uint32_t cnt = bt_cnt(t, c);
-    if (cnt > t.leaf_max) {
-      node.meta[s] = (uint8_t)(0x80u | (uint32_t)s);
-      node.imask |= (uint8_t)(1u << s);
-      if (off_int[k] + int_rank >= node_cap || node.child_base + int_rank >= node_cap) {
-        atomicOr(err, kErrBuild);
-        return;
-      }
-      next_items[off_int[k] + int_rank] = c;
-      int_rank++;
-      sah += A;  // inner node term
-      sahx += Ax;
-    } else {
-      node.meta[s] = (uint8_t)(0x80u | ((cnt - 1u) << 5) | tri_off);
-      // the leaf's triangle records are written after the last level by
-      // k_write_leaves, one thread per leaf: here only its binary subtree is
-      // recorded at the slot of its first triangle
-      if (node.tri_base + tri_off + cnt > tri_cap) {
-        atomicOr(err, kErrBuild);
-        return;
-      }
-      leaf_root[node.tri_base + tri_off] = cnt == 1 ? bt_right(t, c) | kLeafPrim : c;
-      tri_off += cnt;
-      sah += A * (double)((cnt + 3) / 4);  // leaf term: area x Triangle4 blocks
-      sahx += Ax * (double)((cnt + 3) / 4);
-      nleaf++;
-    }
-  }
-  if (level_base + k >= node_cap) {
-    atomicOr(err, kErrBuild);
-    return;
-  }
-  nodes[level_base + k] = node;
-  sah_out = sah;
-  sahx_out = sahx;
-  nleaf_out = nleaf;
-}
-
-// The wide node of item k, built by the 8 lanes of a lane group (lane & 7 is
-// the child index; all 8 lanes call it with the same k; gmask names them).
-// Children are placed in slots greedily, the cheapest (child, free slot) pair
-// first with ties to the lower child and then the lower slot, the cost being
-// the child's offset from the node centre along the slot's octant direction
-// (slot s prefers children far along the direction with sign bits s), so that
-// visiting slots in ascending order of (slot ^ ray octant) is roughly
-// near-to-far.  Planes are quantised outward, internal children are numbered
-// and leaf triangles laid out in slot order.
+// The wide node of item k, built by the 8 lanes of a lane group (lane & 7 is the
+// child index; all 32 lanes call it, `have` is the group's; g: the group's index in
+// the CTA).  Children are placed in slots greedily, the cheapest (child, free slot)
+// pair first with ties to the lower child and then the lower slot, the cost being
+// the child's offset from the node centre along the slot's octant direction (slot s
+// prefers children far along the direction with sign bits s), so that visiting
+// slots in ascending order of (slot ^ ray octant) is roughly near-to-far.  One
+// order of all pairs ranks the slots for every child and the children for every
+// slot, so the greedy choice is the stable assignment, which rounds of offers
+// find: every unplaced child offers for its best slot that has not turned it
+// away, a slot keeps its best offer (3-4 rounds where the greedy form took one
+// per child).  Planes are quantised outward, internal children are numbered and
+// leaf triangles laid out in slot order.
+template <int GROUPS>
 __device__ __forceinline__ void collapse_emit_group(
-    const BinTree& t, const uint32_t* __restrict__ kids_in, uint32_t k, const uint32_t* __restrict__ off_int,
-    const uint32_t* __restrict__ off_tri, uint32_t level_base, uint32_t next_base, uint32_t tri_next,
-    WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root, uint32_t* __restrict__ next_items,
-    uint32_t node_cap, uint32_t tri_cap, uint32_t* err, uint32_t gmask, double& sah_out, double& sahx_out,
-    uint32_t& nleaf_out) {
+    const BinTree& t, const uint32_t* __restrict__ kids_in, uint32_t k, bool have, uint32_t g, EmitSmem<GROUPS>& sm,
+    const uint32_t* __restrict__ off_int, const uint32_t* __restrict__ off_tri, uint32_t level_base,
+    uint32_t next_base, uint32_t tri_next, WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root,
+    uint32_t* __restrict__ next_items, uint32_t node_cap, uint32_t tri_cap, uint32_t* err, double& sah_out,
+    double& sahx_out, uint32_t& nleaf_out) {
   const uint32_t i = threadIdx.x & 7u;
-  const uint32_t kid = kids_in[8 * (size_t)k + i];
+  const uint32_t kid = have ? kids_in[8 * (size_t)k + i] : 0xFFFFFFFFu;
   const bool valid = kid != 0xFFFFFFFFu;
-  const uint32_t vmask = __ballot_sync(gmask, valid) >> (threadIdx.x & 24u) & 0xFFu;
-  const int nk = __popc(vmask);
   float3 lo = make_float3(0.f, 0.f, 0.f), hi = lo;
+  uint32_t prim = 0;  // a leaf node's primitive
   if (valid) {
-    lo = bt_lo(t, kid);
-    hi = bt_hi(t, kid);
+    const float4 a = t.lo[kid], b = t.hi[kid];
+    lo = make_float3(a.x, a.y, a.z);
+    hi = make_float3(b.x, b.y, b.z);
+    prim = __float_as_uint(b.w);
   }
+  uint32_t cnt = valid ? bt_cnt(t, kid) : 0u;
+  const uint32_t oi = have ? off_int[k] : 0u, ot = have ? off_tri[k] : 0u;
   // union box and quantisation frame
   float3 ulo = valid ? lo : make_float3(INFINITY, INFINITY, INFINITY);
   float3 uhi = valid ? hi : make_float3(-INFINITY, -INFINITY, -INFINITY);
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) {
-    ulo.x = fminf(ulo.x, __shfl_xor_sync(gmask, ulo.x, o, 8));
-    ulo.y = fminf(ulo.y, __shfl_xor_sync(gmask, ulo.y, o, 8));
-    ulo.z = fminf(ulo.z, __shfl_xor_sync(gmask, ulo.z, o, 8));
-    uhi.x = fmaxf(uhi.x, __shfl_xor_sync(gmask, uhi.x, o, 8));
-    uhi.y = fmaxf(uhi.y, __shfl_xor_sync(gmask, uhi.y, o, 8));
-    uhi.z = fmaxf(uhi.z, __shfl_xor_sync(gmask, uhi.z, o, 8));
+    ulo.x = fminf(ulo.x, __shfl_xor_sync(0xFFFFFFFFu, ulo.x, o));
+    ulo.y = fminf(ulo.y, __shfl_xor_sync(0xFFFFFFFFu, ulo.y, o));
+    ulo.z = fminf(ulo.z, __shfl_xor_sync(0xFFFFFFFFu, ulo.z, o));
+    uhi.x = fmaxf(uhi.x, __shfl_xor_sync(0xFFFFFFFFu, uhi.x, o));
+    uhi.y = fmaxf(uhi.y, __shfl_xor_sync(0xFFFFFFFFu, uhi.y, o));
+    uhi.z = fmaxf(uhi.z, __shfl_xor_sync(0xFFFFFFFFu, uhi.z, o));
   }
-  const uint32_t Ex = exp_for(__fsub_ru(uhi.x, ulo.x));
-  const uint32_t Ey = exp_for(__fsub_ru(uhi.y, ulo.y));
-  const uint32_t Ez = exp_for(__fsub_ru(uhi.z, ulo.z));
+  // one axis' exponent per lane
+  const uint32_t Ea = exp_for(i == 0u ? __fsub_ru(uhi.x, ulo.x) : i == 1u ? __fsub_ru(uhi.y, ulo.y) : __fsub_ru(uhi.z, ulo.z));
+  const uint32_t Ex = __shfl_sync(0xFFFFFFFFu, Ea, 0, 8), Ey = __shfl_sync(0xFFFFFFFFu, Ea, 1, 8),
+                 Ez = __shfl_sync(0xFFFFFFFFu, Ea, 2, 8);
   const float sx = __uint_as_float(Ex << 23), sy = __uint_as_float(Ey << 23), sz = __uint_as_float(Ez << 23);
   const float ix = __uint_as_float((254u - Ex) << 23), iy = __uint_as_float((254u - Ey) << 23),
               iz = __uint_as_float((254u - Ez) << 23);
@@ -1900,36 +1833,48 @@ __device__ __forceinline__ void collapse_emit_group(
   const float dx = (lo.x + hi.x) * 0.5f - pc.x, dy = (lo.y + hi.y) * 0.5f - pc.y, dz = (lo.z + hi.z) * 0.5f - pc.z;
   float cs[8];
 #pragma unroll
-  for (int s = 0; s < 8; s++) cs[s] = ((s & 1) ? -dx : dx) + ((s & 2) ? -dy : dy) + ((s & 4) ? -dz : dz);
-  // greedy assignment: per round every unplaced child offers its cheapest free
-  // slot; the group takes the least (cost, child, slot)
-  uint32_t used = 0;
-  int my_slot = -1;
-  for (int it = 0; it < nk; it++) {
-    unsigned long long key = ~0ull;
-    if (valid && my_slot < 0) {
+  for (int q = 0; q < 8; q++) cs[q] = ((q & 1) ? -dx : dx) + ((q & 2) ? -dy : dy) + ((q & 4) ? -dz : dz);
+  unsigned long long* key = sm.key[g];
+  uint32_t* words = sm.node[g];
+  key[i] = ~0ull;
+  // empty slots: meta 0, lower planes 255, upper planes 0
+  if (i < 7u) *reinterpret_cast<uint2*>(words + 6 + 2 * i) = i >= 1u && i <= 3u ? make_uint2(~0u, ~0u) : make_uint2(0u, 0u);
+  __syncwarp();
+  uint32_t refused = 0, slot = 8;
+  bool placed = !valid;
+  unsigned long long offer = 0;
+  while (__any_sync(0xFFFFFFFFu, !placed)) {
+    if (!placed) {
       float bc = INFINITY;
       int bs = -1;
 #pragma unroll
-      for (int s = 0; s < 8; s++) {
-        if (used >> s & 1u) continue;
-        if (bs < 0 || cs[s] < bc) {
-          bc = cs[s];
-          bs = s;
+      for (int q = 0; q < 8; q++) {
+        if (!(refused >> q & 1u) && (bs < 0 || cs[q] < bc)) {
+          bc = cs[q];
+          bs = q;
         }
       }
-      key = ((unsigned long long)f2ord(bc + 0.0f) << 32) | (i << 3) | (uint32_t)bs;  // + 0: -0 ties with +0
+      slot = (uint32_t)bs & 7u;
+      offer = ((unsigned long long)f2ord(bc + 0.0f) << 32) | i;  // + 0: -0 ties with +0
+      atomicMin(key + slot, offer);
     }
-    const uint32_t khi = __reduce_min_sync(gmask, (uint32_t)(key >> 32));
-    const uint32_t klo = __reduce_min_sync(gmask, (uint32_t)(key >> 32) == khi ? (uint32_t)key : 0xFFFFFFFFu);
-    const uint32_t win = klo >> 3, ws = klo & 7u;
-    used |= 1u << ws;
-    if (win == i) my_slot = (int)ws;
+    __syncwarp();
+    if (valid) {
+      placed = key[slot] == offer;
+      if (!placed) refused |= 1u << slot;
+    }
+    __syncwarp();
   }
   // this child's planes, its part of the SAH, its place among the slots
-  uint32_t qlx = 0, qly = 0, qlz = 0, qhx = 0, qhy = 0, qhz = 0, cnt = 0;
-  bool internal = false;
-  double A = 0.0, Ax = 0.0;
+  const bool inner = cnt > t.leaf_max;
+  uint32_t places = valid ? (inner ? 8u : cnt) << (4u * slot) : 0u;  // 4 bits per slot: triangles, bit 3 an internal child
+  uint32_t int_slots = inner ? 1u << slot : 0u;
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    places |= __shfl_xor_sync(0xFFFFFFFFu, places, o);
+    int_slots |= __shfl_xor_sync(0xFFFFFFFFu, int_slots, o);
+  }
+  const uint32_t child_base = next_base + oi, tri_base = tri_next + ot;
   if (valid) {
     const float flx = fminf(fmaxf(floorf(__fsub_rd(lo.x, ulo.x) * ix), 0.f), 255.f);
     const float fly = fminf(fmaxf(floorf(__fsub_rd(lo.y, ulo.y) * iy), 0.f), 255.f);
@@ -1937,95 +1882,63 @@ __device__ __forceinline__ void collapse_emit_group(
     const float fhx = fminf(fmaxf(ceilf(__fsub_ru(hi.x, ulo.x) * ix), 0.f), 255.f);
     const float fhy = fminf(fmaxf(ceilf(__fsub_ru(hi.y, ulo.y) * iy), 0.f), 255.f);
     const float fhz = fminf(fmaxf(ceilf(__fsub_ru(hi.z, ulo.z) * iz), 0.f), 255.f);
-    qlx = (uint32_t)flx; qly = (uint32_t)fly; qlz = (uint32_t)flz;
-    qhx = (uint32_t)fhx; qhy = (uint32_t)fhy; qhz = (uint32_t)fhz;
     // decoded (outward-rounded) box, as traversal sees it
     const float3 dlo = make_float3(__fmaf_rd(flx, sx, ulo.x), __fmaf_rd(fly, sy, ulo.y), __fmaf_rd(flz, sz, ulo.z));
     const float3 dhi = make_float3(__fmaf_ru(fhx, sx, ulo.x), __fmaf_ru(fhy, sy, ulo.y), __fmaf_ru(fhz, sz, ulo.z));
-    A = (double)fmaxf(0.f, half_area(dlo, dhi));
-    Ax = (double)fmaxf(0.f, half_area(lo, hi));
-    cnt = bt_cnt(t, kid);
-    internal = cnt > t.leaf_max;
+    const double A = (double)fmaxf(0.f, half_area(dlo, dhi));
+    const double Ax = (double)fmaxf(0.f, half_area(lo, hi));
+    const uint32_t below = places & ((1u << (4u * slot)) - 1u);
+    uint32_t meta;
+    if (inner) {
+      const uint32_t rank = __popc(below & 0x88888888u);
+      meta = 0x80u | slot;
+      if (oi + rank >= node_cap || child_base + rank >= node_cap) atomicOr(err, kErrBuild);
+      else next_items[oi + rank] = kid;
+      sah_out += A;  // inner node term
+      sahx_out += Ax;
+    } else {
+      // triangles of the leaves in lower slots: the sum of their 3-bit counts
+      const uint32_t c = below & 0x77777777u;
+      const uint32_t tri_off = (((c & 0x0F0F0F0Fu) + (c >> 4 & 0x0F0F0F0Fu)) * 0x01010101u) >> 24;
+      meta = 0x80u | ((cnt - 1u) << 5) | tri_off;
+      // the leaf's triangle records are written after the last level by
+      // k_write_leaves, one thread per leaf: here only its binary subtree is
+      // recorded at the slot of its first triangle
+      if (tri_base + tri_off + cnt > tri_cap) atomicOr(err, kErrBuild);
+      else leaf_root[tri_base + tri_off] = cnt == 1 ? prim | kLeafPrim : kid;
+      sah_out += A * (double)((cnt + 3) / 4);  // leaf term: area x Triangle4 blocks
+      sahx_out += Ax * (double)((cnt + 3) / 4);
+      nleaf_out++;
+    }
+    uint8_t* bytes = reinterpret_cast<uint8_t*>(words);
+    bytes[24 + slot] = (uint8_t)meta;
+    bytes[32 + slot] = (uint8_t)flx;
+    bytes[40 + slot] = (uint8_t)fly;
+    bytes[48 + slot] = (uint8_t)flz;
+    bytes[56 + slot] = (uint8_t)fhx;
+    bytes[64 + slot] = (uint8_t)fhy;
+    bytes[72 + slot] = (uint8_t)fhz;
   }
-  const uint32_t slot = valid ? (uint32_t)my_slot : 8u;
-  const uint32_t int_slots = __reduce_or_sync(gmask, internal ? 1u << slot : 0u);
-  uint32_t tri_off = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const uint32_t sj = __shfl_sync(gmask, slot, j, 8);
-    const uint32_t cj = __shfl_sync(gmask, (valid && !internal) ? cnt : 0u, j, 8);
-    if (sj < slot) tri_off += cj;
+  if (i == 0u)
+    *reinterpret_cast<uint4*>(words) = make_uint4(__float_as_uint(ulo.x), __float_as_uint(ulo.y), __float_as_uint(ulo.z),
+                                                  Ex | (Ey << 8) | (Ez << 16) | ((int_slots & 0xFFu) << 24));
+  else if (i == 1u)
+    *reinterpret_cast<uint2*>(words + 4) = make_uint2(child_base, tri_base);
+  else if (i == 2u)
+    *reinterpret_cast<uint4*>(words + 20) = make_uint4(__float_as_uint(sx * 32768.0f), __float_as_uint(sy * 32768.0f),
+                                                       __float_as_uint(sz * 32768.0f), 0u);
+  __syncwarp();
+  if (have) {
+    if (level_base + k >= node_cap) {
+      if (i == 0u) atomicOr(err, kErrBuild);
+    } else if (i < 6u) {
+      reinterpret_cast<uint4*>(nodes + level_base + k)[i] = reinterpret_cast<const uint4*>(words)[i];
+    }
   }
-  const uint32_t oi = off_int[k], ot = off_tri[k];
-  const uint32_t child_base = next_base + oi, tri_base = tri_next + ot;
-  uint32_t meta = 0;
-  if (valid && internal) {
-    const uint32_t rank = __popc(int_slots & ((1u << slot) - 1u));
-    meta = 0x80u | slot;
-    if (oi + rank >= node_cap || child_base + rank >= node_cap) atomicOr(err, kErrBuild);
-    else next_items[oi + rank] = kid;
-    sah_out += A;  // inner node term
-    sahx_out += Ax;
-  } else if (valid) {
-    meta = 0x80u | ((cnt - 1u) << 5) | tri_off;
-    // the leaf's triangle records are written after the last level by
-    // k_write_leaves, one thread per leaf: here only its binary subtree is
-    // recorded at the slot of its first triangle
-    if (tri_base + tri_off + cnt > tri_cap) atomicOr(err, kErrBuild);
-    else leaf_root[tri_base + tri_off] = cnt == 1 ? bt_right(t, kid) | kLeafPrim : kid;
-    sah_out += A * (double)((cnt + 3) / 4);  // leaf term: area x Triangle4 blocks
-    sahx_out += Ax * (double)((cnt + 3) / 4);
-    nleaf_out++;
-  }
-  // the node's words: byte `slot` of each per-slot array (empty slots: meta 0,
-  // lower planes 255, upper planes 0)
-  const uint32_t sh = 8u * (slot & 3u);
-  const bool hi4 = slot >= 4u && slot < 8u, lo4 = slot < 4u;
-  auto word = [&](uint32_t v, bool part) { return part ? v << sh : 0u; };
-  const uint32_t empty = (~used) & 0xFFu;
-  auto fill = [&](uint32_t m4) {  // 0xFF in the bytes of the empty slots m4 (4 bits)
-    return ((m4 & 1u) ? 0xFFu : 0u) | ((m4 & 2u) ? 0xFF00u : 0u) | ((m4 & 4u) ? 0xFF0000u : 0u) |
-           ((m4 & 8u) ? 0xFF000000u : 0u);
-  };
-  const uint32_t m0 = __reduce_or_sync(gmask, word(meta, lo4)), m1 = __reduce_or_sync(gmask, word(meta, hi4));
-  const uint32_t lx0 = __reduce_or_sync(gmask, word(qlx, lo4)) | fill(empty & 15u);
-  const uint32_t lx1 = __reduce_or_sync(gmask, word(qlx, hi4)) | fill(empty >> 4);
-  const uint32_t ly0 = __reduce_or_sync(gmask, word(qly, lo4)) | fill(empty & 15u);
-  const uint32_t ly1 = __reduce_or_sync(gmask, word(qly, hi4)) | fill(empty >> 4);
-  const uint32_t lz0 = __reduce_or_sync(gmask, word(qlz, lo4)) | fill(empty & 15u);
-  const uint32_t lz1 = __reduce_or_sync(gmask, word(qlz, hi4)) | fill(empty >> 4);
-  const uint32_t hx0 = __reduce_or_sync(gmask, word(qhx, lo4)), hx1 = __reduce_or_sync(gmask, word(qhx, hi4));
-  const uint32_t hy0 = __reduce_or_sync(gmask, word(qhy, lo4)), hy1 = __reduce_or_sync(gmask, word(qhy, hi4));
-  const uint32_t hz0 = __reduce_or_sync(gmask, word(qhz, lo4)), hz1 = __reduce_or_sync(gmask, word(qhz, hi4));
-  if (level_base + k >= node_cap) {
-    if (i == 0) atomicOr(err, kErrBuild);
-    return;
-  }
-  // WideNode as six 16-byte words (gb_common.h layout)
-  uint4* dst = reinterpret_cast<uint4*>(nodes + level_base + k);
-  if (i == 0) {
-    dst[0] = make_uint4(__float_as_uint(ulo.x), __float_as_uint(ulo.y), __float_as_uint(ulo.z),
-                        Ex | (Ey << 8) | (Ez << 16) | ((int_slots & 0xFFu) << 24));
-  } else if (i == 1) {
-    dst[1] = make_uint4(child_base, tri_base, m0, m1);
-  } else if (i == 2) {
-    dst[2] = make_uint4(lx0, lx1, ly0, ly1);
-  } else if (i == 3) {
-    dst[3] = make_uint4(lz0, lz1, hx0, hx1);
-  } else if (i == 4) {
-    dst[4] = make_uint4(hy0, hy1, hz0, hz1);
-  } else if (i == 5) {
-    dst[5] = make_uint4(__float_as_uint(sx * 32768.0f), __float_as_uint(sy * 32768.0f),
-                        __float_as_uint(sz * 32768.0f), 0u);
-  }
+  __syncwarp();  // the words are built again for the next node
 }
 
 constexpr int COLLAPSE_THREADS = 128;
-// Levels of at most this many items are emitted by lane groups (latency-bound:
-// one node's greedy slot choice and reductions spread over 8 lanes), wider ones
-// one node per thread.
-constexpr uint32_t kGroupEmitMax = 16384;
-
 // One wide node per 8-lane group; the SAH sums and the leaf count are reduced
 // per CTA first (one atomic per CTA instead of one per node).
 __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_emit(
@@ -2038,21 +1951,11 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_emit(
   const uint32_t next_base = level_base + nitems;
   double sah = 0.0, sahx = 0.0;
   uint32_t nleaf = 0;
-  if (nitems <= kGroupEmitMax) {
-    const uint32_t gmask = 0xFFu << (threadIdx.x & 24u);
-    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 3; k < nitems; k += (gridDim.x * blockDim.x) >> 3)
-      collapse_emit_group(t, kids_in, k, off_int, off_tri, level_base, next_base, tri_next, nodes, leaf_root,
-                          next_items, node_cap, tri_cap, err, gmask, sah, sahx, nleaf);
-  } else {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nitems; k += gridDim.x * blockDim.x) {
-      double a = 0.0, b = 0.0;
-      uint32_t l = 0;
-      collapse_emit_node(t, kids_in, k, off_int, off_tri, level_base, next_base, tri_next, nodes, leaf_root,
-                         next_items, node_cap, tri_cap, err, a, b, l);
-      sah += a;
-      sahx += b;
-      nleaf += l;
-    }
+  __shared__ EmitSmem<COLLAPSE_THREADS / 8> sm;
+  for (uint32_t k0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 3; k0 < nitems; k0 += (gridDim.x * blockDim.x) >> 3) {
+    const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
+    collapse_emit_group(t, kids_in, k, k < nitems, threadIdx.x >> 3, sm, off_int, off_tri, level_base, next_base, tri_next,
+                        nodes, leaf_root, next_items, node_cap, tri_cap, err, sah, sahx, nleaf);
   }
   nleaf = __reduce_add_sync(0xFFFFFFFFu, nleaf);
   if ((threadIdx.x & 31) == 0 && nleaf) atomicAdd(leaf_count, nleaf);
@@ -2110,7 +2013,7 @@ __device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32
 // turns its counts into the level's exclusive offsets from the CTA sums, (3)
 // writes its wide nodes and the next level's items, [barrier].  cta_sums holds
 // 2 * gridDim.x words; *bar is zero on entry.
-__global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 2) k_collapse_all(
+__global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 4) k_collapse_all(
     BinTree t, const ColItems ci, uint32_t* __restrict__ cstate, uint32_t* __restrict__ kids,
     uint32_t* __restrict__ nint, uint32_t* __restrict__ ntri, uint32_t* __restrict__ cta_sums,
     WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root, double* sah_acc, uint32_t* leaf_count,
@@ -2118,6 +2021,7 @@ __global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 2) k_collapse_all(
   uint32_t nitems = __ldcg(cstate + kColN), base = __ldcg(cstate + kColBase), tri_next = __ldcg(cstate + kColTri),
            depth = __ldcg(cstate + kColDepth);
   bool failed = __ldcg(cstate + kColErr) != 0u;
+  __shared__ EmitSmem<COLLAPSE_ALL_THREADS / 8> sm;
   double sah = 0.0, sahx = 0.0;
   uint32_t nleaf = 0;
   while (nitems > 0 && !failed) {
@@ -2127,24 +2031,16 @@ __global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 2) k_collapse_all(
     const uint32_t first = min(blockIdx.x * per, nitems), last = min(first + per, nitems);
     // (1) children and counts
     uint32_t ci_sum = 0, ct_sum = 0;
-    for (uint32_t k = first + threadIdx.x; k < last; k += blockDim.x) {
-      uint32_t kk[8];
-      const int nk = gather_children(t, items[k], kk);
-      uint32_t ni = 0, nt = 0;
-      for (int i = 0; i < 8; i++) {
-        if (i < nk) {
-          const uint32_t c = kk[i];
-          const uint32_t cnt = bt_cnt(t, c);
-          if (cnt > t.leaf_max) ni++; else nt += cnt;
-          kids[8 * (size_t)k + i] = c;
-        } else {
-          kids[8 * (size_t)k + i] = 0xFFFFFFFFu;
-        }
+    for (uint32_t k0 = first + ((threadIdx.x & ~31u) >> 3); k0 < last; k0 += blockDim.x >> 3) {
+      const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
+      uint32_t ni, nt;
+      collapse_count_group(t, items, k, k < last, kids, &ni, &nt);
+      if (k < last && (threadIdx.x & 7u) == 0u) {
+        nint[k] = ni;
+        ntri[k] = nt;
+        ci_sum += ni;
+        ct_sum += nt;
       }
-      nint[k] = ni;
-      ntri[k] = nt;
-      ci_sum += ni;
-      ct_sum += nt;
     }
     {
       uint32_t ta, tb;
@@ -2188,23 +2084,11 @@ __global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 2) k_collapse_all(
       pt += tb;
     }
     __syncthreads();
-    // (3) the wide nodes of this CTA's items: one per 8-lane group on narrow
-    // levels, one per thread on wide ones
-    if (nitems <= kGroupEmitMax) {
-      const uint32_t gmask = 0xFFu << (threadIdx.x & 24u);
-      for (uint32_t k = first + (threadIdx.x >> 3); k < last; k += blockDim.x >> 3)
-        collapse_emit_group(t, kids, k, nint, ntri, base, base + nitems, tri_next, nodes, leaf_root, next_items,
-                            node_cap, tri_cap, err, gmask, sah, sahx, nleaf);
-    } else {
-      for (uint32_t k = first + threadIdx.x; k < last; k += blockDim.x) {
-        double a = 0.0, b = 0.0;
-        uint32_t l = 0;
-        collapse_emit_node(t, kids, k, nint, ntri, base, base + nitems, tri_next, nodes, leaf_root, next_items,
-                           node_cap, tri_cap, err, a, b, l);
-        sah += a;
-        sahx += b;
-        nleaf += l;
-      }
+    // (3) the wide nodes of this CTA's items, one per 8-lane group
+    for (uint32_t k0 = first + ((threadIdx.x & ~31u) >> 3); k0 < last; k0 += blockDim.x >> 3) {
+      const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
+      collapse_emit_group(t, kids, k, k < last, threadIdx.x >> 3, sm, nint, ntri, base, base + nitems, tri_next, nodes,
+                          leaf_root, next_items, node_cap, tri_cap, err, sah, sahx, nleaf);
     }
     // (4) the next level, alike in every CTA
     if (blockIdx.x == 0 && threadIdx.x == 0 && depth < (uint32_t)kColMaxLevels) cstate[kColLevels + depth] = base;
@@ -2663,11 +2547,11 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   uint32_t level = 0;
   const uint32_t max_levels = 0xFFFFFFFFu;  // host-driven: level starts recorded here, no bound
   auto enqueue_level = [&](uint32_t nitems_known) {  // the level's size, read by the host
-    const uint32_t grid = cdiv(nitems_known, 128);
+    const uint32_t grid = cdiv(8ull * nitems_known, 128);
     k_collapse_count<<<grid, 128, 0, st>>>(bt, citems, cstate, kids, nint, ntri);
     note_launches(1);
     scan_excl2(nint, ntri, nitems_known, d_tot + 0, d_tot + 1, scan_sums, st, &acc->pad);
-    k_collapse_emit<<<cdiv((uint64_t)nitems_known * (nitems_known <= kGroupEmitMax ? 8 : 1), COLLAPSE_THREADS),
+    k_collapse_emit<<<cdiv(8ull * nitems_known, COLLAPSE_THREADS),
                       COLLAPSE_THREADS, 0, st>>>(
         bt, kids, cstate, nint, ntri, wnodes, leaf_root, citems, d_sah, d_leaves, maxw, N, &acc->pad);
     k_collapse_advance<<<1, 32, 0, st>>>(d_tot, cstate, maxw, max_levels);
@@ -3218,17 +3102,17 @@ __device__ __forceinline__ void refit_tri(const GeomDesc* __restrict__ geoms, co
 // Refits wide node k from its children's boxes (inner children: node_box of the
 // level below; leaf children: the boxes refit_tri stored for their triangles) and
 // adds the node's SAH terms on the decoded and on the exact boxes.  The 8 lanes of
-// a lane group share the node, lane i its slot i (all 8 call it with the same k;
-// gmask names them): the children's loads are one dependent step instead of eight,
+// a lane group share the node, lane i its slot i (all 32 lanes of the warp call it,
+// `have` is the group's): the children's loads are one dependent step instead of eight,
 // and a level takes as long as its widest lane.  Boxes are read past L1, where
 // another CTA of the same launch may have written them.
 __device__ __forceinline__ void refit_node_group(const float4* tri_box, uint32_t num_tris,
                                                  WideNode* __restrict__ nodes, uint32_t num_nodes, float* node_box,
-                                                 uint32_t k, uint32_t gmask, uint32_t* err, double& sah_out,
+                                                 uint32_t k, bool have, uint32_t* err, double& sah_out,
                                                  double& sahx_out) {
   const uint32_t s = threadIdx.x & 7u;
-  WideNode* node = nodes + k;
-  const uint32_t m = node->meta[s], imask = node->imask;
+  WideNode* node = nodes + (have ? k : 0u);
+  const uint32_t m = have ? node->meta[s] : 0u, imask = node->imask;
   float3 lo = make_float3(INFINITY, INFINITY, INFINITY), hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
   bool ok = true;
   if (m != 0) {
@@ -3257,24 +3141,24 @@ __device__ __forceinline__ void refit_node_group(const float4* tri_box, uint32_t
       }
     }
   }
-  if (__any_sync(gmask, !ok)) {
-    if (s == 0) atomicOr(err, kErrBuild);
-    return;
-  }
+  const uint32_t bad = __ballot_sync(0xFFFFFFFFu, !ok) >> (threadIdx.x & 24u) & 0xFFu;
+  if (bad && s == 0) atomicOr(err, kErrBuild);
+  have = have && bad == 0u;
   float3 ulo = lo, uhi = hi;
 #pragma unroll
   for (int o = 1; o < 8; o <<= 1) {
-    ulo.x = fminf(ulo.x, __shfl_xor_sync(gmask, ulo.x, o, 8));
-    ulo.y = fminf(ulo.y, __shfl_xor_sync(gmask, ulo.y, o, 8));
-    ulo.z = fminf(ulo.z, __shfl_xor_sync(gmask, ulo.z, o, 8));
-    uhi.x = fmaxf(uhi.x, __shfl_xor_sync(gmask, uhi.x, o, 8));
-    uhi.y = fmaxf(uhi.y, __shfl_xor_sync(gmask, uhi.y, o, 8));
-    uhi.z = fmaxf(uhi.z, __shfl_xor_sync(gmask, uhi.z, o, 8));
+    ulo.x = fminf(ulo.x, __shfl_xor_sync(0xFFFFFFFFu, ulo.x, o));
+    ulo.y = fminf(ulo.y, __shfl_xor_sync(0xFFFFFFFFu, ulo.y, o));
+    ulo.z = fminf(ulo.z, __shfl_xor_sync(0xFFFFFFFFu, ulo.z, o));
+    uhi.x = fmaxf(uhi.x, __shfl_xor_sync(0xFFFFFFFFu, uhi.x, o));
+    uhi.y = fmaxf(uhi.y, __shfl_xor_sync(0xFFFFFFFFu, uhi.y, o));
+    uhi.z = fmaxf(uhi.z, __shfl_xor_sync(0xFFFFFFFFu, uhi.z, o));
   }
   const uint32_t Ex = exp_for(__fsub_ru(uhi.x, ulo.x));
   const uint32_t Ey = exp_for(__fsub_ru(uhi.y, ulo.y));
   const uint32_t Ez = exp_for(__fsub_ru(uhi.z, ulo.z));
   const float sx = __uint_as_float(Ex << 23), sy = __uint_as_float(Ey << 23), sz = __uint_as_float(Ez << 23);
+  if (!have) return;
   if (m != 0) {
     const float ix = __uint_as_float((254u - Ex) << 23), iy = __uint_as_float((254u - Ey) << 23),
                 iz = __uint_as_float((254u - Ez) << 23);
@@ -3330,7 +3214,6 @@ __global__ void __launch_bounds__(256) k_refit_all(const GeomDesc* __restrict__ 
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < num_tris; i += gridDim.x * blockDim.x)
     refit_tri(geoms, slot_of, nslots, tris, i, robust, tri_box, err);
   double sah = 0.0, sahx = 0.0;
-  const uint32_t gmask = 0xFFu << (threadIdx.x & 24u);
   bool wide_below = true;
   for (uint32_t l = lv.n; l-- > 0;) {
     const uint32_t begin = lv.start[l], end = min(lv.start[l + 1], num_nodes);
@@ -3346,8 +3229,11 @@ __global__ void __launch_bounds__(256) k_refit_all(const GeomDesc* __restrict__ 
     wide_below = wide;
     if (!wide && blockIdx.x != 0) continue;
     const uint32_t stride = (wide ? gridDim.x * blockDim.x : blockDim.x) >> 3;
-    for (uint32_t k = begin + ((wide ? blockIdx.x * blockDim.x + threadIdx.x : threadIdx.x) >> 3); k < end; k += stride)
-      refit_node_group(tri_box, num_tris, nodes, num_nodes, node_box, k, gmask, err, sah, sahx);
+    const uint32_t warp0 = (wide ? blockIdx.x * blockDim.x : 0u) + (threadIdx.x & ~31u);
+    for (uint32_t k0 = begin + (warp0 >> 3); k0 < end; k0 += stride) {
+      const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
+      refit_node_group(tri_box, num_tris, nodes, num_nodes, node_box, k, k < end, err, sah, sahx);
+    }
   }
   block_add2(sah, sahx, sah_acc);
 }
@@ -3366,8 +3252,7 @@ __global__ void __launch_bounds__(128) k_refit_level(const float4* tri_box, uint
                                                      uint32_t* err) {
   const uint32_t k = begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 3);
   double sah = 0.0, sahx = 0.0;
-  if (k < end && k < num_nodes)
-    refit_node_group(tri_box, num_tris, nodes, num_nodes, node_box, k, 0xFFu << (threadIdx.x & 24u), err, sah, sahx);
+  refit_node_group(tri_box, num_tris, nodes, num_nodes, node_box, k, k < end && k < num_nodes, err, sah, sahx);
   block_add2(sah, sahx, sah_acc);
 }
 
@@ -3408,7 +3293,7 @@ cudaError_t refit_prepare(const GeomDesc* h_geoms, int ngeoms, const DeviceBVH& 
 cudaError_t refit_enqueue(const DeviceBVH& bvh, const RefitScratch& s, cudaStream_t st) {
   RefitResult* r = s.result;
   float* node_box = reinterpret_cast<float*>(r + 1);
-  GB_CHECK(cudaMemsetAsync(r->sah, 0, sizeof(r->sah), st));
+  GB_CHECK(cudaMemsetAsync(r, 0, offsetof(RefitResult, err), st));  // sums and barrier
   const size_t nlevels = bvh.level_start.size() - 1;
   if (nlevels <= (size_t)kColMaxLevels) {
     RefitLevels lv{};
@@ -3425,7 +3310,7 @@ cudaError_t refit_enqueue(const DeviceBVH& bvh, const RefitScratch& s, cudaStrea
     cfg.numAttrs = 1;
     GB_CHECK(cudaLaunchKernelEx(&cfg, k_refit_all, (const GeomDesc*)s.d_geoms, (const uint32_t*)s.d_slot, s.nslots,
                                 bvh.tris, bvh.num_tris, bvh.robust, s.tri_box, bvh.nodes, bvh.num_nodes, node_box, lv,
-                                r->sah, reinterpret_cast<GridBarrier*>(r->bar), &r->bar[2], &r->err));
+                                r->sah, reinterpret_cast<GridBarrier*>(&r->bar), &r->bar_err, &r->err));
     note_launches(1);
     return cudaGetLastError();
   }

@@ -20,8 +20,8 @@ void free_bvh(DeviceBVH* b);
 // updated.  A scratch belongs to the BVH it was prepared for.
 struct RefitResult {
   double sah[2];         // SAH sums on the decoded and on the exact boxes
-  uint32_t err;          // kErr* bits
-  unsigned int bar[3];   // grid barrier (count, generation) and its own error word
+  unsigned int bar, bar_err;  // grid barrier and its own error word (these and the sums are cleared per refit)
+  uint32_t err, pad;          // kErr* bits
 };
 struct RefitScratch {
   GeomDesc* d_geoms = nullptr;
