@@ -104,7 +104,7 @@ __device__ __forceinline__ int find_geom(const GeomDesc* geoms, int ngeoms, uint
   return lo;
 }
 
-// plo[i] = (lo.xyz, geometry slot), phi[i] = (hi.xyz, primID); invalid
+// pbox[2i] = (lo.xyz, geometry slot), pbox[2i + 1] = (hi.xyz, primID); invalid
 // triangles get an empty box (+inf,-inf).  prec[i] (when non-null) receives
 // primitive i's leaf record -- Triangle4 values v0, e1 = v0 - v1, e2 = v2 - v0
 // (triangle.h:40-41), or v0, v1, v2 in robust scenes (trianglev.h:93-115), or
@@ -113,8 +113,7 @@ __device__ __forceinline__ int find_geom(const GeomDesc* geoms, int ngeoms, uint
 // Grid-stride: the bounds and the valid count are reduced per thread, per warp
 // and per CTA, so the global atomics are 13 per CTA (a grid of a few CTAs per SM).
 __global__ void __launch_bounds__(256) k_primrefs(const GeomDesc* __restrict__ geoms, int ngeoms, uint32_t total,
-                                                  float4* __restrict__ plo, float4* __restrict__ phi,
-                                                  BoundsAcc* acc, TriRecord* __restrict__ prec, int robust) {
+                                                  float4* __restrict__ pbox, BoundsAcc* acc, TriRecord* __restrict__ prec, int robust) {
   __shared__ uint32_t s_b[12];
   __shared__ uint32_t s_cnt;
   if (threadIdx.x < 12) s_b[threadIdx.x] = (threadIdx.x % 6) < 3 ? 0xFFFFFFFFu : 0u;
@@ -161,8 +160,8 @@ __global__ void __launch_bounds__(256) k_primrefs(const GeomDesc* __restrict__ g
         }
       }
       }
-      plo[gi] = make_float4(lo.x, lo.y, lo.z, __uint_as_float((uint32_t)gs));
-      phi[gi] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(j));
+      pbox[2 * (size_t)gi] = make_float4(lo.x, lo.y, lo.z, __uint_as_float((uint32_t)gs));
+      pbox[2 * (size_t)gi + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(j));
     }
     v[0] = fminf(v[0], lo.x); v[1] = fminf(v[1], lo.y); v[2] = fminf(v[2], lo.z);
     v[3] = fmaxf(v[3], hi.x); v[4] = fmaxf(v[4], hi.y); v[5] = fmaxf(v[5], hi.z);
@@ -238,7 +237,7 @@ constexpr uint32_t kMaxSegments = 4096;
 
 // Grid-stride; the AND / OR of all keys (constant digits are not sorted) is
 // reduced per thread, per warp and per CTA: two global atomics per CTA.
-__global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ plo, const float4* __restrict__ phi,
+__global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ pbox,
                                                 uint32_t n, BoundsAcc* acc, uint64_t* __restrict__ keys,
                                                 uint32_t* __restrict__ vals, int cube, int segmented, int bits30,
                                                 int key32) {
@@ -252,7 +251,7 @@ __global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ plo, 
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     uint64_t key = bits30 ? (1ull << (segmented ? 42 : 30)) : ~0ull;
     {
-      const float4 a = plo[i], b = phi[i];
+      const float4 a = pbox[2 * (size_t)i], b = pbox[2 * (size_t)i + 1];
       if (a.x <= b.x) {
         const float lo[3] = {ord2f(acc->clo[0]), ord2f(acc->clo[1]), ord2f(acc->clo[2])};
         const float hi[3] = {ord2f(acc->chi[0]), ord2f(acc->chi[1]), ord2f(acc->chi[2])};
@@ -701,14 +700,15 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_lb(ScanPair sp, uint32_t 
 // the SAH statistic's terms (bvh_statistics.cpp:10-160), so the tree minimises
 // the reported SAH for the given binary tree and leaf size.
 //
-// choice[n] packs the decisions: byte 0 = argmin k of D(n, 8) (the split of a
+// link[n] = (left, right, decisions): one 16-byte read per node for the collapse,
+// which follows the decisions from node to node.  Of the decisions, byte 0 = argmin k of D(n, 8) (the split of a
 // wide node made from n); byte i - 1 (i = 2..8) = the k of D(n, i) when it beat
 // cost(n, i - 1), else 0.
 
-__device__ __forceinline__ void dp_store(float4* cost, uint2* choice, uint32_t n, const float c[8], uint2 ch) {
+__device__ __forceinline__ void dp_store(float4* cost, uint4* link, uint32_t n, const float c[8], uint4 lk) {
   __stcg(cost + 2 * (size_t)n, make_float4(c[0], c[1], c[2], c[3]));
   __stcg(cost + 2 * (size_t)n + 1, make_float4(c[4], c[5], c[6], c[7]));
-  __stcg(choice + n, ch);
+  __stcg(link + n, lk);
 }
 
 // A child's cost(., 1..8): a primitive (one triangle) costs its box area
@@ -730,7 +730,7 @@ __device__ __forceinline__ void dp_child_costs(const float4* cost, uint32_t c, u
 // the caller passes); A is n's box area.  The PLOC kernels call it as they
 // create each node, so the table is complete when the clustering ends
 // (children are always created before their parent).
-__device__ __forceinline__ void dp_node(float4* cost, uint2* choice, uint32_t n, uint32_t l, uint32_t r, float A,
+__device__ __forceinline__ void dp_node(float4* cost, uint4* link, uint32_t n, uint32_t l, uint32_t r, float A,
                                         uint32_t cnt_l, uint32_t cnt_r, float Al, float Ar, uint32_t leaf_max) {
   const uint32_t cnt = cnt_l + cnt_r;
   float cl[8], cr[8];
@@ -763,8 +763,8 @@ __device__ __forceinline__ void dp_node(float4* cost, uint2* choice, uint32_t n,
     c[i - 1] = split ? D[i] : c[i - 2];
     b[i - 1] = split ? K[i] : 0u;
   }
-  dp_store(cost, choice, n, c,
-           make_uint2(b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24), b[4] | (b[5] << 8) | (b[6] << 16) | (b[7] << 24)));
+  dp_store(cost, link, n, c,
+           make_uint4(l, r, b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24), b[4] | (b[5] << 8) | (b[6] << 16) | (b[7] << 24)));
 }
 
 
@@ -818,24 +818,23 @@ constexpr int PLOC_SMALL_THREADS = 1024;
 // k_ploc_small's shared memory: boxes, node ids, nearest neighbours, segments, counts
 constexpr size_t kPlocSmallSmem = (size_t)PLOC_SMALL * (2 * sizeof(float3) + 4 * sizeof(uint32_t));
 
-// binary nodes: bnlo[k] = (lo.xyz, left), bnhi[k] = (hi.xyz, right);
+// binary nodes: bnbox[2k] = (lo.xyz, left), bnbox[2k + 1] = (hi.xyz, right), one
+// 32-byte sector (they are read one by one, in no order);
 // leaves k < N: left = -1, right = primref index
 // Cluster boxes carry their segment in clo.w (0 unless the build is segmented)
 // and their triangle count in chi.w (so a merge has both children's counts
 // with their boxes, without a dependent read of bncnt).
-__global__ void __launch_bounds__(256) k_ploc_init(const float4* __restrict__ plo, const float4* __restrict__ phi,
+__global__ void __launch_bounds__(256) k_ploc_init(const float4* __restrict__ pbox,
                                                    const uint32_t* __restrict__ sorted, uint32_t n,
                                                    const uint32_t* __restrict__ d_n,
-                                                   float4* __restrict__ bnlo, float4* __restrict__ bnhi,
-                                                   uint32_t* __restrict__ bncnt, uint32_t* __restrict__ cidx,
+                                                   float4* __restrict__ bnbox, uint32_t* __restrict__ cidx,
                                                    float4* __restrict__ clo, float4* __restrict__ chi, int segmented) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n || i >= *d_n) return;  // n bounds the grid, *d_n is the count of valid primitives
   const uint32_t p = sorted[i];
-  const float4 a = plo[p], b = phi[p];
-  bnlo[i] = make_float4(a.x, a.y, a.z, __int_as_float(-1));
-  bnhi[i] = make_float4(b.x, b.y, b.z, __uint_as_float(p));
-  bncnt[i] = 1;
+  const float4 a = pbox[2 * (size_t)p], b = pbox[2 * (size_t)p + 1];
+  bnbox[2 * (size_t)i] = make_float4(a.x, a.y, a.z, __int_as_float(-1));
+  bnbox[2 * (size_t)i + 1] = make_float4(b.x, b.y, b.z, __uint_as_float(p));
   cidx[i] = i;
   clo[i] = make_float4(a.x, a.y, a.z, segmented ? a.w : __uint_as_float(0u));
   chi[i] = make_float4(b.x, b.y, b.z, __uint_as_float(1u));
@@ -993,10 +992,10 @@ __device__ __forceinline__ uint32_t block_excl_scan_flag(int flag, uint32_t* s_w
 // + rank among its merges.  Each new node's collapse costs are computed here.
 __device__ __forceinline__ void ploc_emit_tile(const PlocBufs& bufs, uint32_t par, const uint32_t* __restrict__ nn,
                                                uint32_t n, uint32_t node_next, uint32_t tile, uint32_t surv_off,
-                                               uint32_t merge_off, float4* __restrict__ bnlo,
-                                               float4* __restrict__ bnhi, uint32_t* __restrict__ bncnt,
+                                               uint32_t merge_off, float4* __restrict__ bnbox,
+                                               uint32_t* __restrict__ bncnt,
                                                uint32_t node_cap, uint32_t* err, float4* __restrict__ dp_cost,
-                                               uint2* __restrict__ dp_choice, uint32_t leaf_max, uint32_t* s_w) {
+                                               uint4* __restrict__ dp_link, uint32_t leaf_max, uint32_t* s_w) {
   const float4* __restrict__ clo = bufs.clo[par];
   const float4* __restrict__ chi = bufs.chi[par];
   const uint32_t* __restrict__ cidx = bufs.cidx[par];
@@ -1032,11 +1031,11 @@ __device__ __forceinline__ void ploc_emit_tile(const PlocBufs& bufs, uint32_t pa
     const float4 lo = make_float4(fminf(a.x, c.x), fminf(a.y, c.y), fminf(a.z, c.z), a.w);
     const uint32_t cnt_l = __float_as_uint(b.w), cnt_r = __float_as_uint(d.w);
     const float4 hi = make_float4(fmaxf(b.x, d.x), fmaxf(b.y, d.y), fmaxf(b.z, d.z), __uint_as_float(cnt_l + cnt_r));
-    bnlo[id] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
-    bnhi[id] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
+    bnbox[2 * (size_t)id] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
+    bnbox[2 * (size_t)id + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
     bncnt[id] = cnt_l + cnt_r;
     if (dp_cost)
-      dp_node(dp_cost, dp_choice, id, l, r, half_area(make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z)),
+      dp_node(dp_cost, dp_link, id, l, r, half_area(make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z)),
               cnt_l, cnt_r, cnt_l == 1 ? half_area(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z)) : 0.f,
               cnt_r == 1 ? half_area(make_float3(c.x, c.y, c.z), make_float3(d.x, d.y, d.z)) : 0.f, leaf_max);
     olo[pos] = lo;
@@ -1053,17 +1052,17 @@ __global__ void __launch_bounds__(PLOC_BLOCK) k_ploc_emit(const PlocBufs bufs, c
                                                           const uint32_t* __restrict__ ploc_state,
                                                           const uint32_t* __restrict__ bsurv_off,
                                                           const uint32_t* __restrict__ bmerge_off,
-                                                          float4* __restrict__ bnlo, float4* __restrict__ bnhi,
+                                                          float4* __restrict__ bnbox,
                                                           uint32_t* __restrict__ bncnt, uint32_t node_cap, uint32_t* err,
-                                                          float4* __restrict__ dp_cost, uint2* __restrict__ dp_choice,
+                                                          float4* __restrict__ dp_cost, uint4* __restrict__ dp_link,
                                                           uint32_t leaf_max) {
   __shared__ uint32_t s_w[PLOC_BLOCK / 32];
   if (ploc_state[kPlocDone]) return;
   const uint32_t n = ploc_state[kPlocN], node_next = ploc_state[kPlocNext];
   const uint32_t par = ploc_state[kPlocParity] & 1u;
   for (uint32_t tile = blockIdx.x; tile * PLOC_BLOCK < n; tile += gridDim.x)
-    ploc_emit_tile(bufs, par, nn, n, node_next, tile, bsurv_off[tile], bmerge_off[tile], bnlo, bnhi, bncnt, node_cap,
-                   err, dp_cost, dp_choice, leaf_max, s_w);
+    ploc_emit_tile(bufs, par, nn, n, node_next, tile, bsurv_off[tile], bmerge_off[tile], bnbox, bncnt, node_cap,
+                   err, dp_cost, dp_link, leaf_max, s_w);
 }
 
 // After a round: the survivors are the new clusters, the merges took the next
@@ -1095,9 +1094,9 @@ template <int PLOC_R>
 __global__ void __launch_bounds__(PLOC_BLOCK) k_ploc_all(const PlocBufs bufs, uint32_t* __restrict__ ploc_state,
                                                          uint32_t* __restrict__ nn, uint32_t* __restrict__ tile_s,
                                                          uint32_t* __restrict__ tile_m, uint32_t* __restrict__ cta_sums,
-                                                         float4* __restrict__ bnlo, float4* __restrict__ bnhi,
+                                                         float4* __restrict__ bnbox,
                                                          uint32_t* __restrict__ bncnt, uint32_t node_cap,
-                                                         float4* __restrict__ dp_cost, uint2* __restrict__ dp_choice,
+                                                         float4* __restrict__ dp_cost, uint4* __restrict__ dp_link,
                                                          uint32_t leaf_max, GridBarrier* bar, unsigned int* err) {
   __shared__ float3 s_lo[PLOC_BLOCK + 2 * PLOC_R], s_hi[PLOC_BLOCK + 2 * PLOC_R];
   __shared__ uint32_t s_seg[PLOC_BLOCK + 2 * PLOC_R];
@@ -1179,7 +1178,7 @@ __global__ void __launch_bounds__(PLOC_BLOCK) k_ploc_all(const PlocBufs bufs, ui
     __syncthreads();  // s_red is reused next round
     uint32_t ps = v[0], pm = v[1];
     for (uint32_t tile = t0; tile < t1; tile++) {
-      ploc_emit_tile(bufs, par, nn, n, node_next, tile, ps, pm, bnlo, bnhi, bncnt, node_cap, err, dp_cost, dp_choice,
+      ploc_emit_tile(bufs, par, nn, n, node_next, tile, ps, pm, bnbox, bncnt, node_cap, err, dp_cost, dp_link,
                      leaf_max, s_w);
       ps += tile_s[tile];
       pm += tile_m[tile];
@@ -1215,13 +1214,12 @@ __global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_small(const float4*
                                                                   const float4* __restrict__ chi_b,
                                                                   const uint32_t* __restrict__ cidx_b,
                                                                   uint32_t* __restrict__ ploc_state,
-                                                                  float4* __restrict__ bnlo,
-                                                                  float4* __restrict__ bnhi,
+                                                                  float4* __restrict__ bnbox,
                                                                   uint32_t* __restrict__ bncnt, uint32_t* root_out,
                                                                   uint32_t* iters_out, uint32_t node_cap,
                                                                   uint32_t* err, uint32_t nseg, int radius,
                                                                   float4* __restrict__ dp_cost,
-                                                                  uint2* __restrict__ dp_choice, uint32_t leaf_max) {
+                                                                  uint4* __restrict__ dp_link, uint32_t leaf_max) {
   extern __shared__ unsigned char smem[];
   float3* s_lo = reinterpret_cast<float3*>(smem);
   float3* s_hi = s_lo + PLOC_SMALL;
@@ -1339,13 +1337,13 @@ __global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_small(const float4*
           const float Ar = cnt_r == 1 ? half_area(s_lo[j], s_hi[j]) : 0.f;
           lo = f3min(lo, s_lo[j]);
           hi = f3max(hi, s_hi[j]);
-          bnlo[nid] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
-          bnhi[nid] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
+          bnbox[2 * (size_t)nid] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
+          bnbox[2 * (size_t)nid + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
           cnt = cnt_l + cnt_r;
           bncnt[nid] = cnt;
           // children come from earlier rounds: their costs were stored before
           // this round's barriers
-          if (dp_cost) dp_node(dp_cost, dp_choice, nid, l, r, half_area(lo, hi), cnt_l, cnt_r, Al, Ar, leaf_max);
+          if (dp_cost) dp_node(dp_cost, dp_link, nid, l, r, half_area(lo, hi), cnt_l, cnt_r, Al, Ar, leaf_max);
           id = nid;
           pm++;
         }
@@ -1416,13 +1414,12 @@ __device__ __forceinline__ void block_add2(double a, double b, double* acc) {
 }
 
 struct BinTree {
-  const float4* lo;
-  const float4* hi;
+  const float4* box;  // two per node: (lo.xyz, left), (hi.xyz, right)
   const uint32_t* cnt;
   uint32_t nleaves;
   uint32_t leaf_max;  // subtrees of at most this many triangles may become leaves
   uint32_t robust;    // write raw vertices into triangle records
-  const uint2* choice;  // SAH-optimal collapse decisions (k_collapse_dp); null: greedy collapse
+  const uint4* link;  // (left, right, SAH-optimal collapse decisions); null: greedy collapse
 };
 
 __device__ __forceinline__ bool bt_leaf(const BinTree& t, uint32_t k) { return k < t.nleaves; }
@@ -1431,62 +1428,27 @@ __device__ __forceinline__ bool bt_leaf(const BinTree& t, uint32_t k) { return k
 // stands for any internal node).
 __device__ __forceinline__ uint32_t bt_cnt(const BinTree& t, uint32_t k) {
   if (t.leaf_max == 1) return bt_leaf(t, k) ? 1u : 2u;
-  return t.cnt[k];
+  return bt_leaf(t, k) ? 1u : t.cnt[k];
 }
-__device__ __forceinline__ uint32_t bt_left(const BinTree& t, uint32_t k) { return __float_as_uint(t.lo[k].w); }
-__device__ __forceinline__ uint32_t bt_right(const BinTree& t, uint32_t k) { return __float_as_uint(t.hi[k].w); }
+__device__ __forceinline__ uint32_t bt_left(const BinTree& t, uint32_t k) { return __float_as_uint(t.box[2 * (size_t)k].w); }
+__device__ __forceinline__ uint32_t bt_right(const BinTree& t, uint32_t k) { return __float_as_uint(t.box[2 * (size_t)k + 1].w); }
 __device__ __forceinline__ float3 bt_lo(const BinTree& t, uint32_t k) {
-  const float4 a = t.lo[k];
+  const float4 a = t.box[2 * (size_t)k];
   return make_float3(a.x, a.y, a.z);
 }
 __device__ __forceinline__ float3 bt_hi(const BinTree& t, uint32_t k) {
-  const float4 a = t.hi[k];
+  const float4 a = t.box[2 * (size_t)k + 1];
   return make_float3(a.x, a.y, a.z);
 }
 
 
-__device__ __forceinline__ uint32_t dp_choice(const BinTree& t, uint32_t n, int i) {
-  const uint2 c = t.choice[n];
-  const uint32_t w = i - 1 < 4 ? c.x : c.y;
-  return (w >> (8 * ((i - 1) & 3))) & 0xFFu;
-}
-
-// Children of the wide node made from binary node b by the recorded DP splits.
-__device__ int gather_children_dp(const BinTree& t, uint32_t b, uint32_t kids[8]) {
-  uint32_t sn[8];
-  int si[8];
-  int sp = 0, nk = 0;
-  const uint32_t k8 = dp_choice(t, b, 1);  // byte 0: split of D(b, 8)
-  sn[sp] = bt_left(t, b);
-  si[sp++] = (int)k8;
-  sn[sp] = bt_right(t, b);
-  si[sp++] = 8 - (int)k8;
-  while (sp > 0) {
-    const uint32_t n = sn[--sp];
-    int i = si[sp];
-    while (i > 1 && (bt_leaf(t, n) || dp_choice(t, n, i) == 0)) i--;
-    // the slots of the pending entries and the emitted children sum to at most
-    // 8, so a split always fits; the capacity test only guards the stack
-    if (i <= 1 || nk + sp + 2 > 8) {
-      if (nk < 8) kids[nk++] = n;
-      continue;
-    }
-    const int k = (int)dp_choice(t, n, i);
-    sn[sp] = bt_left(t, n);
-    si[sp++] = k;
-    sn[sp] = bt_right(t, n);
-    si[sp++] = i - k;
-  }
-  return nk;
-}
-
-// Chooses up to 8 children for the wide node that replaces binary node b.
+// Chooses up to 8 children for the wide node that replaces binary node b, greedily
+// (gpu.collapse=greedy).
 __device__ int gather_children(const BinTree& t, uint32_t b, uint32_t kids[8]) {
   if (bt_leaf(t, b)) {
     kids[0] = b;
     return 1;
   }
-  if (t.choice) return gather_children_dp(t, b, kids);
   kids[0] = bt_left(t, b);
   kids[1] = bt_right(t, b);
   int nk = 2;
@@ -1497,7 +1459,7 @@ __device__ int gather_children(const BinTree& t, uint32_t b, uint32_t kids[8]) {
     for (int i = 0; i < nk; i++) {
       const uint32_t c = kids[i];
       if (bt_leaf(t, c)) continue;
-      const bool mand = t.cnt[c] > t.leaf_max;
+      const bool mand = bt_cnt(t, c) > t.leaf_max;
       const float A = half_area(bt_lo(t, c), bt_hi(t, c));
       if (!mand) {
         // opening a small subtree pays off only if its children's boxes
@@ -1520,13 +1482,14 @@ __device__ int gather_children(const BinTree& t, uint32_t b, uint32_t kids[8]) {
   return nk;
 }
 
-// The same by 8 lanes: lane group lane & ~7 of the warp handles binary node b (all
-// 32 lanes call it; `have` is the group's).  An entry (n, i) -- node n may take up to
-// i slots -- lives in the lane where its slots begin; a split keeps the right child
-// there and sends the left child to the lane behind the right child's slots, so
-// the children come out in the order of the serial form (right subtrees first)
-// and a wide node takes as many dependent reads as its binary subtree is deep,
-// not as it has nodes.  A live lane returns its child in `kid`; live: the group's live lanes.
+// The children of the wide node made from binary node b by the recorded decisions,
+// gathered by the 8 lanes of a lane group (all 32 lanes call it; `have` is the
+// group's).  An entry (n, i) -- node n may take up to i slots -- lives in the lane
+// where its slots begin; a split keeps the right child there and sends the left
+// child to the lane behind the right child's slots, so the children come out with
+// the right subtrees first, and a wide node takes as many dependent reads as its
+// binary subtree is deep, not as it has nodes.  A live lane returns its child in
+// `kid`; live: the group's live lanes.
 __device__ __forceinline__ void gather_group(const BinTree& t, uint32_t b, bool have, uint32_t& kid, uint32_t& live) {
   const uint32_t s = threadIdx.x & 7u, gshift = threadIdx.x & 24u;
   uint32_t n = kInvalidID, i = 0;
@@ -1534,10 +1497,10 @@ __device__ __forceinline__ void gather_group(const BinTree& t, uint32_t b, bool 
     if (bt_leaf(t, b)) {
       if (s == 0) n = b, i = 1;
     } else {
-      const uint32_t k8 = min(max(t.choice[b].x & 0xFFu, 1u), 7u);  // split of D(b, 8)
-      const uint32_t l = bt_left(t, b), r = bt_right(t, b);
-      if (s == 0) n = r, i = 8u - k8;
-      if (s == 8u - k8) n = l, i = k8;
+      const uint4 lk = t.link[b];
+      const uint32_t k8 = min(max(lk.z & 0xFFu, 1u), 7u);  // split of D(b, 8)
+      if (s == 0) n = lk.y, i = 8u - k8;
+      if (s == 8u - k8) n = lk.x, i = k8;
     }
   }
   for (;;) {
@@ -1547,11 +1510,11 @@ __device__ __forceinline__ void gather_group(const BinTree& t, uint32_t b, bool 
       if (bt_leaf(t, n)) {
         i = 1;
       } else {
-        const uint2 ch = t.choice[n];
-        left = bt_left(t, n);
-        right = bt_right(t, n);
+        const uint4 lk = t.link[n];
+        left = lk.x;
+        right = lk.y;
         for (; i > 1u; i--) {
-          k = ((i - 1u < 4u ? ch.x : ch.y) >> (8u * ((i - 1u) & 3u))) & 0xFFu;
+          k = ((i - 1u < 4u ? lk.z : lk.w) >> (8u * ((i - 1u) & 3u))) & 0xFFu;
           if (k != 0u) break;
         }
         split = i > 1u;
@@ -1583,7 +1546,7 @@ __device__ __forceinline__ void collapse_count_group(const BinTree& t, const uin
                                                      uint32_t* nt) {
   const uint32_t s = threadIdx.x & 7u, gshift = threadIdx.x & 24u;
   uint32_t kid = kInvalidID, live = 0;
-  if (t.choice) {
+  if (t.link) {
     gather_group(t, have ? items[k] : 0u, have, kid, live);
   } else {  // greedy: one lane gathers
     uint32_t kk[8];
@@ -1745,10 +1708,10 @@ __device__ __forceinline__ uint32_t exp_for(float ext) {
   return E;
 }
 
-__device__ __forceinline__ void write_tri(const GeomDesc* __restrict__ geoms, const float4* __restrict__ plo,
-                                          const float4* __restrict__ phi, uint32_t prim, TriRecord* dst, bool robust) {
-  const uint32_t gs = __float_as_uint(plo[prim].w);
-  const uint32_t j = __float_as_uint(phi[prim].w);
+__device__ __forceinline__ void write_tri(const GeomDesc* __restrict__ geoms, const float4* __restrict__ pbox,
+                                          uint32_t prim, TriRecord* dst, bool robust) {
+  const uint32_t gs = __float_as_uint(pbox[2 * (size_t)prim].w);
+  const uint32_t j = __float_as_uint(pbox[2 * (size_t)prim + 1].w);
   const GeomDesc g = geoms[gs];
   if (g.kind == 1) {  // instance leaf
     const InstBox bx = reinterpret_cast<const InstBox*>(g.verts)[j];
@@ -1802,7 +1765,7 @@ __device__ __forceinline__ void collapse_emit_group(
   float3 lo = make_float3(0.f, 0.f, 0.f), hi = lo;
   uint32_t prim = 0;  // a leaf node's primitive
   if (valid) {
-    const float4 a = t.lo[kid], b = t.hi[kid];
+    const float4 a = t.box[2 * (size_t)kid], b = t.box[2 * (size_t)kid + 1];
     lo = make_float3(a.x, a.y, a.z);
     hi = make_float3(b.x, b.y, b.z);
     prim = __float_as_uint(b.w);
@@ -2122,7 +2085,7 @@ __global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 4) k_collapse_all(
 // primitive with kLeafPrim set (kInvalidID elsewhere); a subtree's primitives
 // (at most 4) are written in depth-first order, left first.
 __global__ void __launch_bounds__(256) k_write_leaves(BinTree t, const GeomDesc* __restrict__ geoms,
-                                                      const float4* __restrict__ plo, const float4* __restrict__ phi,
+                                                      const float4* __restrict__ pbox,
                                                       const uint32_t* __restrict__ leaf_root, uint32_t ntris,
                                                       TriRecord* __restrict__ tris, uint32_t* err,
                                                       const TriRecord* __restrict__ prec) {
@@ -2133,7 +2096,7 @@ __global__ void __launch_bounds__(256) k_write_leaves(BinTree t, const GeomDesc*
   if (c & kLeafPrim) {  // one triangle: its primitive, no subtree to walk
     const uint32_t prim = c & ~kLeafPrim;
     if (prec) tris[first] = prec[prim];
-    else write_tri(geoms, plo, phi, prim, &tris[first], t.robust != 0);
+    else write_tri(geoms, pbox, prim, &tris[first], t.robust != 0);
     return;
   }
   uint32_t st[8];
@@ -2148,7 +2111,7 @@ __global__ void __launch_bounds__(256) k_write_leaves(BinTree t, const GeomDesc*
         return;
       }
       if (prec) tris[first + w] = prec[bt_right(t, x)];
-      else write_tri(geoms, plo, phi, bt_right(t, x), &tris[first + w], t.robust != 0);
+      else write_tri(geoms, pbox, bt_right(t, x), &tris[first + w], t.robust != 0);
       w++;
     } else {
       if (sp + 2 > 8) {
@@ -2315,10 +2278,9 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   GB_CHECK(arena.alloc(&d_geoms, ngeoms));
   GB_CHECK(cudaMemcpyAsync(d_geoms, h_geoms, sizeof(GeomDesc) * ngeoms, cudaMemcpyHostToDevice, st));
 
-  float4 *plo = nullptr, *phi = nullptr;
+  float4* pbox = nullptr;
   BoundsAcc* acc = nullptr;
-  GB_CHECK(arena.alloc(&plo, total));
-  GB_CHECK(arena.alloc(&phi, total));
+  GB_CHECK(arena.alloc(&pbox, 2 * (size_t)total));
   GB_CHECK(arena.alloc(&acc, 1));
   BoundsAcc h_acc;
   for (int d = 0; d < 3; d++) { h_acc.glo[d] = h_acc.clo[d] = 0xFFFFFFFFu; h_acc.ghi[d] = h_acc.chi[d] = 0u; }
@@ -2330,7 +2292,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   // leaf records in primitive order (read back by k_write_leaves)
   TriRecord* prec = nullptr;
   GB_CHECK(arena.alloc(&prec, total));
-  k_primrefs<<<grid_stride_blocks(total), 256, 0, st>>>(d_geoms, ngeoms, total, plo, phi, acc, prec,
+  k_primrefs<<<grid_stride_blocks(total), 256, 0, st>>>(d_geoms, ngeoms, total, pbox, acc, prec,
                                                         opt.robust ? 1 : 0);
   note_launches(1);
 
@@ -2344,7 +2306,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   const uint32_t nseg = segmented ? (uint32_t)ngeoms : 1u;
   if (segmented && (uint32_t)ngeoms > kMaxSegments) return cudaErrorInvalidValue;
   const bool key32 = opt.morton_bits == 30 && !segmented;  // 30-bit keys sorted as 32-bit words
-  k_morton<<<grid_stride_blocks(total), 256, 0, st>>>(plo, phi, total, acc, keys_a, vals_a, opt.morton_cube,
+  k_morton<<<grid_stride_blocks(total), 256, 0, st>>>(pbox, total, acc, keys_a, vals_a, opt.morton_cube,
                                                       segmented ? 1 : 0, opt.morton_bits == 30 ? 1 : 0,
                                                       key32 ? 1 : 0);
   note_launches(1);
@@ -2355,7 +2317,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   for (int d = 0; d < 3; d++) { out->lo[d] = ord2f(h_acc.glo[d]); out->hi[d] = ord2f(h_acc.ghi[d]); }
   if (N == 0) {
     for (int d = 0; d < 3; d++) { out->lo[d] = INFINITY; out->hi[d] = -INFINITY; }
-    arena.free(d_geoms); arena.free(plo); arena.free(phi); arena.free(acc); arena.free(prec);
+    arena.free(d_geoms); arena.free(pbox); arena.free(acc); arena.free(prec);
     arena.free(keys_a); arena.free(keys_b); arena.free(vals_a); arena.free(vals_b);
     return cudaStreamSynchronize(st);
   }
@@ -2378,7 +2340,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   }
 
   // ---- PLOC over the N valid primitives (sorted positions 0..N-1)
-  float4 *bnlo = nullptr, *bnhi = nullptr;
+  float4* bnbox = nullptr;
   uint32_t* bncnt = nullptr;
   // leaf size: explicit, or by the scene -- flat scenes (centroid box's
   // smallest extent below half the largest: heightfields, terrain) and scenes
@@ -2401,13 +2363,12 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   const uint32_t nnodes_bin = 2 * N - 1;
   // SAH-optimal collapse: the cost table is filled as PLOC creates the nodes
   float4* dp_cost = nullptr;
-  uint2* d_choice = nullptr;
+  uint4* d_link = nullptr;
   if (opt.collapse == 1) {
     GB_CHECK(arena.alloc(&dp_cost, 2 * (size_t)nnodes_bin));
-    GB_CHECK(arena.alloc(&d_choice, nnodes_bin));
+    GB_CHECK(arena.alloc(&d_link, nnodes_bin));
   }
-  GB_CHECK(arena.alloc(&bnlo, nnodes_bin));
-  GB_CHECK(arena.alloc(&bnhi, nnodes_bin));
+  GB_CHECK(arena.alloc(&bnbox, 2 * (size_t)nnodes_bin));
   GB_CHECK(arena.alloc(&bncnt, nnodes_bin));
   float4 *clo_a, *chi_a, *clo_b, *chi_b;
   uint32_t *cidx_a, *cidx_b, *nn;
@@ -2419,7 +2380,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   GB_CHECK(arena.alloc(&cidx_b, N));
   GB_CHECK(arena.alloc(&nn, N));
   const uint32_t leaf_max_used = (uint32_t)std::min(std::max(leaf_max, 1), kLeafMaxLimit);
-  k_ploc_init<<<cdiv(N, 256), 256, 0, st>>>(plo, phi, vals_a, N, &acc->nvalid, bnlo, bnhi, bncnt, cidx_a, clo_a,
+  k_ploc_init<<<cdiv(N, 256), 256, 0, st>>>(pbox, vals_a, N, &acc->nvalid, bnbox, cidx_a, clo_a,
                                             chi_a, segmented ? 1 : 0);
   note_launches(1);
   uint32_t *bsurv, *bmerge, *d_tot, *d_root, *d_iters;
@@ -2460,8 +2421,8 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
     k_ploc_count<<<grid, PLOC_BLOCK, 0, st>>>(nn, ploc_state, bsurv, bmerge);
     note_launches(2);
     scan_excl2(bsurv, bmerge, maxb, d_tot + 0, d_tot + 1, scan_sums, st, &acc->pad, ploc_state + kPlocTiles);
-    k_ploc_emit<<<grid, PLOC_BLOCK, 0, st>>>(pb, nn, ploc_state, bsurv, bmerge, bnlo, bnhi, bncnt, nnodes_bin,
-                                             &acc->pad, dp_cost, d_choice, leaf_max_used);
+    k_ploc_emit<<<grid, PLOC_BLOCK, 0, st>>>(pb, nn, ploc_state, bsurv, bmerge, bnbox, bncnt, nnodes_bin,
+                                             &acc->pad, dp_cost, d_link, leaf_max_used);
     k_ploc_advance<<<1, 32, 0, st>>>(d_tot, ploc_state);
     note_launches(2);
     round++;
@@ -2483,9 +2444,8 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   {
     const size_t smem = kPlocSmallSmem;
     GB_CHECK(cudaFuncSetAttribute(k_ploc_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_ploc_small<<<1, PLOC_SMALL_THREADS, smem, st>>>(clo_a, chi_a, cidx_a, clo_b, chi_b, cidx_b, ploc_state, bnlo,
-                                                      bnhi, bncnt, d_root, d_iters, nnodes_bin, &acc->pad, nseg,
-                                                      radius, dp_cost, d_choice, leaf_max_used);
+    k_ploc_small<<<1, PLOC_SMALL_THREADS, smem, st>>>(clo_a, chi_a, cidx_a, clo_b, chi_b, cidx_b, ploc_state, bnbox, bncnt, d_root, d_iters, nnodes_bin, &acc->pad, nseg,
+                                                      radius, dp_cost, d_link, leaf_max_used);
     note_launches(1);
     GB_CHECK(cudaGetLastError());
   }
@@ -2514,7 +2474,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   arena.free(nn); arena.free(bsurv); arena.free(bmerge); arena.free(ploc_state);
 
   // ---- collapse, level by level (breadth-first node order)
-  BinTree bt{bnlo, bnhi, bncnt, N, leaf_max_used, (uint32_t)(opt.robust != 0), d_choice};
+  BinTree bt{bnbox, bncnt, N, leaf_max_used, (uint32_t)(opt.robust != 0), d_link};
   if (dp_cost) arena.free(dp_cost);
   WideNode* wnodes = nullptr;
   TriRecord* wtris = nullptr;
@@ -2574,7 +2534,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   }
   const uint32_t num_nodes = level_base, depth = (uint32_t)level_start.size();
   const uint32_t tri_next = level < 1 ? 0u : h_col[kColTri];
-  k_write_leaves<<<cdiv(N, 256), 256, 0, st>>>(bt, d_geoms, plo, phi, leaf_root, N, wtris, &acc->pad, prec);
+  k_write_leaves<<<cdiv(N, 256), 256, 0, st>>>(bt, d_geoms, pbox, leaf_root, N, wtris, &acc->pad, prec);
   note_launches(1);
   GB_CHECK(cudaGetLastError());
   arena.free(leaf_root);
@@ -2603,10 +2563,10 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   arena.free(wnodes); arena.free(wtris);
   arena.free(items_a); arena.free(items_b); arena.free(kids);
   arena.free(nint); arena.free(ntri); arena.free(d_sah); arena.free(d_leaves);
-  if (d_choice) arena.free(d_choice);
+  if (d_link) arena.free(d_link);
   arena.free(d_tot); arena.free(d_root); arena.free(d_iters); arena.free(scan_sums);
-  arena.free(bnlo); arena.free(bnhi); arena.free(bncnt);
-  arena.free(plo); arena.free(phi); arena.free(acc); arena.free(d_geoms); arena.free(prec);
+  arena.free(bnbox); arena.free(bncnt);
+  arena.free(pbox); arena.free(acc); arena.free(d_geoms); arena.free(prec);
   arena.free(keys_a); arena.free(keys_b); arena.free(vals_a); arena.free(vals_b);
   GB_CHECK(cudaEventRecord(ev1, st));
   GB_CHECK(cudaStreamSynchronize(st));
@@ -2734,10 +2694,10 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk, PLOC_BLOCK, 0)) != cudaSuccess) return e;
     g->ploc_grid = (uint32_t)std::max(1, std::min(per_sm, 8)) * (uint32_t)num_sms_build();
   }
-  if ((e = alloc(&g->d_geoms, ngeoms)) || (e = alloc(&g->plo, T)) || (e = alloc(&g->phi, T)) ||
+  if ((e = alloc(&g->d_geoms, ngeoms)) || (e = alloc(&g->pbox, 2 * (size_t)T)) ||
       (e = alloc(&acc, 1)) || (e = alloc(&g->keys_a, T)) || (e = alloc(&g->keys_b, T)) ||
       (e = alloc(&g->vals_a, T)) || (e = alloc(&g->vals_b, T)) || (e = alloc(&g->hist, sort_hist_entries(T))) ||
-      (e = alloc(&g->bnlo, 2 * (size_t)N)) || (e = alloc(&g->bnhi, 2 * (size_t)N)) ||
+      (e = alloc(&g->bnbox, 4 * (size_t)N)) ||
       (e = alloc(&g->bncnt, 2 * (size_t)N)) || (e = alloc(&g->clo[0], N)) || (e = alloc(&g->clo[1], N)) ||
       (e = alloc(&g->chi[0], N)) || (e = alloc(&g->chi[1], N)) || (e = alloc(&g->cidx[0], N)) ||
       (e = alloc(&g->cidx[1], N)) || (e = alloc(&g->nn, N)) || (e = alloc(&g->bsurv, g->maxb)) ||
@@ -2745,7 +2705,7 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
       (e = alloc(&g->scan_sums, 2 * (size_t)scan_scratch(std::max(g->maxb, maxw)))) ||
       (e = alloc(&g->d_tot, 4)) || (e = alloc(&g->d_root, g->nseg)) || (e = alloc(&g->d_iters, 1)) ||
       (e = alloc(&g->ploc_state, kPlocStateWords)) || (e = alloc(&g->cost, 2 * (size_t)(2 * N))) ||
-      (e = alloc(&g->choice, 2 * N)) || (e = alloc(&g->nodes, maxw)) || (e = alloc(&g->tris, N)) ||
+      (e = alloc(&g->link, 2 * (size_t)N)) || (e = alloc(&g->nodes, maxw)) || (e = alloc(&g->tris, N)) ||
       (e = alloc(&g->items[0], maxw)) || (e = alloc(&g->items[1], maxw)) || (e = alloc(&g->kids, 8 * (size_t)maxw)) ||
       (e = alloc(&g->nint, maxw)) || (e = alloc(&g->ntri, maxw)) || (e = alloc(&g->leaf_root, N)) ||
       (e = alloc(&g->d_sah, 2)) || (e = alloc(&g->d_leaves, 1)) || (e = alloc(&g->cstate, kColStateWords)) ||
@@ -2783,10 +2743,10 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   };
   stamp(0);
   k_acc_init<<<1, 32, 0, st>>>(acc);
-  k_primrefs<<<grid_stride_blocks(T), 256, 0, st>>>(g.d_geoms, g.ngeoms, T, g.plo, g.phi, acc, g.prec,
+  k_primrefs<<<grid_stride_blocks(T), 256, 0, st>>>(g.d_geoms, g.ngeoms, T, g.pbox, acc, g.prec,
                                                     g.opt.robust ? 1 : 0);
   const bool key32 = g.opt.morton_bits == 30 && !g.opt.segmented;  // 30-bit keys sorted as 32-bit words
-  k_morton<<<grid_stride_blocks(T), 256, 0, st>>>(g.plo, g.phi, T, acc, g.keys_a, g.vals_a, g.opt.morton_cube,
+  k_morton<<<grid_stride_blocks(T), 256, 0, st>>>(g.pbox, T, acc, g.keys_a, g.vals_a, g.opt.morton_cube,
                                                   g.opt.segmented ? 1 : 0, g.opt.morton_bits == 30 ? 1 : 0,
                                                   key32 ? 1 : 0);
   note_launches(3);
@@ -2809,8 +2769,8 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   GB_CHECK(cudaMemsetAsync(g.d_iters, 0, sizeof(uint32_t), st));
   const uint32_t leaf_max = (uint32_t)std::min(std::max(g.plan.leaf_max, 1), kLeafMaxLimit);
   float4* dp_cost = g.opt.collapse == 1 ? g.cost : nullptr;
-  uint2* dp_choice = g.opt.collapse == 1 ? g.choice : nullptr;
-  k_ploc_init<<<cdiv(N, 256), 256, 0, st>>>(g.plo, g.phi, va, N, &acc->nvalid, g.bnlo, g.bnhi, g.bncnt, g.cidx[0],
+  uint4* dp_link = g.opt.collapse == 1 ? g.link : nullptr;
+  k_ploc_init<<<cdiv(N, 256), 256, 0, st>>>(g.pbox, va, N, &acc->nvalid, g.bnbox, g.cidx[0],
                                             g.clo[0], g.chi[0], g.opt.segmented ? 1 : 0);
   stamp(3);
   k_ploc_state_init<<<1, 32, 0, st>>>(acc, g.ploc_state);
@@ -2833,19 +2793,19 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(g.ploc_bar);
     switch (g.radius) {
       case 1: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<1>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
-                                          g.bnlo, g.bnhi, g.bncnt, nbin_cap, dp_cost, dp_choice, leaf_max, bar,
+                                          g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar,
                                           &acc->pad)); break;
       case 2: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<2>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
-                                          g.bnlo, g.bnhi, g.bncnt, nbin_cap, dp_cost, dp_choice, leaf_max, bar,
+                                          g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar,
                                           &acc->pad)); break;
       case 4: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<4>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
-                                          g.bnlo, g.bnhi, g.bncnt, nbin_cap, dp_cost, dp_choice, leaf_max, bar,
+                                          g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar,
                                           &acc->pad)); break;
       case 8: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<8>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
-                                          g.bnlo, g.bnhi, g.bncnt, nbin_cap, dp_cost, dp_choice, leaf_max, bar,
+                                          g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar,
                                           &acc->pad)); break;
       default: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<PLOC_R_MAX>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge,
-                                           g.ploc_sums, g.bnlo, g.bnhi, g.bncnt, nbin_cap, dp_cost, dp_choice,
+                                           g.ploc_sums, g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link,
                                            leaf_max, bar, &acc->pad)); break;
     }
     note_launches(2);
@@ -2854,14 +2814,14 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   {
     const size_t smem = kPlocSmallSmem;
     k_ploc_small<<<1, PLOC_SMALL_THREADS, smem, st>>>(g.clo[0], g.chi[0], g.cidx[0], g.clo[1], g.chi[1], g.cidx[1],
-                                                      g.ploc_state, g.bnlo, g.bnhi, g.bncnt, g.d_root, g.d_iters,
-                                                      nbin_cap, &acc->pad, g.nseg, (int)g.radius, dp_cost, dp_choice,
+                                                      g.ploc_state, g.bnbox, g.bncnt, g.d_root, g.d_iters,
+                                                      nbin_cap, &acc->pad, g.nseg, (int)g.radius, dp_cost, dp_link,
                                                       leaf_max);
     note_launches(1);
   }
   stamp(5);
   // collapse decisions and levels
-  BinTree bt{g.bnlo, g.bnhi, g.bncnt, N, leaf_max, (uint32_t)(g.opt.robust != 0), dp_choice};
+  BinTree bt{g.bnbox, g.bncnt, N, leaf_max, (uint32_t)(g.opt.robust != 0), dp_link};
   GB_CHECK(cudaMemsetAsync(g.leaf_root, 0xFF, sizeof(uint32_t) * N, st));
   GB_CHECK(cudaMemsetAsync(g.d_sah, 0, 2 * sizeof(double), st));
   GB_CHECK(cudaMemsetAsync(g.d_leaves, 0, sizeof(uint32_t), st));
@@ -2889,7 +2849,7 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   }
   note_launches(2);
   stamp(7);
-  k_write_leaves<<<cdiv(N, 256), 256, 0, st>>>(bt, g.d_geoms, g.plo, g.phi, g.leaf_root, N, g.tris, &acc->pad,
+  k_write_leaves<<<cdiv(N, 256), 256, 0, st>>>(bt, g.d_geoms, g.pbox, g.leaf_root, N, g.tris, &acc->pad,
                                                 g.prec);
   stamp(8);
   k_graph_build_check<<<1, 128, 0, st>>>(acc, g.ploc_state, g.cstate, N, g.d_sah, g.d_leaves, g.seg_index, g.nseg,

@@ -70,15 +70,15 @@ struct GraphBuild {
   uint32_t total = 0, nseg = 1, nbin = 0, maxw = 0, maxb = 0, rs_blocks = 0, radius = 1;
   std::vector<void*> allocs;  // every device allocation (released by graph_build_release)
   GeomDesc* d_geoms = nullptr;
-  float4 *plo = nullptr, *phi = nullptr;
+  float4* pbox = nullptr;     // primitive boxes, two words each
   void* acc = nullptr;
   uint64_t *keys_a = nullptr, *keys_b = nullptr;
   uint32_t *vals_a = nullptr, *vals_b = nullptr, *hist = nullptr;
-  float4 *bnlo = nullptr, *bnhi = nullptr, *clo[2] = {nullptr, nullptr}, *chi[2] = {nullptr, nullptr};
+  float4 *bnbox = nullptr, *clo[2] = {nullptr, nullptr}, *chi[2] = {nullptr, nullptr};
   uint32_t *bncnt = nullptr, *cidx[2] = {nullptr, nullptr}, *nn = nullptr, *bsurv = nullptr, *bmerge = nullptr;
   uint32_t *scan_sums = nullptr, *d_tot = nullptr, *d_root = nullptr, *d_iters = nullptr, *ploc_state = nullptr;
   float4* cost = nullptr;
-  uint2* choice = nullptr;
+  uint4* link = nullptr;
   WideNode* nodes = nullptr;
   TriRecord* tris = nullptr;
   uint32_t *items[2] = {nullptr, nullptr}, *kids = nullptr, *nint = nullptr, *ntri = nullptr, *leaf_root = nullptr;
