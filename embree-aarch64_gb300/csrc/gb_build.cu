@@ -883,7 +883,7 @@ __global__ void k_ploc_state_init(const BoundsAcc* __restrict__ acc, uint32_t* _
 // side, same segment) of every cluster of one PLOC_BLOCK tile; the window with
 // its halo is staged in shared memory.
 template <int PLOC_R>
-__device__ __forceinline__ void ploc_nn_tile(const float4* __restrict__ clo, const float4* __restrict__ chi, uint32_t n,
+__device__ __forceinline__ void ploc_nn_tile(const float4* clo, const float4* chi, uint32_t n,
                                              uint32_t tile, uint32_t* __restrict__ nn, float3* s_lo, float3* s_hi,
                                              uint32_t* s_seg) {
   const int base = (int)(tile * PLOC_BLOCK);
@@ -919,7 +919,7 @@ __device__ __forceinline__ void ploc_nn_tile(const float4* __restrict__ clo, con
 // halo clusters just outside a CTA's run of tiles; bit-identical to the tile
 // form: same boxes, same area arithmetic, the least (area, index) key).
 template <int PLOC_R>
-__device__ __forceinline__ uint32_t ploc_nn_one(const float4* __restrict__ clo, const float4* __restrict__ chi,
+__device__ __forceinline__ uint32_t ploc_nn_one(const float4* clo, const float4* chi,
                                                 uint32_t n, int h) {
   const float4 a = clo[h], b = chi[h];
   const float3 lo = make_float3(a.x, a.y, a.z), hi = make_float3(b.x, b.y, b.z);
@@ -985,6 +985,46 @@ __device__ __forceinline__ uint32_t block_excl_scan_flag(int flag, uint32_t* s_w
   return pre + __popc(bal & ((1u << lane) - 1u));
 }
 
+// Output of cluster i at position pos of the next round: itself (j == i), or the
+// new node `id` that merges it with cluster j, whose collapse costs are computed
+// here.
+__device__ __forceinline__ void ploc_emit_one(const PlocBufs& bufs, uint32_t par, uint32_t i, uint32_t j, uint32_t pos,
+                                              uint32_t id, uint32_t n, float4* __restrict__ bnbox,
+                                              uint32_t* __restrict__ bncnt, uint32_t node_cap, uint32_t* err,
+                                              float4* __restrict__ dp_cost, uint4* __restrict__ dp_link,
+                                              uint32_t leaf_max) {
+  const float4 *clo = bufs.clo[par], *chi = bufs.chi[par];
+  const uint32_t* cidx = bufs.cidx[par];
+  float4 lo = clo[i], hi = chi[i];
+  uint32_t out = cidx[i];
+  if (pos >= n) {
+    atomicOr(err, kErrBuild);
+    return;
+  }
+  if (j != i) {
+    const float4 a = lo, b = hi, c = clo[j], d = chi[j];
+    const uint32_t l = out, r = cidx[j];
+    if (id >= node_cap) {
+      atomicOr(err, kErrBuild);
+      return;
+    }
+    lo = make_float4(fminf(a.x, c.x), fminf(a.y, c.y), fminf(a.z, c.z), a.w);
+    const uint32_t cnt_l = __float_as_uint(b.w), cnt_r = __float_as_uint(d.w);
+    hi = make_float4(fmaxf(b.x, d.x), fmaxf(b.y, d.y), fmaxf(b.z, d.z), __uint_as_float(cnt_l + cnt_r));
+    bnbox[2 * (size_t)id] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
+    bnbox[2 * (size_t)id + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
+    bncnt[id] = cnt_l + cnt_r;
+    if (dp_cost)
+      dp_node(dp_cost, dp_link, id, l, r, half_area(make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z)),
+              cnt_l, cnt_r, cnt_l == 1 ? half_area(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z)) : 0.f,
+              cnt_r == 1 ? half_area(make_float3(c.x, c.y, c.z), make_float3(d.x, d.y, d.z)) : 0.f, leaf_max);
+    out = id;
+  }
+  bufs.clo[par ^ 1u][pos] = lo;
+  bufs.chi[par ^ 1u][pos] = hi;
+  bufs.cidx[par ^ 1u][pos] = out;
+}
+
 // Survivors and merges of one tile: a cluster whose nearest neighbour is
 // mutual merges with it (the lower index creates the node, the higher one is
 // dropped), the others survive as they are; outputs go to position
@@ -996,12 +1036,6 @@ __device__ __forceinline__ void ploc_emit_tile(const PlocBufs& bufs, uint32_t pa
                                                uint32_t* __restrict__ bncnt,
                                                uint32_t node_cap, uint32_t* err, float4* __restrict__ dp_cost,
                                                uint4* __restrict__ dp_link, uint32_t leaf_max, uint32_t* s_w) {
-  const float4* __restrict__ clo = bufs.clo[par];
-  const float4* __restrict__ chi = bufs.chi[par];
-  const uint32_t* __restrict__ cidx = bufs.cidx[par];
-  float4* __restrict__ olo = bufs.clo[par ^ 1u];
-  float4* __restrict__ ohi = bufs.chi[par ^ 1u];
-  uint32_t* __restrict__ oidx = bufs.cidx[par ^ 1u];
   const uint32_t i = tile * PLOC_BLOCK + threadIdx.x;
   int surv = 0, merge = 0;
   uint32_t j = 0;
@@ -1014,38 +1048,8 @@ __device__ __forceinline__ void ploc_emit_tile(const PlocBufs& bufs, uint32_t pa
   const uint32_t rs = block_excl_scan_flag(surv, s_w);
   const uint32_t rm = block_excl_scan_flag(merge, s_w);
   if (i >= n || !surv) return;
-  const uint32_t pos = surv_off + rs;
-  const float4 a = clo[i], b = chi[i];
-  if (pos >= n) {
-    atomicOr(err, kErrBuild);
-    return;
-  }
-  if (merge) {
-    const float4 c = clo[j], d = chi[j];
-    const uint32_t id = node_next + merge_off + rm;
-    if (id >= node_cap) {
-      atomicOr(err, kErrBuild);
-      return;
-    }
-    const uint32_t l = cidx[i], r = cidx[j];
-    const float4 lo = make_float4(fminf(a.x, c.x), fminf(a.y, c.y), fminf(a.z, c.z), a.w);
-    const uint32_t cnt_l = __float_as_uint(b.w), cnt_r = __float_as_uint(d.w);
-    const float4 hi = make_float4(fmaxf(b.x, d.x), fmaxf(b.y, d.y), fmaxf(b.z, d.z), __uint_as_float(cnt_l + cnt_r));
-    bnbox[2 * (size_t)id] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
-    bnbox[2 * (size_t)id + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
-    bncnt[id] = cnt_l + cnt_r;
-    if (dp_cost)
-      dp_node(dp_cost, dp_link, id, l, r, half_area(make_float3(lo.x, lo.y, lo.z), make_float3(hi.x, hi.y, hi.z)),
-              cnt_l, cnt_r, cnt_l == 1 ? half_area(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z)) : 0.f,
-              cnt_r == 1 ? half_area(make_float3(c.x, c.y, c.z), make_float3(d.x, d.y, d.z)) : 0.f, leaf_max);
-    olo[pos] = lo;
-    ohi[pos] = hi;
-    oidx[pos] = id;
-  } else {
-    olo[pos] = a;
-    ohi[pos] = b;
-    oidx[pos] = cidx[i];
-  }
+  ploc_emit_one(bufs, par, i, merge ? j : i, surv_off + rs, node_next + merge_off + rm, n, bnbox, bncnt, node_cap, err,
+                dp_cost, dp_link, leaf_max);
 }
 
 __global__ void __launch_bounds__(PLOC_BLOCK) k_ploc_emit(const PlocBufs bufs, const uint32_t* __restrict__ nn,
@@ -1182,6 +1186,183 @@ __global__ void __launch_bounds__(PLOC_BLOCK) k_ploc_all(const PlocBufs bufs, ui
                      leaf_max, s_w);
       ps += tile_s[tile];
       pm += tile_m[tile];
+    }
+    // next round (the k_ploc_advance rules, alike in every CTA)
+    const uint32_t merged = v[3];
+    n = v[2];
+    node_next += merged;
+    rounds += merged > 0 ? 1u : 0u;
+    par ^= 1u;
+    iters++;
+    if (n <= PLOC_SMALL || merged == 0) done = true;
+    if (!grid_sync(bar, err)) break;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ploc_state[kPlocN] = n;
+    ploc_state[kPlocNext] = node_next;
+    ploc_state[kPlocRounds] = rounds;
+    ploc_state[kPlocTiles] = (n + PLOC_BLOCK - 1) / PLOC_BLOCK;
+    ploc_state[kPlocParity] = par;
+    ploc_state[kPlocDone] = done ? 1u : 0u;
+    ploc_state[kPlocIters] = iters;
+  }
+}
+
+// Area of the box around clusters j and j + 1; infinite where they are no
+// neighbours (the ends, another segment).
+__device__ __forceinline__ float ploc_adjacent(const float4* clo, const float4* chi, uint32_t n, int j) {
+  if (j < 0 || j + 1 >= (int)n) return INFINITY;
+  const float4 a = clo[j], b = chi[j], c = clo[j + 1], d = chi[j + 1];
+  if (__float_as_uint(a.w) != __float_as_uint(c.w)) return INFINITY;
+  return half_area(f3min(make_float3(a.x, a.y, a.z), make_float3(c.x, c.y, c.z)),
+                   f3max(make_float3(b.x, b.y, b.z), make_float3(d.x, d.y, d.z)));
+}
+
+// Exclusive block scan of two values (a, b); returns (prefix a, prefix b) and
+// the block totals in *ta, *tb.  All 256 threads call it.
+__device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32_t* ta, uint32_t* tb) {
+  __shared__ uint32_t s_a[8], s_b[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t xa = a, xb = b;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t ya = __shfl_up_sync(0xFFFFFFFFu, xa, o), yb = __shfl_up_sync(0xFFFFFFFFu, xb, o);
+    if (lane >= o) {
+      xa += ya;
+      xb += yb;
+    }
+  }
+  if (lane == 31) {
+    s_a[warp] = xa;
+    s_b[warp] = xb;
+  }
+  __syncthreads();
+  uint32_t oa = 0, ob = 0, sa = 0, sb = 0;
+#pragma unroll
+  for (int w = 0; w < 8; w++) {
+    if (w < warp) {
+      oa += s_a[w];
+      ob += s_b[w];
+    }
+    sa += s_a[w];
+    sb += s_b[w];
+  }
+  __syncthreads();  // s_a, s_b are reused by the next call
+  *ta = sa;
+  *tb = sb;
+  return make_uint2(oa + xa - a, ob + xb - b);
+}
+
+// k_ploc_all for radius 1.  With one neighbour on either side a cluster's nearest
+// neighbour is the side of the smaller adjacent area (the left one in a tie, the
+// least (area, index)), so clusters i and i + 1 merge exactly where the adjacent
+// areas have a local minimum: a[i - 1] > a[i] <= a[i + 1].  That needs no window in
+// shared memory: the warps of a CTA take the 32-cluster tiles of its run in turn,
+// (1) the merges of a tile as a bit mask from shuffles and a ballot, the run's
+// offsets by one block scan over the tiles, [barrier], (2) the tiles' outputs,
+// [barrier].  The tile-per-CTA form waits at six CTA barriers per 256 clusters,
+// which the threads that compute collapse costs reach last (17 of its 29 stall
+// cycles per issue).  tile_m, tile_s, tile_p: one word per tile.  Rounds of the 4M
+// soup: 732 us before, 581 us so (600 with a run of tiles per warp).
+__global__ void __launch_bounds__(PLOC_BLOCK, 4)
+    k_ploc_rounds1(const PlocBufs bufs, uint32_t* __restrict__ ploc_state, uint32_t* tile_m, uint32_t* tile_s,
+                   uint32_t* tile_p, uint32_t* cta_sums, float4* __restrict__ bnbox, uint32_t* __restrict__ bncnt,
+                   uint32_t node_cap, float4* __restrict__ dp_cost, uint4* __restrict__ dp_link, uint32_t leaf_max,
+                   GridBarrier* bar, unsigned int* err) {
+  constexpr uint32_t kWarps = PLOC_BLOCK / 32;
+  __shared__ uint32_t s_red[4][kWarps];
+  __shared__ uint32_t s_before;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  uint32_t n = __ldcg(ploc_state + kPlocN), node_next = __ldcg(ploc_state + kPlocNext);
+  uint32_t par = __ldcg(ploc_state + kPlocParity) & 1u, rounds = __ldcg(ploc_state + kPlocRounds);
+  uint32_t iters = __ldcg(ploc_state + kPlocIters);
+  bool done = __ldcg(ploc_state + kPlocDone) != 0u;
+  while (!done && iters < kPlocMaxIters) {
+    const float4 *clo = bufs.clo[par], *chi = bufs.chi[par];
+    const uint32_t ntiles = (n + 31u) / 32u;
+    const uint32_t per = (ntiles + gridDim.x - 1) / gridDim.x;
+    const uint32_t t0 = min(blockIdx.x * per, ntiles), t1 = min(t0 + per, ntiles);
+    // (1) merges of the run's tiles
+    for (uint32_t t = t0 + warp; t < t1; t += kWarps) {
+      const int i = (int)(32u * t + lane);
+      const float a = ploc_adjacent(clo, chi, n, i);
+      const float edge = lane < 2u ? ploc_adjacent(clo, chi, n, lane ? (int)(32u * t) + 32 : (int)(32u * t) - 1) : 0.f;
+      float left = __shfl_up_sync(0xFFFFFFFFu, a, 1), right = __shfl_down_sync(0xFFFFFFFFu, a, 1);
+      const float e0 = __shfl_sync(0xFFFFFFFFu, edge, 0), e1 = __shfl_sync(0xFFFFFFFFu, edge, 1);
+      if (lane == 0) left = e0;
+      if (lane == 31) right = e1;
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, a != INFINITY && a < left && a <= right);
+      if (lane == 0) tile_m[t] = m;
+    }
+    if (warp == 0 && t0 < t1) {  // whether the pair across the run's start merges
+      const float a = lane < 3u ? ploc_adjacent(clo, chi, n, (int)(32u * t0) - 2 + (int)lane) : 0.f;
+      const float b = __shfl_sync(0xFFFFFFFFu, a, 0), c = __shfl_sync(0xFFFFFFFFu, a, 1), d = __shfl_sync(0xFFFFFFFFu, a, 2);
+      if (lane == 0) s_before = c != INFINITY && c < b && c <= d ? 1u : 0u;
+    }
+    __syncthreads();
+    const uint32_t before = s_before;
+    uint32_t ps = 0, pm = 0;
+    for (uint32_t k0 = t0; k0 < t1; k0 += PLOC_BLOCK) {
+      const uint32_t t = k0 + threadIdx.x;
+      uint32_t a = 0, b = 0;
+      if (t < t1) {
+        const uint32_t m = tile_m[t], carry = t > t0 ? tile_m[t - 1] >> 31 : before;
+        a = min(n - 32u * t, 32u) - __popc(m << 1) - carry;
+        b = __popc(m);
+      }
+      uint32_t ta, tb;
+      const uint2 e = block_excl_scan2(a, b, &ta, &tb);
+      if (t < t1) {
+        tile_s[t] = ps + e.x;
+        tile_p[t] = pm + e.y;
+      }
+      ps += ta;
+      pm += tb;
+    }
+    if (threadIdx.x == 0) {
+      __stcg(cta_sums + blockIdx.x, ps);
+      __stcg(cta_sums + gridDim.x + blockIdx.x, pm);
+    }
+    if (!grid_sync(bar, err)) break;
+    // (2) this CTA's offsets and the round's totals, then its tiles' outputs
+    uint32_t v[4] = {0u, 0u, 0u, 0u};  // prefix survivors, prefix merges, total survivors, total merges
+    for (uint32_t c0 = threadIdx.x; c0 < gridDim.x; c0 += 4 * PLOC_BLOCK) {
+      uint32_t a[4], b[4];  // read together
+#pragma unroll
+      for (uint32_t q = 0; q < 4; q++) {
+        const uint32_t c = c0 + q * PLOC_BLOCK;
+        a[q] = c < gridDim.x ? __ldcg(cta_sums + c) : 0u;
+        b[q] = c < gridDim.x ? __ldcg(cta_sums + gridDim.x + c) : 0u;
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < 4; q++) {
+        v[2] += a[q];
+        v[3] += b[q];
+        if (c0 + q * PLOC_BLOCK < blockIdx.x) {
+          v[0] += a[q];
+          v[1] += b[q];
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      v[q] = __reduce_add_sync(0xFFFFFFFFu, v[q]);
+      if (lane == 0) s_red[q][warp] = v[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      v[q] = 0;
+      for (uint32_t w = 0; w < kWarps; w++) v[q] += s_red[q][w];
+    }
+    for (uint32_t t = t0 + warp; t < t1; t += kWarps) {
+      const uint32_t m = tile_m[t], i = 32u * t + lane, carry = t > t0 ? tile_m[t - 1] >> 31 : before;
+      const uint32_t s0 = tile_s[t], m0 = tile_p[t];
+      const uint32_t in = min(n - 32u * t, 32u), absorbed = (m << 1) | carry;
+      const uint32_t alive = (in == 32u ? 0xFFFFFFFFu : (1u << in) - 1u) & ~absorbed;
+      if (alive >> lane & 1u)
+        ploc_emit_one(bufs, par, i, m >> lane & 1u ? i + 1u : i, v[0] + s0 + __popc(alive & lt),
+                      node_next + v[1] + m0 + __popc(m & lt), n, bnbox, bncnt, node_cap, err, dp_cost, dp_link, leaf_max);
     }
     // next round (the k_ploc_advance rules, alike in every CTA)
     const uint32_t merged = v[3];
@@ -1383,6 +1564,183 @@ __global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_small(const float4*
   }
 }
 
+// k_ploc_small for radius 1, where clusters merge at the local minima of the
+// adjacent areas (k_ploc_rounds1).  A round of one CTA is a chain of steps between
+// barriers, so the new nodes' collapse costs -- two dependent L2 reads and 28
+// sums, the longest step -- are left to the next round, which reads them while it
+// works on its own areas and merges.  The last 4,096 clusters of the 4M soup:
+// 174 us with the costs inside the round, 90 us so.
+struct PlocTask {       // costs to compute: node task_base + index
+  uint32_t l, r;        // children
+  float A, Al, Ar;      // areas (Al, Ar: of primitive children)
+  uint32_t cnt;         // triangles of the children, 255 at most, 8 bits each
+};
+constexpr size_t kPlocFinishSmem = (size_t)PLOC_SMALL * (2 * sizeof(float3) + 3 * sizeof(uint32_t)) +
+                                   (PLOC_SMALL + 2) * sizeof(float) + (PLOC_SMALL / 2) * sizeof(PlocTask);
+
+__global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_finish1(const PlocBufs bufs, uint32_t* __restrict__ ploc_state,
+                                                                     float4* __restrict__ bnbox,
+                                                                     uint32_t* __restrict__ bncnt, uint32_t* root_out,
+                                                                     uint32_t* iters_out, uint32_t node_cap,
+                                                                     uint32_t* err, uint32_t nseg,
+                                                                     float4* __restrict__ dp_cost,
+                                                                     uint4* __restrict__ dp_link, uint32_t leaf_max) {
+  extern __shared__ unsigned char smem[];
+  float3* s_lo = reinterpret_cast<float3*>(smem);
+  float3* s_hi = s_lo + PLOC_SMALL;
+  uint32_t* s_idx = reinterpret_cast<uint32_t*>(s_hi + PLOC_SMALL);
+  uint32_t* s_seg = s_idx + PLOC_SMALL;
+  uint32_t* s_cnt = s_seg + PLOC_SMALL;
+  float* s_area = reinterpret_cast<float*>(s_cnt + PLOC_SMALL) + 1;  // s_area[-1 .. n]: box of clusters i, i + 1
+  PlocTask* s_task = reinterpret_cast<PlocTask*>(s_area + PLOC_SMALL + 1);
+  __shared__ uint32_t s_w[32];
+  constexpr int EPT = PLOC_SMALL / PLOC_SMALL_THREADS;
+  const uint32_t n0 = ploc_state[kPlocN], node_next0 = ploc_state[kPlocNext], par = ploc_state[kPlocParity] & 1u;
+  if (n0 > PLOC_SMALL) {  // the rounds did not get below the threshold (too few enqueued)
+    if (threadIdx.x == 0) atomicOr(err, kErrBuild);
+    return;
+  }
+  for (uint32_t k = threadIdx.x; k < n0; k += blockDim.x) {
+    const float4 a = bufs.clo[par][k], b = bufs.chi[par][k];
+    s_lo[k] = make_float3(a.x, a.y, a.z);
+    s_hi[k] = make_float3(b.x, b.y, b.z);
+    s_idx[k] = bufs.cidx[par][k];
+    s_seg[k] = __float_as_uint(a.w);
+    s_cnt[k] = __float_as_uint(b.w);
+  }
+  if (threadIdx.x == 0) s_area[-1] = INFINITY;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  uint32_t n = n0, node_next = node_next0, iters = 0, tasks = 0;  // tasks: nodes of the last round
+  bool failed = false;
+  auto pay = [&](uint32_t k) {  // the collapse costs of task k
+    const PlocTask t = s_task[k];
+    dp_node(dp_cost, dp_link, node_next - tasks + k, t.l, t.r, t.A, t.cnt & 0xFFu, t.cnt >> 8, t.Al, t.Ar, leaf_max);
+  };
+  __syncthreads();
+  // every round merges at least the closest pair of each segment that still
+  // has two clusters, so n0 - 1 rounds always suffice; the bound only guards
+  // against a logic error.  A round without merges ends the clustering.
+  while (n > 1 && !failed) {
+    if (iters >= PLOC_SMALL) {
+      if (threadIdx.x == 0) atomicOr(err, kErrBuild);
+      break;
+    }
+    iters++;
+    // adjacent areas, and the costs of the last round's nodes
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+      s_area[i] = i + 1 < n && s_seg[i] == s_seg[i + 1]
+                      ? half_area(f3min(s_lo[i], s_lo[i + 1]), f3max(s_hi[i], s_hi[i + 1]))
+                      : INFINITY;
+    for (uint32_t k = threadIdx.x; k < tasks; k += blockDim.x) pay(k);
+    __syncthreads();
+    // the warp's tiles of 32 clusters: merges as bit masks
+    const uint32_t per = (n + PLOC_SMALL_THREADS - 1) / PLOC_SMALL_THREADS, w0 = warp * 32u * per;
+    uint32_t mask[EPT], alive[EPT], survivors = 0, merges = 0, carry = 0;
+    if (w0 > 0 && w0 < n) {
+      const float a = s_area[w0 - 1];
+      carry = a != INFINITY && a < s_area[(int)w0 - 2] && a <= s_area[w0] ? 1u : 0u;
+    }
+#pragma unroll
+    for (int e = 0; e < EPT; e++) {
+      const uint32_t i = w0 + 32u * e + lane;
+      bool m = false;
+      if ((uint32_t)e < per && i < n) {
+        const float a = s_area[i];
+        m = a != INFINITY && a < s_area[(int)i - 1] && a <= s_area[i + 1];
+      }
+      mask[e] = __ballot_sync(0xFFFFFFFFu, m);
+      alive[e] = __ballot_sync(0xFFFFFFFFu, (uint32_t)e < per && i < n) & ~((mask[e] << 1) | carry);
+      carry = mask[e] >> 31;
+      survivors += __popc(alive[e]);
+      merges += __popc(mask[e]);
+    }
+    if (lane == 0) s_w[warp] = survivors | (merges << 16);  // both below 2^16
+    __syncthreads();
+    uint32_t x = s_w[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, x, 31);
+    const uint32_t before = __shfl_sync(0xFFFFFFFFu, x, warp ? warp - 1 : 0);
+    uint32_t ps = warp ? before & 0xFFFFu : 0u, pm = warp ? before >> 16 : 0u;
+    failed = node_next + (total >> 16) > node_cap;
+    // outputs into registers, the new nodes and their tasks
+    float3 olo[EPT], ohi[EPT];
+    uint32_t oidx[EPT], oseg[EPT], ocnt[EPT], opos[EPT];
+#pragma unroll
+    for (int e = 0; e < EPT; e++) {
+      opos[e] = 0xFFFFFFFFu;
+      if ((alive[e] >> lane & 1u) && !failed) {
+        const uint32_t i = w0 + 32u * e + lane;
+        float3 lo = s_lo[i], hi = s_hi[i];
+        uint32_t id = s_idx[i], cnt = s_cnt[i];
+        if (mask[e] >> lane & 1u) {
+          const uint32_t q = pm + __popc(mask[e] & lt), nid = node_next + q;
+          const uint32_t l = id, r = s_idx[i + 1], cnt_l = cnt, cnt_r = s_cnt[i + 1];
+          const float3 rlo = s_lo[i + 1], rhi = s_hi[i + 1];
+          PlocTask t;
+          t.l = l;
+          t.r = r;
+          t.Al = cnt_l == 1 ? half_area(lo, hi) : 0.f;
+          t.Ar = cnt_r == 1 ? half_area(rlo, rhi) : 0.f;
+          t.cnt = min(cnt_l, 255u) | (min(cnt_r, 255u) << 8);
+          lo = f3min(lo, rlo);
+          hi = f3max(hi, rhi);
+          t.A = half_area(lo, hi);
+          s_task[q] = t;
+          bnbox[2 * (size_t)nid] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(l));
+          bnbox[2 * (size_t)nid + 1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(r));
+          cnt = cnt_l + cnt_r;
+          bncnt[nid] = cnt;
+          id = nid;
+        }
+        olo[e] = lo;
+        ohi[e] = hi;
+        oidx[e] = id;
+        oseg[e] = s_seg[i];
+        ocnt[e] = cnt;
+        opos[e] = ps + __popc(alive[e] & lt);
+      }
+      ps += __popc(alive[e]);
+      pm += __popc(mask[e]);
+    }
+    __syncthreads();
+    if (failed) {
+      if (threadIdx.x == 0) atomicOr(err, kErrBuild);
+      tasks = 0;
+      break;
+    }
+#pragma unroll
+    for (int e = 0; e < EPT; e++) {
+      if (opos[e] != 0xFFFFFFFFu) {
+        s_lo[opos[e]] = olo[e];
+        s_hi[opos[e]] = ohi[e];
+        s_idx[opos[e]] = oidx[e];
+        s_seg[opos[e]] = oseg[e];
+        s_cnt[opos[e]] = ocnt[e];
+      }
+    }
+    tasks = total >> 16;
+    node_next += tasks;
+    n = total & 0xFFFFu;
+    if (!dp_cost) tasks = 0;
+    __syncthreads();
+    if ((total >> 16) == 0) break;
+  }
+  for (uint32_t k = threadIdx.x; k < tasks; k += blockDim.x) pay(k);
+  // one root per segment (nseg == 1: the single tree's root)
+  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
+    const uint32_t seg = nseg > 1 ? s_seg[k] : 0u;
+    if (seg < nseg) root_out[seg] = s_idx[k];
+  }
+  if (threadIdx.x == 0) {
+    *iters_out += iters;
+    ploc_state[kPlocNext] = node_next;  // binary nodes in use: [0, node_next)
+  }
+}
+
 // ---------------------------------------------------------------------------
 // 5. collapse to 8-wide quantised nodes
 // ---------------------------------------------------------------------------
@@ -1547,7 +1905,7 @@ __device__ __forceinline__ void collapse_count_group(const BinTree& t, const uin
   const uint32_t s = threadIdx.x & 7u, gshift = threadIdx.x & 24u;
   uint32_t kid = kInvalidID, live = 0;
   if (t.link) {
-    gather_group(t, have ? items[k] : 0u, have, kid, live);
+    gather_group(t, have ? __ldcg(items + k) : 0u, have, kid, live);
   } else {  // greedy: one lane gathers
     uint32_t kk[8];
     const int nk = have && s == 0u ? gather_children(t, items[k], kk) : 0;
@@ -1935,41 +2293,6 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_emit(
 
 constexpr int COLLAPSE_ALL_THREADS = 256;
 
-// Exclusive block scan of two values (a, b); returns (prefix a, prefix b) and
-// the block totals in *ta, *tb.  All threads call it.
-__device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32_t* ta, uint32_t* tb) {
-  __shared__ uint32_t s_a[COLLAPSE_ALL_THREADS / 32], s_b[COLLAPSE_ALL_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t xa = a, xb = b;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t ya = __shfl_up_sync(0xFFFFFFFFu, xa, o), yb = __shfl_up_sync(0xFFFFFFFFu, xb, o);
-    if (lane >= o) {
-      xa += ya;
-      xb += yb;
-    }
-  }
-  if (lane == 31) {
-    s_a[warp] = xa;
-    s_b[warp] = xb;
-  }
-  __syncthreads();
-  uint32_t oa = 0, ob = 0, sa = 0, sb = 0;
-#pragma unroll
-  for (int w = 0; w < COLLAPSE_ALL_THREADS / 32; w++) {
-    if (w < warp) {
-      oa += s_a[w];
-      ob += s_b[w];
-    }
-    sa += s_a[w];
-    sb += s_b[w];
-  }
-  __syncthreads();  // s_a, s_b are reused by the next call
-  *ta = sa;
-  *tb = sb;
-  return make_uint2(oa + xa - a, ob + xb - b);
-}
-
 // Every level of the collapse, from the roots in cstate: each CTA takes a
 // contiguous chunk of the level's items, (1) gathers their children and counts
 // internal children and leaf triangles, publishes its sums, [barrier], (2)
@@ -2217,6 +2540,27 @@ static cudaError_t onesweep_sort(K*& ka, uint32_t*& va, K*& kb, uint32_t*& vb, u
 // Stream-ordered scratch of one build: device allocations, pinned host
 // buffers and events are released when the arena goes out of scope, on every
 // return path (free() releases a buffer early to lower the peak).
+// The one-CTA finish of the clustering, by search radius.
+static cudaError_t ploc_finish_prepare() {
+  GB_CHECK(cudaFuncSetAttribute(k_ploc_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlocSmallSmem));
+  return cudaFuncSetAttribute(k_ploc_finish1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlocFinishSmem);
+}
+static cudaError_t ploc_finish(const PlocBufs& pb, uint32_t* ploc_state, float4* bnbox, uint32_t* bncnt,
+                               uint32_t* root_out, uint32_t* iters_out, uint32_t node_cap, uint32_t* err,
+                               uint32_t nseg, int radius, float4* dp_cost, uint4* dp_link, uint32_t leaf_max,
+                               cudaStream_t st) {
+  if (radius == 1)
+    k_ploc_finish1<<<1, PLOC_SMALL_THREADS, kPlocFinishSmem, st>>>(pb, ploc_state, bnbox, bncnt, root_out, iters_out,
+                                                                   node_cap, err, nseg, dp_cost, dp_link, leaf_max);
+  else
+    k_ploc_small<<<1, PLOC_SMALL_THREADS, kPlocSmallSmem, st>>>(pb.clo[0], pb.chi[0], pb.cidx[0], pb.clo[1], pb.chi[1],
+                                                                pb.cidx[1], ploc_state, bnbox, bncnt, root_out,
+                                                                iters_out, node_cap, err, nseg, radius, dp_cost,
+                                                                dp_link, leaf_max);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
 struct BuildArena {
   cudaStream_t st;
   std::vector<void*> dev, pinned;
@@ -2442,12 +2786,9 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   // segments it means every segment is down to one cluster (<= kMaxSegments)
   const uint32_t iters = round > 0 ? h_tot[kPlocRounds] : 0u;
   {
-    const size_t smem = kPlocSmallSmem;
-    GB_CHECK(cudaFuncSetAttribute(k_ploc_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_ploc_small<<<1, PLOC_SMALL_THREADS, smem, st>>>(clo_a, chi_a, cidx_a, clo_b, chi_b, cidx_b, ploc_state, bnbox, bncnt, d_root, d_iters, nnodes_bin, &acc->pad, nseg,
-                                                      radius, dp_cost, d_link, leaf_max_used);
-    note_launches(1);
-    GB_CHECK(cudaGetLastError());
+    GB_CHECK(ploc_finish_prepare());
+    GB_CHECK(ploc_finish(pb, ploc_state, bnbox, bncnt, d_root, d_iters, nnodes_bin, &acc->pad, nseg, radius, dp_cost,
+                         d_link, leaf_max_used, st));
   }
   uint32_t small_iters = 0, berr = 0;
   std::vector<uint32_t> seg_root(nseg, kInvalidID);
@@ -2686,7 +3027,7 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
       return e;
     g->col_grid = (uint32_t)std::max(1, std::min(per_sm, 4)) * (uint32_t)num_sms_build();
     // and the cooperative PLOC rounds (of the chosen search radius)
-    const void* pk = g->radius == 1   ? (const void*)k_ploc_all<1>
+    const void* pk = g->radius == 1   ? (const void*)k_ploc_rounds1
                      : g->radius == 2 ? (const void*)k_ploc_all<2>
                      : g->radius == 4 ? (const void*)k_ploc_all<4>
                      : g->radius == 8 ? (const void*)k_ploc_all<8>
@@ -2700,8 +3041,8 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
       (e = alloc(&g->bnbox, 4 * (size_t)N)) ||
       (e = alloc(&g->bncnt, 2 * (size_t)N)) || (e = alloc(&g->clo[0], N)) || (e = alloc(&g->clo[1], N)) ||
       (e = alloc(&g->chi[0], N)) || (e = alloc(&g->chi[1], N)) || (e = alloc(&g->cidx[0], N)) ||
-      (e = alloc(&g->cidx[1], N)) || (e = alloc(&g->nn, N)) || (e = alloc(&g->bsurv, g->maxb)) ||
-      (e = alloc(&g->bmerge, g->maxb)) ||
+      (e = alloc(&g->cidx[1], N)) || (e = alloc(&g->nn, N)) || (e = alloc(&g->bsurv, cdiv(N, 32))) ||
+      (e = alloc(&g->bmerge, cdiv(N, 32))) ||
       (e = alloc(&g->scan_sums, 2 * (size_t)scan_scratch(std::max(g->maxb, maxw)))) ||
       (e = alloc(&g->d_tot, 4)) || (e = alloc(&g->d_root, g->nseg)) || (e = alloc(&g->d_iters, 1)) ||
       (e = alloc(&g->ploc_state, kPlocStateWords)) || (e = alloc(&g->cost, 2 * (size_t)(2 * N))) ||
@@ -2729,8 +3070,7 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
     e = cudaFuncSetAttribute(k_os_scatter<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)os_scatter_smem<uint32_t>());
   if (e != cudaSuccess) graph_build_release(g);
-  const size_t smem = kPlocSmallSmem;
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ploc_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = ploc_finish_prepare();
   return e;
 }
 
@@ -2792,9 +3132,8 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
     cfg.numAttrs = 1;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(g.ploc_bar);
     switch (g.radius) {
-      case 1: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<1>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
-                                          g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar,
-                                          &acc->pad)); break;
+      case 1: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_rounds1, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
+                                          g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar, &acc->pad)); break;
       case 2: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<2>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
                                           g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar,
                                           &acc->pad)); break;
@@ -2812,12 +3151,8 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   }
   stamp(4);
   {
-    const size_t smem = kPlocSmallSmem;
-    k_ploc_small<<<1, PLOC_SMALL_THREADS, smem, st>>>(g.clo[0], g.chi[0], g.cidx[0], g.clo[1], g.chi[1], g.cidx[1],
-                                                      g.ploc_state, g.bnbox, g.bncnt, g.d_root, g.d_iters,
-                                                      nbin_cap, &acc->pad, g.nseg, (int)g.radius, dp_cost, dp_link,
-                                                      leaf_max);
-    note_launches(1);
+    GB_CHECK(ploc_finish(pb, g.ploc_state, g.bnbox, g.bncnt, g.d_root, g.d_iters, nbin_cap, &acc->pad, g.nseg,
+                         (int)g.radius, dp_cost, dp_link, leaf_max, st));
   }
   stamp(5);
   // collapse decisions and levels
