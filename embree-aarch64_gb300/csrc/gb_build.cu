@@ -701,9 +701,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_lb(ScanPair sp, uint32_t 
 // the reported SAH for the given binary tree and leaf size.
 //
 // link[n] = (left, right, decisions): one 16-byte read per node for the collapse,
-// which follows the decisions from node to node.  Of the decisions, byte 0 = argmin k of D(n, 8) (the split of a
-// wide node made from n); byte i - 1 (i = 2..8) = the k of D(n, i) when it beat
-// cost(n, i - 1), else 0.
+// which follows the decisions from node to node.  Byte 0 of the decisions is the
+// split of a wide node made from n, byte i - 1 (i = 2..8) the split of n in i slots:
+// the slots of the left child in the low and of the right child in the high four
+// bits, 0 where n stays one child (then for all fewer slots too).
 
 __device__ __forceinline__ void dp_store(float4* cost, uint4* link, uint32_t n, const float c[8], uint4 lk) {
   __stcg(cost + 2 * (size_t)n, make_float4(c[0], c[1], c[2], c[3]));
@@ -741,13 +742,13 @@ __device__ __forceinline__ void dp_node(float4* cost, uint4* link, uint32_t n, u
 #pragma unroll
   for (int i = 2; i <= 8; i++) {
     D[i] = INFINITY;
-    K[i] = 1;
+    K[i] = 1u | (uint32_t)(i - 1) << 4;
 #pragma unroll
     for (int k = 1; k < i; k++) {
       const float v = cl[k - 1] + cr[i - k - 1];
       if (v < D[i]) {
         D[i] = v;
-        K[i] = (uint32_t)k;
+        K[i] = (uint32_t)k | (uint32_t)(i - k) << 4;
       }
     }
   }
@@ -761,7 +762,7 @@ __device__ __forceinline__ void dp_node(float4* cost, uint4* link, uint32_t n, u
   for (int i = 2; i <= 8; i++) {
     const bool split = D[i] < c[i - 2];
     c[i - 1] = split ? D[i] : c[i - 2];
-    b[i - 1] = split ? K[i] : 0u;
+    b[i - 1] = split ? K[i] : i > 2 ? b[i - 2] : 0u;
   }
   dp_store(cost, link, n, c,
            make_uint4(l, r, b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24), b[4] | (b[5] << 8) | (b[6] << 16) | (b[7] << 24)));
@@ -777,16 +778,17 @@ struct GridBarrier {
 // is zero before the launch (a barrier adds gridDim.x to it).  A CTA that waits for
 // more than kLbSpinLimit re-reads (a CTA missing) sets kErrBuild in *err; false
 // once *err is set, so the grid leaves its loop.  A build waits at about 70 of
-// these and a refit at 12, so their latency counts: one arriving atomic and reads of
-// the same word between two acquire-release fences take 1.5 us over 456 CTAs;
-// a separate generation word, sequentially consistent fences and sleeping between
-// the reads took 2.3 us.
+// these and a refit at 12, so their latency counts: one
+// releasing atomic, plain reads of the same word and one acquiring read at the end.
+// (Acquire-release fences around the atomic and the reads cost 0.3 us more per
+// barrier, the rounds of the 4M soup 571 us instead of 555; a separate generation
+// word, sequentially consistent fences and sleeping between the reads 1.1 us more.)
 __device__ __forceinline__ bool grid_sync(GridBarrier* b, unsigned int* err) {
   __shared__ bool s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    const unsigned int ticket = atomicAdd(&b->count, 1u);
+    unsigned int ticket;
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(&b->count) : "memory");
     const unsigned int target = (ticket / gridDim.x + 1u) * gridDim.x;
     uint32_t it = 0, e = lb_load(err);
     while (lb_load(&b->count) < target && e == 0u && it < kLbSpinLimit) {
@@ -794,7 +796,8 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* b, unsigned int* err) {
       it++;
     }
     if (it == kLbSpinLimit) atomicOr(err, kErrBuild);
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    unsigned int last;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(last) : "l"(&b->count) : "memory");
     s_ok = e == 0u && it < kLbSpinLimit;
   }
   __syncthreads();
@@ -1219,9 +1222,12 @@ __device__ __forceinline__ float ploc_adjacent(const float4* clo, const float4* 
 }
 
 // Exclusive block scan of two values (a, b); returns (prefix a, prefix b) and
-// the block totals in *ta, *tb.  All 256 threads call it.
+// the block totals in *ta, *tb.  All THREADS threads call it.
+template <int THREADS = 256>
 __device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32_t* ta, uint32_t* tb) {
-  __shared__ uint32_t s_a[8], s_b[8];
+  constexpr int kWarps = THREADS / 32;
+  static_assert(kWarps <= 32, "every warp adds up the warps' sums");
+  __shared__ uint2 s_ab[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t xa = a, xb = b;
 #pragma unroll
@@ -1232,24 +1238,14 @@ __device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32
       xb += yb;
     }
   }
-  if (lane == 31) {
-    s_a[warp] = xa;
-    s_b[warp] = xb;
-  }
+  if (lane == 31) s_ab[warp] = make_uint2(xa, xb);
   __syncthreads();
-  uint32_t oa = 0, ob = 0, sa = 0, sb = 0;
-#pragma unroll
-  for (int w = 0; w < 8; w++) {
-    if (w < warp) {
-      oa += s_a[w];
-      ob += s_b[w];
-    }
-    sa += s_a[w];
-    sb += s_b[w];
-  }
-  __syncthreads();  // s_a, s_b are reused by the next call
-  *ta = sa;
-  *tb = sb;
+  const uint2 w = s_ab[min(lane, kWarps - 1)];
+  const bool all = lane < kWarps, before = lane < warp;
+  *ta = __reduce_add_sync(0xFFFFFFFFu, all ? w.x : 0u);
+  *tb = __reduce_add_sync(0xFFFFFFFFu, all ? w.y : 0u);
+  const uint32_t oa = __reduce_add_sync(0xFFFFFFFFu, before ? w.x : 0u), ob = __reduce_add_sync(0xFFFFFFFFu, before ? w.y : 0u);
+  __syncthreads();  // s_ab is used again by the next call
   return make_uint2(oa + xa - a, ob + xb - b);
 }
 
@@ -1856,9 +1852,9 @@ __device__ __forceinline__ void gather_group(const BinTree& t, uint32_t b, bool 
       if (s == 0) n = b, i = 1;
     } else {
       const uint4 lk = t.link[b];
-      const uint32_t k8 = min(max(lk.z & 0xFFu, 1u), 7u);  // split of D(b, 8)
-      if (s == 0) n = lk.y, i = 8u - k8;
-      if (s == 8u - k8) n = lk.x, i = k8;
+      const uint32_t k = lk.z & 15u, rem = lk.z >> 4 & 15u;
+      if (s == 0) n = lk.y, i = rem;
+      if (s == rem) n = lk.x, i = k;
     }
   }
   for (;;) {
@@ -1871,24 +1867,21 @@ __device__ __forceinline__ void gather_group(const BinTree& t, uint32_t b, bool 
         const uint4 lk = t.link[n];
         left = lk.x;
         right = lk.y;
-        for (; i > 1u; i--) {
-          k = ((i - 1u < 4u ? lk.z : lk.w) >> (8u * ((i - 1u) & 3u))) & 0xFFu;
-          if (k != 0u) break;
-        }
-        split = i > 1u;
-        k = min(k, i - 1u);
+        const uint32_t d = (i < 5u ? lk.z >> (8u * (i - 1u)) : lk.w >> (8u * (i - 5u))) & 0xFFu;
+        split = d != 0u;
+        k = d & 15u;
+        i = split ? d >> 4 : 1u;
       }
     }
     live = __ballot_sync(0xFFFFFFFFu, i > 0u) >> gshift & 0xFFu;
     if (!__any_sync(0xFFFFFFFFu, split)) break;
-    const uint32_t dst = split ? s + i - k : 8u;
+    const uint32_t dst = split ? s + i : 8u;
     const uint32_t below = live & ((1u << s) - 1u);
     const int src = below ? 31 - __clz(below) : 0;  // the entry whose slots this lane may lie in
     const uint32_t d2 = __shfl_sync(0xFFFFFFFFu, dst, src, 8), k2 = __shfl_sync(0xFFFFFFFFu, k, src, 8);
     const uint32_t l2 = __shfl_sync(0xFFFFFFFFu, left, src, 8);
     if (split) {
       n = right;
-      i -= k;
     } else if (i == 0u && below && d2 == s) {
       n = l2;
       i = k2;
@@ -1969,12 +1962,25 @@ __device__ __forceinline__ uint32_t cta_excl_scan_1024(uint32_t v, uint32_t* s_w
 
 // First level: the roots of the non-empty segments in segment order (one CTA
 // of 1024 threads, nseg <= 4 x 1024); seg_index[s] = position of segment s's
-// root (kInvalidID for an empty segment).
+// root (kInvalidID for an empty segment).  It also zeroes what the collapse adds
+// to (cstate, the SAH sums, the leaf count, the CTA sums and barrier of
+// k_collapse_all): as memsets these were four launches of a captured build.
 __global__ void __launch_bounds__(1024) k_collapse_roots(const uint32_t* __restrict__ d_root, uint32_t nseg,
                                                          uint32_t nbin, uint32_t* __restrict__ items,
                                                          uint32_t* __restrict__ seg_index,
-                                                         uint32_t* __restrict__ cstate) {
+                                                         uint32_t* __restrict__ cstate, double* __restrict__ sah_acc,
+                                                         uint32_t* __restrict__ leaf_count,
+                                                         unsigned long long* __restrict__ cta_sums, uint32_t nsums,
+                                                         GridBarrier* __restrict__ bar) {
   __shared__ uint32_t s_w[32];
+  for (uint32_t k = threadIdx.x; k < (uint32_t)kColStateWords; k += 1024) cstate[k] = 0;
+  for (uint32_t k = threadIdx.x; k < nsums; k += 1024) cta_sums[k] = 0ull;
+  if (threadIdx.x < 2) sah_acc[threadIdx.x] = 0.0;
+  if (threadIdx.x == 0) {
+    *leaf_count = 0;
+    if (bar) bar->count = 0;
+  }
+  __syncthreads();
   uint32_t r[4], cnt = 0;
   const uint32_t s0 = threadIdx.x * 4;
 #pragma unroll
@@ -2056,14 +2062,11 @@ __global__ void k_collapse_advance(const uint32_t* __restrict__ tot, uint32_t* _
 }
 
 __device__ __forceinline__ uint32_t exp_for(float ext) {
-  // smallest power of two 2^(E-127) with 255 * 2^(E-127) >= ext
-  const float x = __fdiv_ru(ext, 255.0f);
-  const uint32_t bits = __float_as_uint(x);
-  uint32_t E = (bits >> 23) & 0xFFu;
-  if (bits & 0x7FFFFFu) E += 1;
-  if (E < 1) E = 1;
-  if (E > 253) E = 253;
-  return E;
+  // smallest power of two 2^(E-127) with 255 * 2^(E-127) >= ext: with ext = m 2^e,
+  // 1 <= m < 2, that is e - 7 while m <= 255 / 128 and e - 6 above
+  const uint32_t bits = __float_as_uint(ext), e = bits >> 23 & 0xFFu;
+  if (e == 255u) return 253u;
+  return min(max(e + ((bits & 0x7FFFFFu) > 0x7F0000u ? 1u : 0u), 8u) - 7u, 253u);
 }
 
 __device__ __forceinline__ void write_tri(const GeomDesc* __restrict__ geoms, const float4* __restrict__ pbox,
@@ -2089,11 +2092,9 @@ __device__ __forceinline__ void write_tri(const GeomDesc* __restrict__ geoms, co
   dst->c = make_float4(e2.x, e2.y, e2.z, 0.f);
 }
 
-// Shared memory of the lane groups that emit wide nodes: the slot auction and the
-// node's words.
+// Shared memory of the lane groups that emit wide nodes: the node's words.
 template <int GROUPS>
 struct EmitSmem {
-  unsigned long long key[GROUPS][8];
   alignas(16) uint32_t node[GROUPS][sizeof(WideNode) / 4];
 };
 
@@ -2106,14 +2107,17 @@ struct EmitSmem {
 // slots in ascending order of (slot ^ ray octant) is roughly near-to-far.  One
 // order of all pairs ranks the slots for every child and the children for every
 // slot, so the greedy choice is the stable assignment, which rounds of offers
-// find: every unplaced child offers for its best slot that has not turned it
-// away, a slot keeps its best offer (3-4 rounds where the greedy form took one
-// per child).  Planes are quantised outward, internal children are numbered and
+// find: every child stands at its next slot, and of the children at one slot all
+// but the first move on to theirs.  Opposite slots have opposite costs, so 16
+// comparisons rank a child's slots and 56 tell which children come before it at
+// each; a round is then four votes.  (With every child scanning the free slots and
+// 64-bit shared atomics for the offers, a level waited up to 4,300 cycles for the
+// slots of its slowest node; so, 700.)  Planes are quantised outward, internal children are numbered and
 // leaf triangles laid out in slot order.
 template <int GROUPS>
 __device__ __forceinline__ void collapse_emit_group(
     const BinTree& t, const uint32_t* __restrict__ kids_in, uint32_t k, bool have, uint32_t g, EmitSmem<GROUPS>& sm,
-    const uint32_t* __restrict__ off_int, const uint32_t* __restrict__ off_tri, uint32_t level_base,
+    const uint32_t* __restrict__ off_int, const uint32_t* __restrict__ off_tri, uint2 off, uint32_t level_base,
     uint32_t next_base, uint32_t tri_next, WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root,
     uint32_t* __restrict__ next_items, uint32_t node_cap, uint32_t tri_cap, uint32_t* err, double& sah_out,
     double& sahx_out, uint32_t& nleaf_out) {
@@ -2129,7 +2133,7 @@ __device__ __forceinline__ void collapse_emit_group(
     prim = __float_as_uint(b.w);
   }
   uint32_t cnt = valid ? bt_cnt(t, kid) : 0u;
-  const uint32_t oi = have ? off_int[k] : 0u, ot = have ? off_tri[k] : 0u;
+  const uint32_t oi = have ? off.x + off_int[k] : 0u, ot = have ? off.y + off_tri[k] : 0u;
   // union box and quantisation frame
   float3 ulo = valid ? lo : make_float3(INFINITY, INFINITY, INFINITY);
   float3 uhi = valid ? hi : make_float3(-INFINITY, -INFINITY, -INFINITY);
@@ -2152,40 +2156,61 @@ __device__ __forceinline__ void collapse_emit_group(
   // slot costs of this lane's child
   const float3 pc = make_float3((ulo.x + uhi.x) * 0.5f, (ulo.y + uhi.y) * 0.5f, (ulo.z + uhi.z) * 0.5f);
   const float dx = (lo.x + hi.x) * 0.5f - pc.x, dy = (lo.y + hi.y) * 0.5f - pc.y, dz = (lo.z + hi.z) * 0.5f - pc.z;
-  float cs[8];
+  // cost of slot q < 4 as an integer of the same order (zeros of both signs equal);
+  // slot 7 - q costs -c[q]
+  auto ordered = [](float x) {
+    const int b = __float_as_int(x);
+    return b < 0 ? -(b & 0x7FFFFFFF) : b;
+  };
+  const int c[4] = {ordered((dx + dy) + dz), ordered((-dx + dy) + dz), ordered((dx - dy) + dz), ordered((-dx - dy) + dz)};
+  // ranks of slots 0..3 (4 bits each): slots before them, equal costs in slot order
+  uint32_t ranks = 0;
 #pragma unroll
-  for (int q = 0; q < 8; q++) cs[q] = ((q & 1) ? -dx : dx) + ((q & 2) ? -dy : dy) + ((q & 4) ? -dz : dz);
-  unsigned long long* key = sm.key[g];
+  for (int q = 0; q < 4; q++) {
+#pragma unroll
+    for (int w = q; w < 4; w++) {
+      if (w > q) ranks += c[w] < c[q] ? 1u << (4 * q) : 1u << (4 * w);
+      // slot 7 - w before slot q, and 7 - q before w
+      if (-c[w] < c[q]) ranks += w > q ? (1u << (4 * q)) + (1u << (4 * w)) : 1u << (4 * q);
+    }
+  }
+  uint32_t order = 0;  // the slots, cheapest first, 4 bits each
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const uint32_t r4 = (ranks >> (4 * q) & 7u) * 4u;
+    order |= ((uint32_t)q << r4) | ((7u - q) << (28u - r4));
+  }
+  // the children that come before this one at slot q (byte q of w03) and at slot
+  // 7 - q (byte q of w74)
+  uint32_t w03 = 0, w74 = 0;
+#pragma unroll
+  for (uint32_t d = 1; d < 8; d++) {
+    const uint32_t bit = 1u << (i ^ d);
+    const int lower = i >> (d < 2u ? 0 : d < 4u ? 1 : 2) & 1u;  // child i ^ d is the lower one: it wins a tie
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int o = __shfl_xor_sync(0xFFFFFFFFu, c[q], d);
+      if (o < c[q] + lower) w03 |= bit << (8 * q);
+      if (o > c[q] - lower) w74 |= bit << (8 * q);
+    }
+  }
   uint32_t* words = sm.node[g];
-  key[i] = ~0ull;
   // empty slots: meta 0, lower planes 255, upper planes 0
   if (i < 7u) *reinterpret_cast<uint2*>(words + 6 + 2 * i) = i >= 1u && i <= 3u ? make_uint2(~0u, ~0u) : make_uint2(0u, 0u);
   __syncwarp();
-  uint32_t refused = 0, slot = 8;
-  bool placed = !valid;
-  unsigned long long offer = 0;
-  while (__any_sync(0xFFFFFFFFu, !placed)) {
-    if (!placed) {
-      float bc = INFINITY;
-      int bs = -1;
+  const uint32_t gshift = threadIdx.x & 24u, kids8 = __ballot_sync(0xFFFFFFFFu, valid) >> gshift & 0xFFu;
+  for (bool lost = true; __any_sync(0xFFFFFFFFu, lost);) {
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        if (!(refused >> q & 1u) && (bs < 0 || cs[q] < bc)) {
-          bc = cs[q];
-          bs = q;
-        }
-      }
-      slot = (uint32_t)bs & 7u;
-      offer = ((unsigned long long)f2ord(bc + 0.0f) << 32) | i;  // + 0: -0 ties with +0
-      atomicMin(key + slot, offer);
+    for (int r = 0; r < 2; r++) {  // two rounds per vote on going on: one too many changes nothing
+      const uint32_t q = order & 7u;
+      const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, q & 1u), b1 = __ballot_sync(0xFFFFFFFFu, q & 2u),
+                     b2 = __ballot_sync(0xFFFFFFFFu, q & 4u);
+      const uint32_t same = ((q & 1u ? b0 : ~b0) & (q & 2u ? b1 : ~b1) & (q & 4u ? b2 : ~b2)) >> gshift & kids8;
+      lost = (same & __funnelshift_r(q < 4u ? w03 : w74, 0u, 8u * (q < 4u ? q : 7u - q))) != 0u && valid;
+      if (lost) order >>= 4;
     }
-    __syncwarp();
-    if (valid) {
-      placed = key[slot] == offer;
-      if (!placed) refused |= 1u << slot;
-    }
-    __syncwarp();
   }
+  const uint32_t slot = valid ? order & 7u : 8u;
   // this child's planes, its part of the SAH, its place among the slots
   const bool inner = cnt > t.leaf_max;
   uint32_t places = valid ? (inner ? 8u : cnt) << (4u * slot) : 0u;  // 4 bits per slot: triangles, bit 3 an internal child
@@ -2196,49 +2221,43 @@ __device__ __forceinline__ void collapse_emit_group(
     int_slots |= __shfl_xor_sync(0xFFFFFFFFu, int_slots, o);
   }
   const uint32_t child_base = next_base + oi, tri_base = tri_next + ot;
+  float A = 0.f, Ax = 0.f;
   if (valid) {
-    const float flx = fminf(fmaxf(floorf(__fsub_rd(lo.x, ulo.x) * ix), 0.f), 255.f);
-    const float fly = fminf(fmaxf(floorf(__fsub_rd(lo.y, ulo.y) * iy), 0.f), 255.f);
-    const float flz = fminf(fmaxf(floorf(__fsub_rd(lo.z, ulo.z) * iz), 0.f), 255.f);
-    const float fhx = fminf(fmaxf(ceilf(__fsub_ru(hi.x, ulo.x) * ix), 0.f), 255.f);
-    const float fhy = fminf(fmaxf(ceilf(__fsub_ru(hi.y, ulo.y) * iy), 0.f), 255.f);
-    const float fhz = fminf(fmaxf(ceilf(__fsub_ru(hi.z, ulo.z) * iz), 0.f), 255.f);
+    const uint32_t qlx = min(__float2uint_rd(__fsub_rd(lo.x, ulo.x) * ix), 255u);
+    const uint32_t qly = min(__float2uint_rd(__fsub_rd(lo.y, ulo.y) * iy), 255u);
+    const uint32_t qlz = min(__float2uint_rd(__fsub_rd(lo.z, ulo.z) * iz), 255u);
+    const uint32_t qhx = min(__float2uint_ru(__fsub_ru(hi.x, ulo.x) * ix), 255u);
+    const uint32_t qhy = min(__float2uint_ru(__fsub_ru(hi.y, ulo.y) * iy), 255u);
+    const uint32_t qhz = min(__float2uint_ru(__fsub_ru(hi.z, ulo.z) * iz), 255u);
+    // a byte as a float: in the mantissa of 2^23
+    auto f = [](uint32_t q) { return __uint_as_float(0x4B000000u | q) - 8388608.0f; };
+    const float flx = f(qlx), fly = f(qly), flz = f(qlz), fhx = f(qhx), fhy = f(qhy), fhz = f(qhz);
     // decoded (outward-rounded) box, as traversal sees it
     const float3 dlo = make_float3(__fmaf_rd(flx, sx, ulo.x), __fmaf_rd(fly, sy, ulo.y), __fmaf_rd(flz, sz, ulo.z));
     const float3 dhi = make_float3(__fmaf_ru(fhx, sx, ulo.x), __fmaf_ru(fhy, sy, ulo.y), __fmaf_ru(fhz, sz, ulo.z));
-    const double A = (double)fmaxf(0.f, half_area(dlo, dhi));
-    const double Ax = (double)fmaxf(0.f, half_area(lo, hi));
-    const uint32_t below = places & ((1u << (4u * slot)) - 1u);
-    uint32_t meta;
-    if (inner) {
-      const uint32_t rank = __popc(below & 0x88888888u);
-      meta = 0x80u | slot;
-      if (oi + rank >= node_cap || child_base + rank >= node_cap) atomicOr(err, kErrBuild);
-      else next_items[oi + rank] = kid;
-      sah_out += A;  // inner node term
-      sahx_out += Ax;
-    } else {
-      // triangles of the leaves in lower slots: the sum of their 3-bit counts
-      const uint32_t c = below & 0x77777777u;
-      const uint32_t tri_off = (((c & 0x0F0F0F0Fu) + (c >> 4 & 0x0F0F0F0Fu)) * 0x01010101u) >> 24;
-      meta = 0x80u | ((cnt - 1u) << 5) | tri_off;
-      // the leaf's triangle records are written after the last level by
-      // k_write_leaves, one thread per leaf: here only its binary subtree is
-      // recorded at the slot of its first triangle
-      if (tri_base + tri_off + cnt > tri_cap) atomicOr(err, kErrBuild);
-      else leaf_root[tri_base + tri_off] = cnt == 1 ? prim | kLeafPrim : kid;
-      sah_out += A * (double)((cnt + 3) / 4);  // leaf term: area x Triangle4 blocks
-      sahx_out += Ax * (double)((cnt + 3) / 4);
-      nleaf_out++;
-    }
+    A = fmaxf(0.f, half_area(dlo, dhi));
+    Ax = fmaxf(0.f, half_area(lo, hi));
+    // an inner child's place among the next level's items; a leaf's triangles behind
+    // those of the leaves in lower slots (the sum of their 3-bit counts)
+    const uint32_t below = places & ((1u << (4u * slot)) - 1u), c = below & 0x77777777u;
+    const uint32_t tri_off = (((c & 0x0F0F0F0Fu) + (c >> 4 & 0x0F0F0F0Fu)) * 0x01010101u) >> 24;
+    const uint32_t rank = __popc(below & 0x88888888u);
+    const uint32_t meta = inner ? 0x80u | slot : 0x80u | ((cnt - 1u) << 5) | tri_off;
+    // a leaf's triangle records are written after the last level by k_write_leaves,
+    // one thread per leaf: here only its binary subtree is recorded at the slot of
+    // its first triangle
+    const uint32_t at = inner ? oi + rank : tri_base + tri_off;
+    const bool fits = inner ? at < node_cap && child_base + rank < node_cap : at + cnt <= tri_cap;
+    if (fits) (inner ? next_items : leaf_root)[at] = inner || cnt > 1u ? kid : prim | kLeafPrim;
+    else atomicOr(err, kErrBuild);
     uint8_t* bytes = reinterpret_cast<uint8_t*>(words);
     bytes[24 + slot] = (uint8_t)meta;
-    bytes[32 + slot] = (uint8_t)flx;
-    bytes[40 + slot] = (uint8_t)fly;
-    bytes[48 + slot] = (uint8_t)flz;
-    bytes[56 + slot] = (uint8_t)fhx;
-    bytes[64 + slot] = (uint8_t)fhy;
-    bytes[72 + slot] = (uint8_t)fhz;
+    bytes[32 + slot] = (uint8_t)qlx;
+    bytes[40 + slot] = (uint8_t)qly;
+    bytes[48 + slot] = (uint8_t)qlz;
+    bytes[56 + slot] = (uint8_t)qhx;
+    bytes[64 + slot] = (uint8_t)qhy;
+    bytes[72 + slot] = (uint8_t)qhz;
   }
   if (i == 0u)
     *reinterpret_cast<uint4*>(words) = make_uint4(__float_as_uint(ulo.x), __float_as_uint(ulo.y), __float_as_uint(ulo.z),
@@ -2255,6 +2274,11 @@ __device__ __forceinline__ void collapse_emit_group(
     } else if (i < 6u) {
       reinterpret_cast<uint4*>(nodes + level_base + k)[i] = reinterpret_cast<const uint4*>(words)[i];
     }
+  }
+  if (valid) {  // the SAH's terms: area for an inner node, area x Triangle4 blocks for a leaf
+    sah_out += (double)A;
+    sahx_out += (double)Ax;
+    if (!inner) nleaf_out++;
   }
   __syncwarp();  // the words are built again for the next node
 }
@@ -2275,7 +2299,7 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_emit(
   __shared__ EmitSmem<COLLAPSE_THREADS / 8> sm;
   for (uint32_t k0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 3; k0 < nitems; k0 += (gridDim.x * blockDim.x) >> 3) {
     const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
-    collapse_emit_group(t, kids_in, k, k < nitems, threadIdx.x >> 3, sm, off_int, off_tri, level_base, next_base, tri_next,
+    collapse_emit_group(t, kids_in, k, k < nitems, threadIdx.x >> 3, sm, off_int, off_tri, make_uint2(0u, 0u), level_base, next_base, tri_next,
                         nodes, leaf_root, next_items, node_cap, tri_cap, err, sah, sahx, nleaf);
   }
   nleaf = __reduce_add_sync(0xFFFFFFFFu, nleaf);
@@ -2291,23 +2315,82 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_emit(
 // CTA 0 writes it back to cstate at the end.
 
 
-constexpr int COLLAPSE_ALL_THREADS = 256;
+// Threads of a CTA of k_collapse_all, one CTA per SM: 512 threads have registers for
+// two node's reads in flight and wait less at each other (a level of few nodes takes
+// 13,000 cycles against 16,000), 1024 threads have the warps that a wide level needs.
+// The levels of a tree of 8k / 300k / 1M / 4M triangles take 50 / 150 / 273 / 726 us
+// with 512 threads and 57 / 161 / 254 / 583 with 1024, so the line lies between 300k
+// and 1M.  (Four CTAs of 256 threads per SM: 73 / 217 / - / 664, most of it at the
+// barriers, where 608 CTAs arrive and read each other's sums instead of 152.)
+constexpr int COLLAPSE_NARROW_THREADS = 512, COLLAPSE_WIDE_THREADS = 1024;
+constexpr uint32_t COLLAPSE_WIDE_TRIS = 1u << 19;
+
+// Every CTA of a cooperative launch gives a pair (a, b), below 2^28 each, of its
+// thread 0 and gets the sums of the pairs of the CTAs before it (in x and y) and of
+// all CTAs (z, w); all threads call it.  The words of all CTAs are zero before the
+// launch, tag is not zero and another one in each call, and a grid barrier lies
+// between two calls.  A CTA reads the others' words until they bear the tag, so no
+// barrier and second read of the sums is needed: 1,150 cycles with 152 CTAs of 512
+// threads and 1,750 with 1024, where the barrier, the sums and their block scans took
+// 6,000 with 608 of 256.
+template <int THREADS>
+__device__ __forceinline__ bool grid_sums(unsigned long long* __restrict__ words, uint32_t tag, uint32_t a, uint32_t b,
+                                          uint4& sums, unsigned int* err) {
+  __shared__ uint4 s_sums[THREADS / 32];
+  if (threadIdx.x == 0) {
+    if ((a | b) >> 28) atomicOr(err, kErrBuild);
+    *reinterpret_cast<volatile unsigned long long*>(words + blockIdx.x) =
+        (unsigned long long)tag << 56 | (unsigned long long)(b & 0xFFFFFFFu) << 28 | (a & 0xFFFFFFFu);
+  }
+  uint4 s = make_uint4(0, 0, 0, 0);
+  bool ok = true;
+  for (uint32_t c = threadIdx.x; c < gridDim.x; c += THREADS) {
+    const volatile unsigned long long* w = words + c;
+    unsigned long long v = *w;
+    for (uint32_t it = 0; ok && (uint32_t)(v >> 56) != tag; it++) {
+      if (it == kLbSpinLimit) atomicOr(err, kErrBuild);
+      ok = it < kLbSpinLimit && lb_load(err) == 0u;
+      v = *w;
+    }
+    const uint32_t x = (uint32_t)v & 0xFFFFFFFu, y = (uint32_t)(v >> 28) & 0xFFFFFFFu;
+    s.z += x;
+    s.w += y;
+    if (c < blockIdx.x) s.x += x, s.y += y;
+  }
+  const uint32_t warps = min(THREADS / 32u, (gridDim.x + 31u) / 32u);  // that read a word
+  if (threadIdx.x >> 5 < warps) {
+    s = make_uint4(__reduce_add_sync(0xFFFFFFFFu, s.x), __reduce_add_sync(0xFFFFFFFFu, s.y),
+                   __reduce_add_sync(0xFFFFFFFFu, s.z), __reduce_add_sync(0xFFFFFFFFu, s.w));
+    if ((threadIdx.x & 31) == 0) s_sums[threadIdx.x >> 5] = s;
+  }
+  ok = __syncthreads_and(ok);
+  sums = make_uint4(0, 0, 0, 0);
+  for (uint32_t k = 0; k < warps; k++) {
+    const uint4 o = s_sums[k];
+    sums.x += o.x;
+    sums.y += o.y;
+    sums.z += o.z;
+    sums.w += o.w;
+  }
+  return ok;
+}
 
 // Every level of the collapse, from the roots in cstate: each CTA takes a
 // contiguous chunk of the level's items, (1) gathers their children and counts
-// internal children and leaf triangles, publishes its sums, [barrier], (2)
-// turns its counts into the level's exclusive offsets from the CTA sums, (3)
-// writes its wide nodes and the next level's items, [barrier].  cta_sums holds
-// 2 * gridDim.x words; *bar is zero on entry.
-__global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 4) k_collapse_all(
+// internal children and leaf triangles, (2) scans the counts within the chunk and
+// sums them with the other CTAs (grid_sums), (3) writes its wide nodes and the next
+// level's items, [barrier].  cta_sums holds gridDim.x words; these and *bar are zero
+// on entry.
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_collapse_all(
     BinTree t, const ColItems ci, uint32_t* __restrict__ cstate, uint32_t* __restrict__ kids,
-    uint32_t* __restrict__ nint, uint32_t* __restrict__ ntri, uint32_t* __restrict__ cta_sums,
+    uint32_t* __restrict__ nint, uint32_t* __restrict__ ntri, unsigned long long* __restrict__ cta_sums,
     WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root, double* sah_acc, uint32_t* leaf_count,
     uint32_t node_cap, uint32_t tri_cap, uint32_t max_levels, GridBarrier* bar, unsigned int* err) {
   uint32_t nitems = __ldcg(cstate + kColN), base = __ldcg(cstate + kColBase), tri_next = __ldcg(cstate + kColTri),
            depth = __ldcg(cstate + kColDepth);
   bool failed = __ldcg(cstate + kColErr) != 0u;
-  __shared__ EmitSmem<COLLAPSE_ALL_THREADS / 8> sm;
+  __shared__ EmitSmem<THREADS / 8> sm;
   double sah = 0.0, sahx = 0.0;
   uint32_t nleaf = 0;
   while (nitems > 0 && !failed) {
@@ -2316,7 +2399,6 @@ __global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 4) k_collapse_all(
     const uint32_t per = (nitems + gridDim.x - 1) / gridDim.x;
     const uint32_t first = min(blockIdx.x * per, nitems), last = min(first + per, nitems);
     // (1) children and counts
-    uint32_t ci_sum = 0, ct_sum = 0;
     for (uint32_t k0 = first + ((threadIdx.x & ~31u) >> 3); k0 < last; k0 += blockDim.x >> 3) {
       const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
       uint32_t ni, nt;
@@ -2324,64 +2406,53 @@ __global__ void __launch_bounds__(COLLAPSE_ALL_THREADS, 4) k_collapse_all(
       if (k < last && (threadIdx.x & 7u) == 0u) {
         nint[k] = ni;
         ntri[k] = nt;
-        ci_sum += ni;
-        ct_sum += nt;
       }
-    }
-    {
-      uint32_t ta, tb;
-      block_excl_scan2(ci_sum, ct_sum, &ta, &tb);
-      if (threadIdx.x == 0) {
-        __stcg(cta_sums + blockIdx.x, ta);
-        __stcg(cta_sums + gridDim.x + blockIdx.x, tb);
-      }
-    }
-    if (!grid_sync(bar, err)) break;
-    // (2) offsets: this CTA's prefix and the level's totals from the CTA sums
-    uint32_t pi = 0, pt = 0, ti = 0, tt = 0;
-    for (uint32_t c = threadIdx.x; c < gridDim.x; c += blockDim.x) {
-      const uint32_t a = __ldcg(cta_sums + c), b = __ldcg(cta_sums + gridDim.x + c);
-      ti += a;
-      tt += b;
-      if (c < blockIdx.x) {
-        pi += a;
-        pt += b;
-      }
-    }
-    {
-      uint32_t s0, s1, s2, s3;
-      block_excl_scan2(pi, pt, &s0, &s1);
-      block_excl_scan2(ti, tt, &s2, &s3);
-      pi = s0;
-      pt = s1;
-      ti = s2;
-      tt = s3;
-    }
-    for (uint32_t k0 = first; k0 < last; k0 += blockDim.x) {
-      const uint32_t k = k0 + threadIdx.x;
-      const uint32_t a = k < last ? nint[k] : 0u, b = k < last ? ntri[k] : 0u;
-      uint32_t ta, tb;
-      const uint2 e = block_excl_scan2(a, b, &ta, &tb);
-      if (k < last) {
-        nint[k] = pi + e.x;
-        ntri[k] = pt + e.y;
-      }
-      pi += ta;
-      pt += tb;
     }
     __syncthreads();
+    // (2) offsets within the chunk; the chunk's place and the level's totals
+    uint32_t ci_sum = 0, ct_sum = 0;
+    if (last - first <= 32u) {  // one warp
+      if (threadIdx.x < 32u) {
+        const uint32_t k = first + threadIdx.x;
+        const uint32_t a = k < last ? nint[k] : 0u, b = k < last ? ntri[k] : 0u;
+        uint32_t xa = a, xb = b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t ya = __shfl_up_sync(0xFFFFFFFFu, xa, o), yb = __shfl_up_sync(0xFFFFFFFFu, xb, o);
+          if (threadIdx.x >= o) xa += ya, xb += yb;
+        }
+        if (k < last) {
+          nint[k] = xa - a;
+          ntri[k] = xb - b;
+        }
+        ci_sum = __shfl_sync(0xFFFFFFFFu, xa, 31);
+        ct_sum = __shfl_sync(0xFFFFFFFFu, xb, 31);
+      }
+    } else for (uint32_t k0 = first; k0 < last; k0 += blockDim.x) {
+      const uint32_t k = k0 + threadIdx.x;
+      uint32_t ta, tb;
+      const uint2 e = block_excl_scan2<THREADS>(k < last ? nint[k] : 0u, k < last ? ntri[k] : 0u, &ta, &tb);
+      if (k < last) {
+        nint[k] = ci_sum + e.x;
+        ntri[k] = ct_sum + e.y;
+      }
+      ci_sum += ta;
+      ct_sum += tb;
+    }
+    uint4 sums;
+    if (!grid_sums<THREADS>(cta_sums, depth + 1u, ci_sum, ct_sum, sums, err)) break;
     // (3) the wide nodes of this CTA's items, one per 8-lane group
     for (uint32_t k0 = first + ((threadIdx.x & ~31u) >> 3); k0 < last; k0 += blockDim.x >> 3) {
       const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
-      collapse_emit_group(t, kids, k, k < last, threadIdx.x >> 3, sm, nint, ntri, base, base + nitems, tri_next, nodes,
+      collapse_emit_group(t, kids, k, k < last, threadIdx.x >> 3, sm, nint, ntri, make_uint2(sums.x, sums.y), base, base + nitems, tri_next, nodes,
                           leaf_root, next_items, node_cap, tri_cap, err, sah, sahx, nleaf);
     }
     // (4) the next level, alike in every CTA
     if (blockIdx.x == 0 && threadIdx.x == 0 && depth < (uint32_t)kColMaxLevels) cstate[kColLevels + depth] = base;
     base += nitems;
-    tri_next += tt;
+    tri_next += sums.w;
     depth++;
-    uint32_t next = ti;
+    uint32_t next = sums.z;
     if ((next > 0 && depth >= max_levels) || base + next > node_cap) {
       failed = true;
       next = 0;
@@ -2835,14 +2906,12 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   uint32_t* d_leaves = nullptr;
   GB_CHECK(arena.alloc(&d_sah, 2));  // quantised, exact
   GB_CHECK(arena.alloc(&d_leaves, 1));
-  GB_CHECK(cudaMemsetAsync(d_sah, 0, 2 * sizeof(double), st));
-  GB_CHECK(cudaMemsetAsync(d_leaves, 0, sizeof(uint32_t), st));
   uint32_t *cstate = nullptr, *seg_index = nullptr, *h_col = nullptr;
   GB_CHECK(arena.alloc(&cstate, kColStateWords));
   GB_CHECK(arena.alloc(&seg_index, nseg));
   GB_CHECK(arena.host(&h_col, kColStateWords));
-  GB_CHECK(cudaMemsetAsync(cstate, 0, sizeof(uint32_t) * kColStateWords, st));
-  k_collapse_roots<<<1, 1024, 0, st>>>(d_root, nseg, nnodes_bin, items_a, seg_index, cstate);
+  k_collapse_roots<<<1, 1024, 0, st>>>(d_root, nseg, nnodes_bin, items_a, seg_index, cstate, d_sah, d_leaves, nullptr, 0,
+                                       nullptr);
   note_launches(1);
   const ColItems citems{{items_a, items_b}};
   uint32_t level = 0;
@@ -3022,10 +3091,11 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
   // the cooperative collapse: as many CTAs as can be resident at once
   {
     int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_collapse_all, COLLAPSE_ALL_THREADS, 0)) !=
-        cudaSuccess)
-      return e;
-    g->col_grid = (uint32_t)std::max(1, std::min(per_sm, 4)) * (uint32_t)num_sms_build();
+    g->col_threads = N > COLLAPSE_WIDE_TRIS ? COLLAPSE_WIDE_THREADS : COLLAPSE_NARROW_THREADS;
+    const void* collapse = g->col_threads == COLLAPSE_WIDE_THREADS ? (const void*)k_collapse_all<COLLAPSE_WIDE_THREADS>
+                                                                   : (const void*)k_collapse_all<COLLAPSE_NARROW_THREADS>;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, collapse, g->col_threads, 0)) != cudaSuccess) return e;
+    g->col_grid = (uint32_t)std::max(1, std::min(per_sm, 1)) * (uint32_t)num_sms_build();
     // and the cooperative PLOC rounds (of the chosen search radius)
     const void* pk = g->radius == 1   ? (const void*)k_ploc_rounds1
                      : g->radius == 2 ? (const void*)k_ploc_all<2>
@@ -3052,7 +3122,7 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
       (e = alloc(&g->d_sah, 2)) || (e = alloc(&g->d_leaves, 1)) || (e = alloc(&g->cstate, kColStateWords)) ||
       (e = alloc(&g->seg_index, g->nseg)) ||
       (e = cudaMallocHost((void**)&g->out, sizeof(GraphBuildOut) + sizeof(uint32_t) * g->nseg)) ||
-      (e = alloc(&g->col_sums, 2 * (size_t)g->col_grid)) || (e = alloc(&g->col_bar, 2)) ||
+      (e = alloc(&g->col_sums, g->col_grid)) || (e = alloc(&g->col_bar, 2)) ||
       (e = alloc(&g->prec, T)) || (e = alloc(&g->ploc_sums, 2 * (size_t)g->ploc_grid)) ||
       (e = alloc(&g->ploc_bar, 2)) || (opt.phase_stamps && (e = alloc(&g->stamps, kBuildPhases + 1)))) {
     graph_build_release(g);
@@ -3158,19 +3228,16 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   // collapse decisions and levels
   BinTree bt{g.bnbox, g.bncnt, N, leaf_max, (uint32_t)(g.opt.robust != 0), dp_link};
   GB_CHECK(cudaMemsetAsync(g.leaf_root, 0xFF, sizeof(uint32_t) * N, st));
-  GB_CHECK(cudaMemsetAsync(g.d_sah, 0, 2 * sizeof(double), st));
-  GB_CHECK(cudaMemsetAsync(g.d_leaves, 0, sizeof(uint32_t), st));
-  GB_CHECK(cudaMemsetAsync(g.cstate, 0, sizeof(uint32_t) * kColStateWords, st));
   // collapse levels in a loop the device ends
   stamp(6);
   // all collapse levels in one cooperative launch
-  k_collapse_roots<<<1, 1024, 0, st>>>(g.d_root, g.nseg, g.nbin, g.items[0], g.seg_index, g.cstate);
-  GB_CHECK(cudaMemsetAsync(g.col_bar, 0, sizeof(GridBarrier), st));
+  k_collapse_roots<<<1, 1024, 0, st>>>(g.d_root, g.nseg, g.nbin, g.items[0], g.seg_index, g.cstate, g.d_sah, g.d_leaves,
+                                       g.col_sums, g.col_grid, reinterpret_cast<GridBarrier*>(g.col_bar));
   {
     const ColItems ci{{g.items[0], g.items[1]}};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.col_grid);
-    cfg.blockDim = dim3(COLLAPSE_ALL_THREADS);
+    cfg.blockDim = dim3(g.col_threads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -3178,7 +3245,9 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    GB_CHECK(cudaLaunchKernelEx(&cfg, k_collapse_all, bt, ci, g.cstate, g.kids, g.nint, g.ntri, g.col_sums, g.nodes,
+    const auto collapse = g.col_threads == COLLAPSE_WIDE_THREADS ? k_collapse_all<COLLAPSE_WIDE_THREADS>
+                                                                 : k_collapse_all<COLLAPSE_NARROW_THREADS>;
+    GB_CHECK(cudaLaunchKernelEx(&cfg, collapse, bt, ci, g.cstate, g.kids, g.nint, g.ntri, g.col_sums, g.nodes,
                                 g.leaf_root, g.d_sah, g.d_leaves, maxw, N, (uint32_t)kColMaxLevels,
                                 reinterpret_cast<GridBarrier*>(g.col_bar), &acc->pad));
   }

@@ -86,7 +86,9 @@ struct GraphBuild {
   uint32_t *d_leaves = nullptr, *cstate = nullptr, *seg_index = nullptr;
   GraphBuildOut* out = nullptr;                         // results (page-locked host memory)
   uint32_t col_grid = 0;                                // CTAs of the cooperative collapse
-  uint32_t *col_sums = nullptr, *col_bar = nullptr;     // its per-CTA sums and grid barrier
+  int col_threads = 0;                     // of a CTA of the cooperative collapse
+  unsigned long long* col_sums = nullptr;  // its per-CTA sums
+  uint32_t* col_bar = nullptr;             // and grid barrier
   TriRecord* prec = nullptr;                            // leaf records in primitive order
   unsigned long long* stamps = nullptr;                 // phase timestamps (BuildOptions::phase_stamps)
   uint32_t ploc_grid = 0;                               // CTAs of the cooperative PLOC rounds
