@@ -136,6 +136,32 @@ __device__ __forceinline__ uint32_t encode_level(const uint16_t* __restrict__ Pb
   return pack_bf2(s0, s1);
 }
 
+// encode_level for level l (0..7) of the origin (dir false) or of the direction at
+// point q, in one instruction stream for both: where only one of the two levels is dense, both indices are formed.
+__device__ __forceinline__ uint32_t encode_either(const uint16_t* __restrict__ Pb, const float q[3], int l, bool dir) {
+  const uint32_t ra = level_res(l), rb = level_res(kOriginLevels + l), R = dir ? rb : ra;
+  const bool dense_a = (uint64_t)(ra + 1) * (ra + 1) * (ra + 1) <= kTableSize;
+  const bool dense_b = (uint64_t)(rb + 1) * (rb + 1) * (rb + 1) <= kTableSize;
+  const Cell c = level_cell(q, R);
+  const uint32_t* tab = reinterpret_cast<const uint32_t*>(Pb + kOffTable) + (size_t)(dir ? kOriginLevels + l : l) * kTableSize;
+  float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const uint32_t x = c.i[0] + (k & 1), y = c.i[1] + ((k >> 1) & 1), z = c.i[2] + ((k >> 2) & 1);
+    const uint32_t dense = x + (R + 1) * (y + (R + 1) * z);
+    const uint32_t hash = (x ^ (y * 2654435761u) ^ (z * 805459861u)) & (kTableSize - 1u);
+    const uint32_t e = (dir ? dense_b : dense_a) ? dense : hash;
+    const float wx = (k & 1) ? c.f[0] : __fsub_rn(1.0f, c.f[0]);
+    const float wy = (k & 2) ? c.f[1] : __fsub_rn(1.0f, c.f[1]);
+    const float wz = (k & 4) ? c.f[2] : __fsub_rn(1.0f, c.f[2]);
+    const float w = __fmul_rn(__fmul_rn(wx, wy), wz);
+    const uint32_t pr = __ldg(tab + e);
+    s0 = __fadd_rn(s0, __fmul_rn(w, bf2f((uint16_t)(pr & 0xFFFFu))));
+    s1 = __fadd_rn(s1, __fmul_rn(w, bf2f((uint16_t)(pr >> 16))));
+  }
+  return pack_bf2(s0, s1);
+}
+
 __global__ void k_encode_fwd(const char* rays, uint64_t stride, const uint32_t* idx, uint32_t B, GridSpec g,
                              const uint16_t* __restrict__ Pb, uint16_t* X0) {
   const uint64_t it = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -436,7 +462,8 @@ struct PropSmem {
   float b[3][kHidden];
 };
 static_assert(offsetof(PropSmem, w4) % 16 == 0, "cp.async destination alignment");
-static_assert((kLdH * 2) % 16 == 0, "row pitch of the streamed stage");
+static_assert((kLdH * 2) % 16 == 0 && (kLdX * 2) % 16 == 0, "16-byte pieces of a row");
+static_assert(kOriginLevels == 8 && kLevels == 16, "the encoder takes 8 levels per lane");
 
 template <int K, int LDA>
 __device__ __forceinline__ void hidden_layer(const uint16_t* A, const uint16_t* W, int ldw, const float* bias,
@@ -772,70 +799,84 @@ __global__ void k_permute_w4(const uint16_t* __restrict__ Pb, const float* __res
   *reinterpret_cast<uint4*>(w4p + (size_t)c * kTcN * kTcK + umma_off(r, kc * 8)) = v;
 }
 
-// Encoder and hidden layers for tiles of 128 rays (8 warps, 16 rows each):
-// each tile's last hidden layer is written, with the bias ones, in the UMMA
-// layout k_propose_tc bulk-copies (tile t at H + t * kTcRays * kTcK).
+// Encoder and hidden layers, 16 rays per warp: each one's last hidden layer is
+// written, with the bias ones, in the UMMA layout k_propose_tc bulk-copies (tile t
+// of 128 rays at H + t * kTcRays * kTcK).  The time goes to the latency of the table
+// reads, 128 a ray in 16 MB of tables: lanes 0-15 read the origin's and 16-31 the
+// direction's eight levels of the warp's rays, one level at a time (lanes share
+// lines where rays are near each other or a level is small; a ray's point is formed
+// twice instead of 16 times), and warps share only the weights, so they wait for
+// nobody and what shared memory they leave caches the tables.  2M rays: 0.96 ms with
+// two rays of 16 levels per warp and tiles of 128 rays per CTA, 0.70 with one level
+// of 32 rays per warp in such tiles, 0.45 so (the inference as a whole 1.81, 1.55 and
+// 1.31 ms); 3 x 512 threads 1.38, 2 x 768 1.36, 1 x 1024 1.30, 4 x 256 1.34 ms.
+constexpr int kHidThreads = 512, kHidCtas = 2, kHidWarps = kHidThreads / 32;
 struct HidSmem {
-  uint16_t x[kTcRays * kLdX];
-  uint16_t h[kTcRays * kLdH];
+  alignas(16) uint16_t h[kHidWarps][16 * kLdH];  // the features, then the layers
   uint16_t w1[kHidden * kLdX];
   uint16_t w2[kHidden * kLdH];
   uint16_t w3[kHidden * kLdH];
   float b[3][kHidden];
 };
 
-__global__ void __launch_bounds__(256) k_propose_hidden(const char* rays, uint64_t stride, uint32_t M,
-                                                        const uint32_t* d_count, GridSpec grid,
-                                                        const uint16_t* __restrict__ Pb, const float* __restrict__ P,
-                                                        uint16_t* __restrict__ H) {
+__global__ void __launch_bounds__(kHidThreads, kHidCtas)
+    k_propose_hidden(const char* rays, uint64_t stride, uint32_t M, const uint32_t* d_count, GridSpec grid,
+                     const uint16_t* __restrict__ Pb, const float* __restrict__ P, uint16_t* __restrict__ H) {
   extern __shared__ __align__(16) unsigned char hid_smem_raw[];
   HidSmem& S = *reinterpret_cast<HidSmem*>(hid_smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  for (int i = tid; i < kHidden * kIn / 2; i += 256) {
+  for (int i = tid; i < kHidden * kIn / 2; i += kHidThreads) {
     const int o = (2 * i) / kIn, k = (2 * i) % kIn;
     *reinterpret_cast<uint32_t*>(S.w1 + o * kLdX + k) = reinterpret_cast<const uint32_t*>(Pb + kOffW1)[i];
   }
-  for (int i = tid; i < kHidden * kHidden / 2; i += 256) {
+  for (int i = tid; i < kHidden * kHidden / 2; i += kHidThreads) {
     const int o = (2 * i) / kHidden, k = (2 * i) % kHidden;
     *reinterpret_cast<uint32_t*>(S.w2 + o * kLdH + k) = reinterpret_cast<const uint32_t*>(Pb + kOffW2)[i];
     *reinterpret_cast<uint32_t*>(S.w3 + o * kLdH + k) = reinterpret_cast<const uint32_t*>(Pb + kOffW3)[i];
   }
-  for (int i = tid; i < 3 * kHidden; i += 256) {
+  for (int i = tid; i < 3 * kHidden; i += kHidThreads) {
     const size_t off = i < kHidden ? kOffB1 : (i < 2 * kHidden ? kOffB2 : kOffB3);
     S.b[i / kHidden][i % kHidden] = P[off + i % kHidden];
   }
   __syncthreads();
   if (d_count) M = min(M, *d_count);
-  const uint32_t ntiles = (M + kTcRays - 1) / kTcRays;
-  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const uint32_t r0 = tile * kTcRays;
-    for (int it = tid; it < kTcRays * kLevels; it += 256) {
-      const int rr = it / kLevels, l = it % kLevels;
-      const uint32_t rid = r0 + rr;
-      const uint32_t pk = rid < M ? encode_level(Pb, rays + (uint64_t)rid * stride, grid, l) : 0u;
-      *reinterpret_cast<uint32_t*>(S.x + rr * kLdX + 2 * l) = pk;
-    }
-    __syncthreads();
+  // whole 128-ray tiles: the rows past the last ray have features of zero
+  const uint32_t nblocks = (M + kTcRays - 1) / kTcRays * (kTcRays / 16);
+  uint16_t* h = S.h[warp];
+  for (uint32_t blk = blockIdx.x * kHidWarps + warp; blk < nblocks; blk += gridDim.x * kHidWarps) {
     {
-      const int row0 = warp * 16;
-      uint16_t* hrow = S.h + row0 * kLdH;
-      hidden_layer<kIn, kLdX>(S.x + row0 * kLdX, S.w1, kLdX, S.b[0], hrow, g, t);
-      __syncwarp();
-      hidden_layer<kHidden, kLdH>(hrow, S.w2, kLdH, S.b[1], hrow, g, t);
-      __syncwarp();
-      hidden_layer<kHidden, kLdH>(hrow, S.w3, kLdH, S.b[2], hrow, g, t);
+      const int row = lane & 15;
+      const bool dir = lane >= 16;
+      const uint32_t rid = blk * 16 + row;
+      uint32_t pk[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      if (rid < M) {
+        float q[3];
+        level_point(rays + (uint64_t)rid * stride, grid, dir ? kOriginLevels : 0, q);
+#pragma unroll
+        for (int l = 0; l < 8; l++) pk[l] = encode_either(Pb, q, l, dir);
+      }
+      uint4* x = reinterpret_cast<uint4*>(h + row * kLdH + (dir ? 16 : 0));
+      x[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      x[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
     }
-    __syncthreads();
+    __syncwarp();
+    hidden_layer<kIn, kLdH>(h, S.w1, kLdX, S.b[0], h, g, t);
+    __syncwarp();
+    hidden_layer<kHidden, kLdH>(h, S.w2, kLdH, S.b[1], h, g, t);
+    __syncwarp();
+    hidden_layer<kHidden, kLdH>(h, S.w3, kLdH, S.b[2], h, g, t);
+    __syncwarp();
     // 16-byte pieces in memory order: row group, K core matrix, row within the group
-    uint4* dst = reinterpret_cast<uint4*>(H + (size_t)tile * kTcRays * kTcK);
-    for (int pc = tid; pc < kTcRays * (kTcK / 8); pc += 256) {
-      const int grp = pc / (kTcK), rem = pc % (kTcK), kc = rem >> 3, r = grp * 8 + (rem & 7);
+    uint4* dst = reinterpret_cast<uint4*>(H + (size_t)blk * 16 * kTcK);
+    for (int pc = lane; pc < 16 * (kTcK / 8); pc += 32) {
+      const int grp = pc / kTcK, rem = pc % kTcK, kc = rem >> 3, r = grp * 8 + (rem & 7);
       uint4 v;
-      if (kc < kHidden / 8) v = *reinterpret_cast<const uint4*>(S.h + r * kLdH + kc * 8);
+      if (kc < kHidden / 8) v = *reinterpret_cast<const uint4*>(h + r * kLdH + kc * 8);
       else if (kc == kHidden / 8) v = make_uint4(0x3F803F80u, 0u, 0u, 0u);  // 1.0, 1.0 in BF16
       else v = make_uint4(0u, 0u, 0u, 0u);
       dst[pc] = v;
     }
+    __syncwarp();
   }
 }
 
@@ -1256,7 +1297,8 @@ cudaError_t Proposer::predict(const char* rays, uint64_t stride, uint32_t M, uin
       GB_TRY(cudaMalloc(&H_, (size_t)ntiles * kTcTileBytes));
       hcap_ = (size_t)ntiles * kTcRays * kTcK;
     }
-    k_propose_hidden<<<std::min<uint32_t>(ntiles, (uint32_t)num_sms() * 4), 256, sizeof(HidSmem), st>>>(
+    const uint32_t hid_ctas = (ntiles * (kTcRays / 16) + kHidWarps - 1) / kHidWarps;
+    k_propose_hidden<<<std::min<uint32_t>(hid_ctas, (uint32_t)num_sms() * kHidCtas), kHidThreads, sizeof(HidSmem), st>>>(
         rays, stride, M, d_count, grid, Pb_, P_, H_);
     // only the chunks that hold treelets: the rest of the outputs carry a -inf bias
     // and are never proposed (2M rays, 1,024 of 4,096 treelets: 2.68 -> 1.82 ms)
