@@ -499,14 +499,16 @@ __device__ __forceinline__ void hidden_layer(const uint16_t* A, const uint16_t* 
 // tie keeps the lower column.
 __device__ __forceinline__ void top4_insert(float (&v)[4], int (&ix)[4], float x, int i) {
   if (!(x > v[3])) return;
-  if (x > v[2]) {
-    v[3] = v[2]; ix[3] = ix[2];
-    if (x > v[1]) {
-      v[2] = v[1]; ix[2] = ix[1];
-      if (x > v[0]) { v[1] = v[0]; ix[1] = ix[0]; v[0] = x; ix[0] = i; }
-      else { v[1] = x; ix[1] = i; }
-    } else { v[2] = x; ix[2] = i; }
-  } else { v[3] = x; ix[3] = i; }
+  // no branch below: the lanes that insert do so at different places
+  const bool c2 = x > v[2], c1 = x > v[1], c0 = x > v[0];
+  v[3] = c2 ? v[2] : x;
+  ix[3] = c2 ? ix[2] : i;
+  v[2] = c1 ? v[1] : c2 ? x : v[2];
+  ix[2] = c1 ? ix[1] : c2 ? i : ix[2];
+  v[1] = c0 ? v[0] : c1 ? x : v[1];
+  ix[1] = c0 ? ix[0] : c1 ? i : ix[1];
+  v[0] = c0 ? x : v[0];
+  ix[0] = c0 ? i : ix[0];
 }
 
 // Top 4 of the four lanes (t = 0..3) that share a row; ties to the lower column.
@@ -647,11 +649,11 @@ __global__ void __launch_bounds__(kPW * 32, 2)
 }
 
 // ---------------------------------------------------------------------------
-// Inference on the 5th-generation tensor cores (tcgen05).  One CTA per SM
-// holds all 512 TMEM columns: two 128x256 FP32 accumulators.  Warps 0-15
-// encode the rays, run the hidden layers and scan the accumulators; warp 16
-// (the producer) streams the output weights and issues the MMAs.  Hand-offs
-// are mbarriers, never CTA-wide barriers:
+// Inference on the 5th-generation tensor cores (tcgen05).  Each of two CTAs per SM
+// holds 256 TMEM columns: two 128x128 FP32 accumulators.  Warps 0-15 scan the
+// accumulators for the best four logits of each ray; warp 16 (the producer) streams
+// the last hidden layers and the output weights and issues the MMAs.  Hand-offs are
+// mbarriers, and one barrier of the scanning warps per tile:
 //   tma_bar[s]  stage s holds a weight chunk (bulk copy complete)
 //   mma_bar[b]  accumulator b holds a chunk's logits (tcgen05.commit)
 //   epi_bar[b]  accumulator b has been read by all 16 scanning warps
@@ -659,22 +661,30 @@ __global__ void __launch_bounds__(kPW * 32, 2)
 // The output weights live in global memory in the UMMA canonical K-major
 // layout with K = 80: the 64 weights, then the bias split into two BF16 parts
 // (hi, lo) that the A operand multiplies by ones, so the MMA adds the bias;
-// unused treelets carry a -inf bias.  Each 256-treelet chunk (40 KB) is one
+// unused treelets carry a -inf bias.  Each 128-treelet chunk (20 KB) is one
 // contiguous block for one bulk copy.  In the scan, warp w reads TMEM lanes
 // 32 (w % 4) .. +31 (its rows) and the column quarter w / 4 of each chunk; the
-// four partial top-4 lists of a row are merged through shared memory at the
-// end of the tile.  Every mbarrier wait is bounded; on a timeout the kernel
-// sets kErrIterationLimit and stops.
+// four partial top-4 lists of a row are merged through shared memory, by the warps
+// of quarter k % 4 for tile k while the others scan the next tile (the lists are
+// double-buffered, so the barrier that publishes tile k + 1's also says that tile
+// k's have been read).  The scan's instructions bound the kernel (5.8 a lane
+// and logit, at 66 % of the issue rate): 500k rays over 1,024 treelets take 129 us,
+// where one CTA per SM with 128x256 accumulators, whose warps all waited for each
+// merge and branched within an insertion, took 281 (6.8 at 35 %).  Columns in groups
+// of 8 under one comparison; 4 or 16 are 1 % slower, insertion without a test for
+// each column 20 %.  Every mbarrier wait is bounded; on a timeout the kernel sets
+// kErrIterationLimit and stops.
 // ---------------------------------------------------------------------------
 
 constexpr int kTcScanWarps = 16;
 constexpr int kTcScanThreads = kTcScanWarps * 32;
 constexpr int kTcThreads = kTcScanThreads + 32;     // + the producer warp
 constexpr int kTcRays = 128;                        // UMMA M
-constexpr int kTcN = 256;                           // UMMA N: treelets per chunk
+constexpr int kTcN = 128;                           // UMMA N: treelets per chunk
 constexpr int kTcK = kHidden + 16;                  // 64 weights + bias (hi, lo) + zero padding
-constexpr uint32_t kTcChunkBytes = kTcN * kTcK * 2; // 40 KB
-constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kTcChunkBytes = kTcN * kTcK * 2; // 20 KB
+constexpr uint32_t kTmemCols = 2 * kTcN;
+constexpr int kTcCtas = 2;                          // per SM
 constexpr uint32_t kTcStages = 2;                   // weight chunks in flight
 // kind::f16 instruction descriptor: FP32 accumulator (bits 4-5 = 1), BF16 A and
 // B (bits 7-9 = 1, 10-12 = 1), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
@@ -684,8 +694,8 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTc
 struct TcSmem {
   uint16_t w4[kTcStages][kTcN * kTcK];  // streamed output weights + bias (UMMA layout)
   uint16_t a[2][kTcRays * kTcK];    // last hidden layers of two tiles + ones (UMMA layout)
-  float mv[kTcRays][4][4];          // partial top-4 per row and column quarter
-  int mi[kTcRays][4][4];
+  float4 mv[2][4][kTcRays];         // partial top-4 per tile parity, column quarter and row
+  ushort4 mi[2][4][kTcRays];
   unsigned long long tma_bar[kTcStages];
   unsigned long long a_bar[2];
   unsigned long long mma_bar[2];
@@ -761,15 +771,24 @@ __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-// two 32-column loads, one wait
+// 32 columns of the warp's 32 lanes
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
                : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
-// barrier among the scanning warps only (the producer warp does not take part)
-__device__ __forceinline__ void scan_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(kTcScanThreads) : "memory"); }
+// barrier among the scanning warps only (the producer warp does not take part);
+// whether x holds for any of their threads
+__device__ __forceinline__ bool scan_sync_or(bool x) {
+  uint32_t r;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, 1, %2, q;\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(r)
+      : "r"((uint32_t)x), "n"(kTcScanThreads)
+      : "memory");
+  return r != 0u;
+}
 
 __device__ __forceinline__ uint16_t bf16_bits(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 
@@ -880,7 +899,7 @@ __global__ void __launch_bounds__(kHidThreads, kHidCtas)
   }
 }
 
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kTcThreads, kTcCtas)
     k_propose_tc(uint32_t M, const uint32_t* d_count, const uint32_t nchunks, const uint16_t* __restrict__ H,
                  const uint16_t* __restrict__ W4p, const uint32_t* __restrict__ node_of_treelet, uint4* seeds,
                  uint32_t* treelets, uint32_t* err) {
@@ -982,73 +1001,80 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const uint32_t s = gc & 1u;
         if (!mbar_wait(&S.mma_bar[s], (gc >> 1) & 1u)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + s * kTcN + (uint32_t)quarter * 64;
-        uint32_t acc0[32], acc1[32];
-        tmem_ld32(taddr, acc0);
-        tmem_ld32(taddr + 32, acc1);
+        const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + s * kTcN + (uint32_t)quarter * 32;
+        uint32_t acc[32];
+        tmem_ld32(taddr, acc);
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&S.epi_bar[s]);  // this warp is done with accumulator s
-        const int col0 = (int)c * kTcN + quarter * 64;
-        float m0 = __uint_as_float(acc0[0]), m1 = __uint_as_float(acc1[0]);
+        const int col0 = (int)c * kTcN + quarter * 32;
 #pragma unroll
-        for (int q = 1; q < 32; q++) {
-          m0 = fmaxf(m0, __uint_as_float(acc0[q]));
-          m1 = fmaxf(m1, __uint_as_float(acc1[q]));
-        }
-        if (m0 > v[3]) {
+        for (int b = 0; b < 32; b += 8) {
+          float m = __uint_as_float(acc[b]);
 #pragma unroll
-          for (int q = 0; q < 32; q++) top4_insert(v, ix, __uint_as_float(acc0[q]), col0 + q);
-        }
-        if (m1 > v[3]) {
+          for (int q = 1; q < 8; q++) m = fmaxf(m, __uint_as_float(acc[b + q]));
+          if (m > v[3]) {
 #pragma unroll
-          for (int q = 0; q < 32; q++) top4_insert(v, ix, __uint_as_float(acc1[q]), col0 + 32 + q);
+            for (int q = 0; q < 8; q++) top4_insert(v, ix, __uint_as_float(acc[b + q]), col0 + b + q);
+          }
         }
       }
-      // the failure decision is taken by all scanning warps together, after a
-      // barrier they all reach (a warp that timed out left its chunk loop early)
-      volatile uint32_t* fail_flag = &S.fail;
-      if (!ok) *fail_flag = 1u;
-      {  // merge the four column quarters of each row (ties to the lower column)
-        const int row = (warp & 3) * 32 + lane;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          S.mv[row][quarter][q] = v[q];
-          S.mi[row][quarter][q] = ix[q];
-        }
-      }
-      scan_sync();
-      if (*fail_flag) {
+      // the four column quarters of each row are merged by the warps of one of them;
+      // the failure decision is one of all scanning warps (a warp that timed out left
+      // its chunk loop early)
+      const int row = (warp & 3) * 32 + lane, buf = (int)(k & 1u);
+      S.mv[buf][quarter][row] = make_float4(v[0], v[1], v[2], v[3]);
+      S.mi[buf][quarter][row] =
+          make_ushort4((uint16_t)ix[0], (uint16_t)ix[1], (uint16_t)ix[2], (uint16_t)ix[3]);  // -1 is 0xFFFF
+      if (scan_sync_or(!ok || *(volatile uint32_t*)&S.fail)) {
         if (tid == 0) atomicOr(err, kErrIterationLimit);
         break;
       }
-      if (tid < kTcRays) {
-        float bv[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        int bi[4] = {-1, -1, -1, -1};
-        for (int qq = 0; qq < 4; qq++)
-          for (int q = 0; q < 4; q++) {
-            const float x = S.mv[tid][qq][q];
-            const int i = S.mi[tid][qq][q];
-            if (i < 0) continue;
-            int pos = 4;
-            while (pos > 0 && (x > bv[pos - 1] || (x == bv[pos - 1] && (unsigned)i < (unsigned)bi[pos - 1]))) pos--;
-            if (pos < 4) {
-              for (int m = 3; m > pos; m--) { bv[m] = bv[m - 1]; bi[m] = bi[m - 1]; }
-              bv[pos] = x;
-              bi[pos] = i;
+      if (quarter == (int)(k & 3u)) {
+        const float* mv = reinterpret_cast<const float*>(&S.mv[buf][0][row]);
+        const uint16_t* mi = reinterpret_cast<const uint16_t*>(&S.mi[buf][0][row]);
+        float hv[4];  // the heads of the lists
+        uint32_t hi[4], at = 0u;  // at: byte q = entries taken of list q
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          hv[q] = mv[q * 4 * kTcRays];
+          hi[q] = mi[q * 4 * kTcRays];
+        }
+        int best[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          float bv = hv[0];
+          uint32_t bi = hi[0], b = 0;
+#pragma unroll
+          for (uint32_t q = 1; q < 4; q++) {  // ties to the lower column
+            const bool better = hv[q] > bv || (hv[q] == bv && hi[q] < bi);
+            bv = better ? hv[q] : bv;
+            bi = better ? hi[q] : bi;
+            b = better ? q : b;
+          }
+          best[r] = bi == 0xFFFFu ? -1 : (int)bi;
+          if (r < 3) {
+            at += 1u << (8 * b);
+            const uint32_t e = b * 4 * kTcRays + (at >> (8 * b) & 3u);  // at most the fourth entry
+            const float nv = mv[e];
+            const uint32_t ni = mi[e];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++) {
+              hv[q] = q == b ? nv : hv[q];
+              hi[q] = q == b ? ni : hi[q];
             }
           }
-        const uint32_t rid = tile * kTcRays + tid;
+        }
+        const uint32_t rid = tile * kTcRays + row;
         if (rid < M) {
           auto node = [&](int tl) { return tl >= 0 ? __ldg(node_of_treelet + tl) : kInvalidID; };
-          if (seeds) seeds[rid] = make_uint4(node(bi[0]), node(bi[1]), node(bi[2]), node(bi[3]));
+          if (seeds) seeds[rid] = make_uint4(node(best[0]), node(best[1]), node(best[2]), node(best[3]));
           if (treelets)
             reinterpret_cast<uint4*>(treelets)[rid] =
-                make_uint4((uint32_t)bi[0], (uint32_t)bi[1], (uint32_t)bi[2], (uint32_t)bi[3]);
+                make_uint4((uint32_t)best[0], (uint32_t)best[1], (uint32_t)best[2], (uint32_t)best[3]);
         }
       }
-      scan_sync();  // S.mv is written again by the next tile
     }
   }
   tc_fence_before();
@@ -1301,9 +1327,9 @@ cudaError_t Proposer::predict(const char* rays, uint64_t stride, uint32_t M, uin
     k_propose_hidden<<<std::min<uint32_t>(hid_ctas, (uint32_t)num_sms() * kHidCtas), kHidThreads, sizeof(HidSmem), st>>>(
         rays, stride, M, d_count, grid, Pb_, P_, H_);
     // only the chunks that hold treelets: the rest of the outputs carry a -inf bias
-    // and are never proposed (2M rays, 1,024 of 4,096 treelets: 2.68 -> 1.82 ms)
+    // and are never proposed (the scan's time is in proportion to the chunks)
     const uint32_t nchunks = std::max(1u, (num_treelets + kTcN - 1) / kTcN);
-    k_propose_tc<<<std::min<uint32_t>(ntiles, (uint32_t)num_sms()), kTcThreads, sizeof(TcSmem), st>>>(
+    k_propose_tc<<<std::min<uint32_t>(ntiles, (uint32_t)num_sms() * kTcCtas), kTcThreads, sizeof(TcSmem), st>>>(
         M, d_count, nchunks, H_, W4p_, node_of_treelet_, seeds, treelets, err ? err : err_);
     note_launches(2);
     return cudaGetLastError();
