@@ -869,8 +869,10 @@ struct PlocBufs {
 // The clusters alternate between two buffers, one round reading A and writing
 // B, the next the reverse; kPlocParity counts (mod 2) the rounds that ran, so
 // the current clusters are in B when it is 1 whatever no-op rounds followed.
-__global__ void k_ploc_state_init(const BoundsAcc* __restrict__ acc, uint32_t* __restrict__ ploc_state) {
+// bar, the cooperative rounds' barrier (or null), is zeroed too.
+__global__ void k_ploc_state_init(const BoundsAcc* __restrict__ acc, uint32_t* __restrict__ ploc_state, GridBarrier* bar) {
   if (threadIdx.x == 0) {
+    if (bar) bar->count = 0;
     const uint32_t n = acc->nvalid;
     ploc_state[kPlocN] = n;
     ploc_state[kPlocNext] = n;  // binary leaves are the primitives 0..n-1
@@ -1249,6 +1251,45 @@ __device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32
   return make_uint2(oa + xa - a, ob + xb - b);
 }
 
+// Every CTA of a cooperative launch gives a pair (a, b) of its thread 0; after the
+// grid barrier in here it has the sums of the pairs of the CTAs before it (in x and
+// y) and of all CTAs (z, w).  All threads call it; words holds gridDim.x pairs, and
+// another grid barrier lies between two calls.  False as grid_sync.  Reading tagged
+// words in a loop until all have arrived, without the barrier, is slower (152 CTAs
+// of 1024 threads: rounds of the 4M soup 580 us against 530, of 300k triangles 151
+// against 107; collapse of 8k triangles 50 against 46): the CTAs that wait then
+// delay the stores they wait for.
+template <int THREADS>
+__device__ __forceinline__ bool grid_sums(uint2* __restrict__ words, uint32_t a, uint32_t b, uint4& sums,
+                                          GridBarrier* bar, unsigned int* err) {
+  __shared__ uint4 s_sums[THREADS / 32];
+  if (threadIdx.x == 0) __stcg(words + blockIdx.x, make_uint2(a, b));
+  if (!grid_sync(bar, err)) return false;
+  uint4 s = make_uint4(0, 0, 0, 0);
+  for (uint32_t c = threadIdx.x; c < gridDim.x; c += THREADS) {
+    const uint2 v = __ldcg(words + c);
+    s.z += v.x;
+    s.w += v.y;
+    if (c < blockIdx.x) s.x += v.x, s.y += v.y;
+  }
+  const uint32_t warps = min(THREADS / 32u, (gridDim.x + 31u) / 32u);  // that read a word
+  if (threadIdx.x >> 5 < warps) {
+    s = make_uint4(__reduce_add_sync(0xFFFFFFFFu, s.x), __reduce_add_sync(0xFFFFFFFFu, s.y),
+                   __reduce_add_sync(0xFFFFFFFFu, s.z), __reduce_add_sync(0xFFFFFFFFu, s.w));
+    if ((threadIdx.x & 31) == 0) s_sums[threadIdx.x >> 5] = s;
+  }
+  __syncthreads();
+  sums = make_uint4(0, 0, 0, 0);
+  for (uint32_t k = 0; k < warps; k++) {
+    const uint4 o = s_sums[k];
+    sums.x += o.x;
+    sums.y += o.y;
+    sums.z += o.z;
+    sums.w += o.w;
+  }
+  return true;
+}
+
 // k_ploc_all for radius 1.  With one neighbour on either side a cluster's nearest
 // neighbour is the side of the smaller adjacent area (the left one in a tie, the
 // least (area, index)), so clusters i and i + 1 merge exactly where the adjacent
@@ -1258,15 +1299,18 @@ __device__ __forceinline__ uint2 block_excl_scan2(uint32_t a, uint32_t b, uint32
 // offsets by one block scan over the tiles, [barrier], (2) the tiles' outputs,
 // [barrier].  The tile-per-CTA form waits at six CTA barriers per 256 clusters,
 // which the threads that compute collapse costs reach last (17 of its 29 stall
-// cycles per issue).  tile_m, tile_s, tile_p: one word per tile.  Rounds of the 4M
-// soup: 732 us before, 581 us so (600 with a run of tiles per warp).
-__global__ void __launch_bounds__(PLOC_BLOCK, 4)
+// cycles per issue).  tile_m, tile_s, tile_p: one word per tile.  One CTA per SM: a
+// round ends at two grid barriers, and 152 CTAs arrive sooner and read fewer sums
+// than 608 of 256 threads.  Rounds of 8k / 300k / 1M / 4M triangles: 23 / 105 / 190 /
+// 527 us, with 4 x 256 threads per SM 27 / 129 / 216 / 563, with 2 x 512 23 / 110 /
+// 196 / 534 (tile per CTA: 732 us at 4M).
+constexpr int PLOC1_THREADS = 1024, PLOC1_CTAS = 1;
+__global__ void __launch_bounds__(PLOC1_THREADS, PLOC1_CTAS)
     k_ploc_rounds1(const PlocBufs bufs, uint32_t* __restrict__ ploc_state, uint32_t* tile_m, uint32_t* tile_s,
-                   uint32_t* tile_p, uint32_t* cta_sums, float4* __restrict__ bnbox, uint32_t* __restrict__ bncnt,
+                   uint32_t* tile_p, uint2* cta_sums, float4* __restrict__ bnbox, uint32_t* __restrict__ bncnt,
                    uint32_t node_cap, float4* __restrict__ dp_cost, uint4* __restrict__ dp_link, uint32_t leaf_max,
                    GridBarrier* bar, unsigned int* err) {
-  constexpr uint32_t kWarps = PLOC_BLOCK / 32;
-  __shared__ uint32_t s_red[4][kWarps];
+  constexpr uint32_t kWarps = PLOC1_THREADS / 32;
   __shared__ uint32_t s_before;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
   uint32_t n = __ldcg(ploc_state + kPlocN), node_next = __ldcg(ploc_state + kPlocNext);
@@ -1298,7 +1342,7 @@ __global__ void __launch_bounds__(PLOC_BLOCK, 4)
     __syncthreads();
     const uint32_t before = s_before;
     uint32_t ps = 0, pm = 0;
-    for (uint32_t k0 = t0; k0 < t1; k0 += PLOC_BLOCK) {
+    for (uint32_t k0 = t0; k0 < t1; k0 += PLOC1_THREADS) {
       const uint32_t t = k0 + threadIdx.x;
       uint32_t a = 0, b = 0;
       if (t < t1) {
@@ -1307,7 +1351,7 @@ __global__ void __launch_bounds__(PLOC_BLOCK, 4)
         b = __popc(m);
       }
       uint32_t ta, tb;
-      const uint2 e = block_excl_scan2(a, b, &ta, &tb);
+      const uint2 e = block_excl_scan2<PLOC1_THREADS>(a, b, &ta, &tb);
       if (t < t1) {
         tile_s[t] = ps + e.x;
         tile_p[t] = pm + e.y;
@@ -1315,54 +1359,22 @@ __global__ void __launch_bounds__(PLOC_BLOCK, 4)
       ps += ta;
       pm += tb;
     }
-    if (threadIdx.x == 0) {
-      __stcg(cta_sums + blockIdx.x, ps);
-      __stcg(cta_sums + gridDim.x + blockIdx.x, pm);
-    }
-    if (!grid_sync(bar, err)) break;
-    // (2) this CTA's offsets and the round's totals, then its tiles' outputs
-    uint32_t v[4] = {0u, 0u, 0u, 0u};  // prefix survivors, prefix merges, total survivors, total merges
-    for (uint32_t c0 = threadIdx.x; c0 < gridDim.x; c0 += 4 * PLOC_BLOCK) {
-      uint32_t a[4], b[4];  // read together
-#pragma unroll
-      for (uint32_t q = 0; q < 4; q++) {
-        const uint32_t c = c0 + q * PLOC_BLOCK;
-        a[q] = c < gridDim.x ? __ldcg(cta_sums + c) : 0u;
-        b[q] = c < gridDim.x ? __ldcg(cta_sums + gridDim.x + c) : 0u;
-      }
-#pragma unroll
-      for (uint32_t q = 0; q < 4; q++) {
-        v[2] += a[q];
-        v[3] += b[q];
-        if (c0 + q * PLOC_BLOCK < blockIdx.x) {
-          v[0] += a[q];
-          v[1] += b[q];
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      v[q] = __reduce_add_sync(0xFFFFFFFFu, v[q]);
-      if (lane == 0) s_red[q][warp] = v[q];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      v[q] = 0;
-      for (uint32_t w = 0; w < kWarps; w++) v[q] += s_red[q][w];
-    }
+    // (2) this CTA's offsets and the round's totals (survivors, merges), then its
+    // tiles' outputs
+    uint4 v;
+    if (!grid_sums<PLOC1_THREADS>(cta_sums, ps, pm, v, bar, err)) break;
     for (uint32_t t = t0 + warp; t < t1; t += kWarps) {
       const uint32_t m = tile_m[t], i = 32u * t + lane, carry = t > t0 ? tile_m[t - 1] >> 31 : before;
       const uint32_t s0 = tile_s[t], m0 = tile_p[t];
       const uint32_t in = min(n - 32u * t, 32u), absorbed = (m << 1) | carry;
       const uint32_t alive = (in == 32u ? 0xFFFFFFFFu : (1u << in) - 1u) & ~absorbed;
       if (alive >> lane & 1u)
-        ploc_emit_one(bufs, par, i, m >> lane & 1u ? i + 1u : i, v[0] + s0 + __popc(alive & lt),
-                      node_next + v[1] + m0 + __popc(m & lt), n, bnbox, bncnt, node_cap, err, dp_cost, dp_link, leaf_max);
+        ploc_emit_one(bufs, par, i, m >> lane & 1u ? i + 1u : i, v.x + s0 + __popc(alive & lt),
+                      node_next + v.y + m0 + __popc(m & lt), n, bnbox, bncnt, node_cap, err, dp_cost, dp_link, leaf_max);
     }
     // next round (the k_ploc_advance rules, alike in every CTA)
-    const uint32_t merged = v[3];
-    n = v[2];
+    const uint32_t merged = v.w;
+    n = v.z;
     node_next += merged;
     rounds += merged > 0 ? 1u : 0u;
     par ^= 1u;
@@ -1963,18 +1975,16 @@ __device__ __forceinline__ uint32_t cta_excl_scan_1024(uint32_t v, uint32_t* s_w
 // First level: the roots of the non-empty segments in segment order (one CTA
 // of 1024 threads, nseg <= 4 x 1024); seg_index[s] = position of segment s's
 // root (kInvalidID for an empty segment).  It also zeroes what the collapse adds
-// to (cstate, the SAH sums, the leaf count, the CTA sums and barrier of
-// k_collapse_all): as memsets these were four launches of a captured build.
+// to (cstate, the SAH sums, the leaf count, the barrier of k_collapse_all): as
+// memsets these were four launches of a captured build.
 __global__ void __launch_bounds__(1024) k_collapse_roots(const uint32_t* __restrict__ d_root, uint32_t nseg,
                                                          uint32_t nbin, uint32_t* __restrict__ items,
                                                          uint32_t* __restrict__ seg_index,
                                                          uint32_t* __restrict__ cstate, double* __restrict__ sah_acc,
                                                          uint32_t* __restrict__ leaf_count,
-                                                         unsigned long long* __restrict__ cta_sums, uint32_t nsums,
                                                          GridBarrier* __restrict__ bar) {
   __shared__ uint32_t s_w[32];
   for (uint32_t k = threadIdx.x; k < (uint32_t)kColStateWords; k += 1024) cstate[k] = 0;
-  for (uint32_t k = threadIdx.x; k < nsums; k += 1024) cta_sums[k] = 0ull;
   if (threadIdx.x < 2) sah_acc[threadIdx.x] = 0.0;
   if (threadIdx.x == 0) {
     *leaf_count = 0;
@@ -2318,73 +2328,23 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_emit(
 // Threads of a CTA of k_collapse_all, one CTA per SM: 512 threads have registers for
 // two node's reads in flight and wait less at each other (a level of few nodes takes
 // 13,000 cycles against 16,000), 1024 threads have the warps that a wide level needs.
-// The levels of a tree of 8k / 300k / 1M / 4M triangles take 50 / 150 / 273 / 726 us
-// with 512 threads and 57 / 161 / 254 / 583 with 1024, so the line lies between 300k
-// and 1M.  (Four CTAs of 256 threads per SM: 73 / 217 / - / 664, most of it at the
-// barriers, where 608 CTAs arrive and read each other's sums instead of 152.)
+// The levels of a tree of 8k / 300k / 1M / 4M triangles take 44 / 137 / 269 / 744 us
+// with 512 threads and 53 / 144 / 244 / 573 with 1024, so the line lies between 300k
+// and 1M.  (Four CTAs of 256 threads per SM waited longer at the barriers, where 608
+// arrive and read each other's sums instead of 152.)
 constexpr int COLLAPSE_NARROW_THREADS = 512, COLLAPSE_WIDE_THREADS = 1024;
 constexpr uint32_t COLLAPSE_WIDE_TRIS = 1u << 19;
-
-// Every CTA of a cooperative launch gives a pair (a, b), below 2^28 each, of its
-// thread 0 and gets the sums of the pairs of the CTAs before it (in x and y) and of
-// all CTAs (z, w); all threads call it.  The words of all CTAs are zero before the
-// launch, tag is not zero and another one in each call, and a grid barrier lies
-// between two calls.  A CTA reads the others' words until they bear the tag, so no
-// barrier and second read of the sums is needed: 1,150 cycles with 152 CTAs of 512
-// threads and 1,750 with 1024, where the barrier, the sums and their block scans took
-// 6,000 with 608 of 256.
-template <int THREADS>
-__device__ __forceinline__ bool grid_sums(unsigned long long* __restrict__ words, uint32_t tag, uint32_t a, uint32_t b,
-                                          uint4& sums, unsigned int* err) {
-  __shared__ uint4 s_sums[THREADS / 32];
-  if (threadIdx.x == 0) {
-    if ((a | b) >> 28) atomicOr(err, kErrBuild);
-    *reinterpret_cast<volatile unsigned long long*>(words + blockIdx.x) =
-        (unsigned long long)tag << 56 | (unsigned long long)(b & 0xFFFFFFFu) << 28 | (a & 0xFFFFFFFu);
-  }
-  uint4 s = make_uint4(0, 0, 0, 0);
-  bool ok = true;
-  for (uint32_t c = threadIdx.x; c < gridDim.x; c += THREADS) {
-    const volatile unsigned long long* w = words + c;
-    unsigned long long v = *w;
-    for (uint32_t it = 0; ok && (uint32_t)(v >> 56) != tag; it++) {
-      if (it == kLbSpinLimit) atomicOr(err, kErrBuild);
-      ok = it < kLbSpinLimit && lb_load(err) == 0u;
-      v = *w;
-    }
-    const uint32_t x = (uint32_t)v & 0xFFFFFFFu, y = (uint32_t)(v >> 28) & 0xFFFFFFFu;
-    s.z += x;
-    s.w += y;
-    if (c < blockIdx.x) s.x += x, s.y += y;
-  }
-  const uint32_t warps = min(THREADS / 32u, (gridDim.x + 31u) / 32u);  // that read a word
-  if (threadIdx.x >> 5 < warps) {
-    s = make_uint4(__reduce_add_sync(0xFFFFFFFFu, s.x), __reduce_add_sync(0xFFFFFFFFu, s.y),
-                   __reduce_add_sync(0xFFFFFFFFu, s.z), __reduce_add_sync(0xFFFFFFFFu, s.w));
-    if ((threadIdx.x & 31) == 0) s_sums[threadIdx.x >> 5] = s;
-  }
-  ok = __syncthreads_and(ok);
-  sums = make_uint4(0, 0, 0, 0);
-  for (uint32_t k = 0; k < warps; k++) {
-    const uint4 o = s_sums[k];
-    sums.x += o.x;
-    sums.y += o.y;
-    sums.z += o.z;
-    sums.w += o.w;
-  }
-  return ok;
-}
 
 // Every level of the collapse, from the roots in cstate: each CTA takes a
 // contiguous chunk of the level's items, (1) gathers their children and counts
 // internal children and leaf triangles, (2) scans the counts within the chunk and
-// sums them with the other CTAs (grid_sums), (3) writes its wide nodes and the next
-// level's items, [barrier].  cta_sums holds gridDim.x words; these and *bar are zero
-// on entry.
+// sums them with the other CTAs (grid_sums), [barrier in there], (3) writes its wide
+// nodes and the next level's items, [barrier].  cta_sums holds gridDim.x pairs; *bar
+// is zero on entry.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_collapse_all(
     BinTree t, const ColItems ci, uint32_t* __restrict__ cstate, uint32_t* __restrict__ kids,
-    uint32_t* __restrict__ nint, uint32_t* __restrict__ ntri, unsigned long long* __restrict__ cta_sums,
+    uint32_t* __restrict__ nint, uint32_t* __restrict__ ntri, uint2* __restrict__ cta_sums,
     WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root, double* sah_acc, uint32_t* leaf_count,
     uint32_t node_cap, uint32_t tri_cap, uint32_t max_levels, GridBarrier* bar, unsigned int* err) {
   uint32_t nitems = __ldcg(cstate + kColN), base = __ldcg(cstate + kColBase), tri_next = __ldcg(cstate + kColTri),
@@ -2440,7 +2400,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_collapse_all(
       ct_sum += tb;
     }
     uint4 sums;
-    if (!grid_sums<THREADS>(cta_sums, depth + 1u, ci_sum, ct_sum, sums, err)) break;
+    if (!grid_sums<THREADS>(cta_sums, ci_sum, ct_sum, sums, bar, err)) break;
     // (3) the wide nodes of this CTA's items, one per 8-lane group
     for (uint32_t k0 = first + ((threadIdx.x & ~31u) >> 3); k0 < last; k0 += blockDim.x >> 3) {
       const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
@@ -2818,7 +2778,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   GB_CHECK(arena.alloc(&ploc_state, kPlocStateWords));
   uint32_t* h_tot = nullptr;
   GB_CHECK(arena.host(&h_tot, kPlocStateWords));
-  k_ploc_state_init<<<1, 32, 0, st>>>(acc, ploc_state);
+  k_ploc_state_init<<<1, 32, 0, st>>>(acc, ploc_state, nullptr);
   note_launches(1);
   const int radius = opt.ploc_radius == 1 || opt.ploc_radius == 2 || opt.ploc_radius == 4 || opt.ploc_radius == 8
                          ? opt.ploc_radius
@@ -2910,8 +2870,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   GB_CHECK(arena.alloc(&cstate, kColStateWords));
   GB_CHECK(arena.alloc(&seg_index, nseg));
   GB_CHECK(arena.host(&h_col, kColStateWords));
-  k_collapse_roots<<<1, 1024, 0, st>>>(d_root, nseg, nnodes_bin, items_a, seg_index, cstate, d_sah, d_leaves, nullptr, 0,
-                                       nullptr);
+  k_collapse_roots<<<1, 1024, 0, st>>>(d_root, nseg, nnodes_bin, items_a, seg_index, cstate, d_sah, d_leaves, nullptr);
   note_launches(1);
   const ColItems citems{{items_a, items_b}};
   uint32_t level = 0;
@@ -3102,8 +3061,10 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
                      : g->radius == 4 ? (const void*)k_ploc_all<4>
                      : g->radius == 8 ? (const void*)k_ploc_all<8>
                                       : (const void*)k_ploc_all<PLOC_R_MAX>;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk, PLOC_BLOCK, 0)) != cudaSuccess) return e;
-    g->ploc_grid = (uint32_t)std::max(1, std::min(per_sm, 8)) * (uint32_t)num_sms_build();
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk, g->radius == 1 ? PLOC1_THREADS : PLOC_BLOCK, 0)) !=
+        cudaSuccess)
+      return e;
+    g->ploc_grid = (uint32_t)std::max(1, std::min(per_sm, g->radius == 1 ? PLOC1_CTAS : 8)) * (uint32_t)num_sms_build();
   }
   if ((e = alloc(&g->d_geoms, ngeoms)) || (e = alloc(&g->pbox, 2 * (size_t)T)) ||
       (e = alloc(&acc, 1)) || (e = alloc(&g->keys_a, T)) || (e = alloc(&g->keys_b, T)) ||
@@ -3183,16 +3144,15 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   k_ploc_init<<<cdiv(N, 256), 256, 0, st>>>(g.pbox, va, N, &acc->nvalid, g.bnbox, g.cidx[0],
                                             g.clo[0], g.chi[0], g.opt.segmented ? 1 : 0);
   stamp(3);
-  k_ploc_state_init<<<1, 32, 0, st>>>(acc, g.ploc_state);
+  k_ploc_state_init<<<1, 32, 0, st>>>(acc, g.ploc_state, reinterpret_cast<GridBarrier*>(g.ploc_bar));
   note_launches(2);
   const uint32_t nbin_cap = 2 * N;
   const PlocBufs pb{{g.clo[0], g.clo[1]}, {g.chi[0], g.chi[1]}, {g.cidx[0], g.cidx[1]}};
   // the rounds above PLOC_SMALL clusters in one cooperative launch, then the one-CTA finish
-  GB_CHECK(cudaMemsetAsync(g.ploc_bar, 0, sizeof(GridBarrier), st));
   {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.ploc_grid);
-    cfg.blockDim = dim3(PLOC_BLOCK);
+    cfg.blockDim = dim3(g.radius == 1 ? PLOC1_THREADS : PLOC_BLOCK);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -3202,7 +3162,8 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
     cfg.numAttrs = 1;
     GridBarrier* bar = reinterpret_cast<GridBarrier*>(g.ploc_bar);
     switch (g.radius) {
-      case 1: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_rounds1, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
+      case 1: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_rounds1, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge,
+                                          reinterpret_cast<uint2*>(g.ploc_sums),
                                           g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar, &acc->pad)); break;
       case 2: GB_CHECK(cudaLaunchKernelEx(&cfg, k_ploc_all<2>, pb, g.ploc_state, g.nn, g.bsurv, g.bmerge, g.ploc_sums,
                                           g.bnbox, g.bncnt, nbin_cap, dp_cost, dp_link, leaf_max, bar,
@@ -3232,7 +3193,7 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   stamp(6);
   // all collapse levels in one cooperative launch
   k_collapse_roots<<<1, 1024, 0, st>>>(g.d_root, g.nseg, g.nbin, g.items[0], g.seg_index, g.cstate, g.d_sah, g.d_leaves,
-                                       g.col_sums, g.col_grid, reinterpret_cast<GridBarrier*>(g.col_bar));
+                                       reinterpret_cast<GridBarrier*>(g.col_bar));
   {
     const ColItems ci{{g.items[0], g.items[1]}};
     cudaLaunchConfig_t cfg = {};

@@ -87,7 +87,7 @@ struct GraphBuild {
   GraphBuildOut* out = nullptr;                         // results (page-locked host memory)
   uint32_t col_grid = 0;                                // CTAs of the cooperative collapse
   int col_threads = 0;                     // of a CTA of the cooperative collapse
-  unsigned long long* col_sums = nullptr;  // its per-CTA sums
+  uint2* col_sums = nullptr;               // its per-CTA sums
   uint32_t* col_bar = nullptr;             // and grid barrier
   TriRecord* prec = nullptr;                            // leaf records in primitive order
   unsigned long long* stamps = nullptr;                 // phase timestamps (BuildOptions::phase_stamps)
