@@ -347,8 +347,13 @@ cudaError_t copy_device(void* dst, const void* src, size_t bytes, cudaStream_t s
 // stable 8-bit LSD sort, one histogram + scatter round per digit over task blocks.
 
 constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 16;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
+// Keys per thread: 16 where the tiles fill the chip, else 4, so that more SMs work
+// and a tile's rows are ranked in a quarter of the time.  Sort of 8k / 60k / 120k /
+// 250k keys of 30 bits with 4: 27 / 34 / 40 / 52 us, with 16: 42 / 48 / 51 / 57 us;
+// of 300k 55 / 58, of 600k 78 / 65 us.
+constexpr int RS_ITEMS = 16, RS_FEW_ITEMS = 4;
+constexpr uint32_t RS_FEW = 1u << 18;
+constexpr uint32_t os_tile(uint32_t n) { return RS_THREADS * (n <= RS_FEW ? RS_FEW_ITEMS : RS_ITEMS); }
 
 // look-back status words: flag bits over a 30-bit count
 constexpr uint32_t kLbAggregate = 1u << 30;   // the tile's own count is published
@@ -442,17 +447,33 @@ __global__ void __launch_bounds__(256) k_os_hist(const K* __restrict__ keys, uin
 // the keys are placed in shared memory in (digit, original order) order and written
 // out in runs, consecutive threads to consecutive positions of a digit's bucket.
 constexpr int RS_WARPS = RS_THREADS / 32;
-template <typename K>
-constexpr size_t os_scatter_smem() { return (size_t)RS_TILE * (sizeof(K) + sizeof(uint32_t)); }
 
-template <typename K>
+// Lanes of the warp whose keys are in and have this lane's digit d (8 bits), for a
+// lane whose key is: a vote per bit (with match_any, whose time grows with the number
+// of different digits, the sort of 4M keys took 224 us instead of 189).
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool in) {
+  uint32_t peers = __ballot_sync(0xFFFFFFFFu, in);
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    const bool one = d >> b & 1u;
+    const uint32_t vote = __ballot_sync(0xFFFFFFFFu, one);
+    peers &= one ? vote : ~vote;
+  }
+  return peers;
+}
+
+template <typename K, int ITEMS>
+constexpr size_t os_scatter_smem() { return (size_t)RS_THREADS * ITEMS * (sizeof(K) + sizeof(uint32_t)); }
+
+template <typename K, int ITEMS>
 __global__ void __launch_bounds__(RS_THREADS) k_os_scatter(const K* __restrict__ kin,
                                                            const uint32_t* __restrict__ vin,
                                                            K* __restrict__ kout, uint32_t* __restrict__ vout,
                                                            uint32_t n, int shift, uint32_t* __restrict__ scratch,
                                                            uint32_t pass_slot, uint32_t* __restrict__ status,
                                                            unsigned int* __restrict__ err) {
-  extern __shared__ __align__(16) unsigned char s_stage[];               // RS_TILE keys, then RS_TILE values
+  extern __shared__ __align__(16) unsigned char s_stage[];               // the tile's keys, then its values
+  constexpr int RS_TILE = RS_THREADS * ITEMS;
   K* s_keys = reinterpret_cast<K*>(s_stage);
   uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + RS_TILE);
   __shared__ uint32_t s_tile;
@@ -470,16 +491,16 @@ __global__ void __launch_bounds__(RS_THREADS) k_os_scatter(const K* __restrict__
   const uint32_t tile_n = min((uint32_t)RS_TILE, n - base);
   const uint32_t lt = (1u << lane) - 1u;
   // ---- per-warp ranking (warp-synchronous: each warp owns its row of s_wcnt)
-  K k[RS_ITEMS];
-  uint32_t pos[RS_ITEMS];
-  const uint32_t wbase = base + (uint32_t)warp * (RS_ITEMS * 32);
+  K k[ITEMS];
+  uint32_t pos[ITEMS];
+  const uint32_t wbase = base + (uint32_t)warp * (ITEMS * 32);
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; r++) {
+  for (int r = 0; r < ITEMS; r++) {
     const uint32_t i = wbase + r * 32 + lane;
     const bool in = i < n;
     k[r] = in ? kin[i] : (K)0;
-    const uint32_t d = in ? (uint32_t)(k[r] >> shift) & 0xFFu : 256u;
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+    const uint32_t d = (uint32_t)(k[r] >> shift) & 0xFFu;
+    const uint32_t peers = digit_peers(d, in);
     const uint32_t rank = __popc(peers & lt);
     pos[r] = (in ? s_wcnt[warp][d] : 0u) + rank;
     __syncwarp();
@@ -523,7 +544,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_os_scatter(const K* __restrict__
   __syncthreads();
   // ---- keys to shared memory in (digit, original order) order
 #pragma unroll
-  for (int r = 0; r < RS_ITEMS; r++) {
+  for (int r = 0; r < ITEMS; r++) {
     const uint32_t i = wbase + r * 32 + lane;
     if (i < n) {
       const uint32_t d = (uint32_t)(k[r] >> shift) & 0xFFu;
@@ -542,6 +563,119 @@ __global__ void __launch_bounds__(RS_THREADS) k_os_scatter(const K* __restrict__
       vout[out] = s_vals[j];
     } else {
       atomicOr(err, kErrBuild);
+    }
+  }
+}
+
+// The same sort of at most kSortOneMax keys by one CTA that keeps keys and values on
+// chip over all passes (result in keys / vals).  Each pass ranks the keys as
+// k_os_scatter does -- warp w those from w * 32 * ROWS on, row by row -- and places
+// them by the digits' starts and the counts of the warps before.  A small build's
+// sort is a chain of launches (a memset, the histogram, four scatters): 512 / 2048 /
+// 3872 keys of 30 bits take 18 / 23 / 25 us so and 14 / 15 / 16 us in one CTA, 8192
+// 27 us so and 29 in one CTA of 8 rows.
+constexpr int kSortOneThreads = 1024, kSortOneWarps = kSortOneThreads / 32, kSortOneRows = 4;
+constexpr uint32_t kSortOneMax = kSortOneThreads * kSortOneRows;
+template <typename K>
+constexpr size_t sort_one_smem() {
+  return (sizeof(K) + sizeof(uint32_t)) * kSortOneMax + sizeof(uint32_t) * kSortOneWarps * 256;
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kSortOneThreads, 1) k_sort_one(K* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                                 uint32_t n, uint32_t digit_mask) {
+  constexpr int ROWS = kSortOneRows;
+  extern __shared__ __align__(16) unsigned char s_one[];
+  K* s_keys = reinterpret_cast<K*>(s_one);
+  uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + kSortOneMax);
+  uint32_t(*s_cnt)[256] = reinterpret_cast<uint32_t(*)[256]>(s_vals + kSortOneMax);  // per warp: its digit counts
+  __shared__ uint32_t s_group[4][256];  // per 8 warps: counts of each digit, then where they start
+  __shared__ uint32_t s_w[8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int digit = tid & 255, group = tid >> 8;
+  const uint32_t lt = (1u << lane) - 1u, base = (uint32_t)warp * (32 * ROWS) + lane;
+  K k[ROWS];
+  uint32_t v[ROWS], pos[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; r++) {
+    const uint32_t i = base + 32 * r;
+    k[r] = i < n ? keys[i] : (K)0;
+    v[r] = i < n ? vals[i] : 0u;
+  }
+  for (int pass = 0; pass < (int)sizeof(K); pass++) {
+    if (!(digit_mask >> pass & 1u)) continue;
+    const int shift = 8 * pass;
+#pragma unroll
+    for (int w = 0; w < 8; w++) s_cnt[8 * group + w][digit] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      const bool in = base + 32 * r < n;
+      const uint32_t d = (uint32_t)(k[r] >> shift) & 0xFFu;
+      const uint32_t peers = digit_peers(d, in), rank = __popc(peers & lt);
+      pos[r] = (in ? s_cnt[warp][d] : 0u) + rank;
+      __syncwarp();
+      if (in && rank == 0) s_cnt[warp][d] += __popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t sum = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      const uint32_t c = s_cnt[8 * group + w][digit];
+      s_cnt[8 * group + w][digit] = sum;
+      sum += c;
+    }
+    s_group[group][digit] = sum;
+    __syncthreads();
+    uint32_t g[4] = {0u, 0u, 0u, 0u}, x = 0, total = 0;
+    if (tid < 256) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        g[q] = total;
+        total += s_group[q][tid];
+      }
+      x = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) s_w[warp] = x;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t start = x - total;
+      for (int w = 0; w < warp; w++) start += s_w[w];
+#pragma unroll
+      for (int q = 0; q < 4; q++) s_group[q][tid] = start + g[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      if (base + 32 * r < n) {
+        const uint32_t d = (uint32_t)(k[r] >> shift) & 0xFFu;
+        const uint32_t j = s_group[warp >> 3][d] + s_cnt[warp][d] + pos[r];  // a permutation of 0 .. n - 1
+        s_keys[j] = k[r];
+        s_vals[j] = v[r];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+      const uint32_t i = base + 32 * r;
+      if (i < n) {
+        k[r] = s_keys[i];
+        v[r] = s_vals[i];
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; r++) {
+    const uint32_t i = base + 32 * r;
+    if (i < n) {
+      keys[i] = k[r];
+      vals[i] = v[r];
     }
   }
 }
@@ -2528,7 +2662,7 @@ static void scan_excl2(uint32_t* a, uint32_t* b, uint32_t n, uint32_t* ta, uint3
 
 // Scratch words of onesweep_sort for n keys and `passes` digit passes.
 static inline size_t onesweep_scratch_words(uint32_t n, int passes) {
-  return kOsStatus + (size_t)passes * cdiv(n, RS_TILE) * 256u;
+  return kOsStatus + (size_t)passes * cdiv(n, os_tile(n)) * 256u;
 }
 
 // Stable LSD sort of (ka, va) by the digits set in digit_mask (bit d: key bits
@@ -2543,23 +2677,35 @@ static cudaError_t onesweep_sort(K*& ka, uint32_t*& va, K*& kb, uint32_t*& vb, u
   const int passes = __builtin_popcount(digit_mask);
   if (n == 0 || passes == 0) return cudaSuccess;
   if (n >= kLbValue) return cudaErrorInvalidValue;  // look-back counts are 30-bit
-  const uint32_t ntiles = cdiv(n, RS_TILE);
+  if (n <= kSortOneMax) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GB_CHECK(cudaStreamIsCapturing(st, &cap));
+    if (cap == cudaStreamCaptureStatusNone)
+      GB_CHECK(cudaFuncSetAttribute(k_sort_one<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_one_smem<K>()));
+    if (!err) GB_CHECK(cudaMemsetAsync(scratch + kOsErr, 0, sizeof(uint32_t), st));
+    k_sort_one<K><<<1, kSortOneThreads, sort_one_smem<K>(), st>>>(ka, va, n, digit_mask);
+    note_launches(1);
+    return cudaGetLastError();
+  }
+  const uint32_t ntiles = cdiv(n, os_tile(n));
   GB_CHECK(cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * onesweep_scratch_words(n, passes), st));
   const uint32_t hgrid = std::min<uint32_t>(ntiles, 4u * (uint32_t)num_sms_build());
-  // 32 or 48 KB of staged keys and values beyond the static shared memory (per
+  // up to 48 KB of staged keys and values beyond the static shared memory (per
   // device; a captured build sets it in graph_build_prepare)
-  constexpr size_t smem = os_scatter_smem<K>();
+  const bool few = n <= RS_FEW;
+  const auto scatter = few ? k_os_scatter<K, RS_FEW_ITEMS> : k_os_scatter<K, RS_ITEMS>;
+  const size_t smem = few ? os_scatter_smem<K, RS_FEW_ITEMS>() : os_scatter_smem<K, RS_ITEMS>();
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   GB_CHECK(cudaStreamIsCapturing(st, &cap));
   if (cap == cudaStreamCaptureStatusNone)
-    GB_CHECK(cudaFuncSetAttribute(k_os_scatter<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GB_CHECK(cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_os_hist<K><<<hgrid, 256, 0, st>>>(ka, n, digit_mask & ((1u << sizeof(K)) - 1u), scratch);
   uint32_t slot = 0;
   for (int d = 0; d < (int)sizeof(K); d++) {
     if (!(digit_mask >> d & 1u)) continue;
-    k_os_scatter<K><<<ntiles, RS_THREADS, smem, st>>>(ka, va, kb, vb, n, 8 * d, scratch, slot,
-                                                      scratch + kOsStatus + (size_t)slot * ntiles * 256u,
-                                                      err ? err : scratch + kOsErr);
+    scatter<<<ntiles, RS_THREADS, smem, st>>>(ka, va, kb, vb, n, 8 * d, scratch, slot,
+                                              scratch + kOsStatus + (size_t)slot * ntiles * 256u,
+                                              err ? err : scratch + kOsErr);
     std::swap(ka, kb);
     std::swap(va, vb);
     slot++;
@@ -3034,7 +3180,7 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
   g->nbin = 2 * N - plan.roots;
   g->maxw = N;
   g->maxb = cdiv(N, PLOC_BLOCK);
-  g->rs_blocks = cdiv(g->total, RS_TILE);
+  g->rs_blocks = cdiv(g->total, os_tile(g->total));
   g->radius = (opt.ploc_radius == 1 || opt.ploc_radius == 2 || opt.ploc_radius == 4 || opt.ploc_radius == 8)
                   ? (uint32_t)opt.ploc_radius
                   : (uint32_t)PLOC_R_MAX;
@@ -3095,13 +3241,19 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
   if (e == cudaSuccess)
     e = cudaMemset(g->scan_sums, 0, sizeof(uint32_t) * 2 * scan_scratch(std::max(g->maxb, maxw)));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_os_scatter<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)os_scatter_smem<uint64_t>());
+    e = cudaFuncSetAttribute(k_os_scatter<uint64_t, RS_ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)os_scatter_smem<uint64_t, RS_ITEMS>());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_os_scatter<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)os_scatter_smem<uint32_t>());
-  if (e != cudaSuccess) graph_build_release(g);
+    e = cudaFuncSetAttribute(k_os_scatter<uint32_t, RS_ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)os_scatter_smem<uint32_t, RS_ITEMS>());
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_sort_one<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sort_one_smem<uint64_t>());
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_sort_one<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sort_one_smem<uint32_t>());
   if (e == cudaSuccess) e = ploc_finish_prepare();
+  if (e != cudaSuccess) graph_build_release(g);
   return e;
 }
 
