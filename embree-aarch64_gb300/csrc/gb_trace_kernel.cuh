@@ -266,11 +266,17 @@ struct Ctx {
   uint32_t num_tris;
 };
 
-// Batched queries look up each ray's batch when they fetch it, and their scenes
-// are small (8 node visits a ray), so fetching weighs more: a warp waits for this
-// many times the idle lanes of the launch shape.  128 scenes, 14.6M rays: 2.08 ms
-// with a factor of 1, 1.95 with 2, 1.93 with 3, 2.01 with 4.
-constexpr int kBatchedRefill = 3;
+// A refill runs with the idle lanes alone, so it weighs more the fewer nodes a ray
+// visits: where the rays that a warp last ended visited fewer than kShortVisits nodes
+// each, it waits for kShortRefill times the idle lanes of the launch shape.  Kernel
+// time without / with: 1M primary rays on the 131k heightfield (3.5 nodes a ray)
+// 92.8 / 84.6 us, 1M rays in a robust scene (3.2) 181 / 171 us, 14.6M batched rays
+// (8) 2.08 / 1.92 ms, 16M rays on the 4M soup (34) 9.32 / 9.25 ms; waiting for three
+// times the lanes always costs the soup's shadow rays 9 %.  Twice 91 and 174 us, four
+// times 88 and 166 us but 1 % on the batched rays.  Scenes with instances, whose rays
+// that miss all instances are short, lose 1.5 % and do without.
+constexpr uint32_t kShortVisits = 12;
+constexpr int kShortRefill = 3;
 
 // Leaves wait for their triangle tests in a ring per warp (k_trace below): up
 // to 31 waiting + 32 new.
@@ -297,7 +303,8 @@ __device__ __forceinline__ void load_ray(const char* p, TRay& r, float& tfar) {
 }
 
 // Persistent traversal.  Every lane owns one ray at a time; a warp refills
-// its idle lanes with one atomic once SH::kRefillIdle of them are idle.  Each
+// its idle lanes with one atomic once SH::kRefillIdle of them are idle (three times
+// as many where rays are short).  Each
 // loop iteration an active lane (1) visits one node of its current group,
 // (2) queues the triangles of the leaves it hit, and (3) pops the stack when
 // its group is exhausted.
@@ -433,7 +440,8 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
     --sp;
     return sp < kSharedStack ? s_stack[sp][stk_tid] : stack[sp];
   };
-  bool active = false, exhausted = false, seeding = false;
+  int wait = SH::kRefillIdle;  // idle lanes to wait for before a refill; 33: no ray is left
+  bool active = false, seeding = false;
   uint32_t rid = 0;
   TRay r;
   r.org = r.dir = r.rdir = make_float3(0.f, 0.f, 0.f);
@@ -563,7 +571,7 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
   for (;;) {
     // ---- write finished rays, refill idle lanes
     uint32_t idle = __ballot_sync(0xFFFFFFFFu, !active);
-    const bool refill = idle == 0xFFFFFFFFu || (!exhausted && __popc(idle) >= SH::kRefillIdle * (P.batch_root ? kBatchedRefill : 1));
+    const bool refill = idle == 0xFFFFFFFFu || __popc(idle) >= wait;
     // waiting leaves (at most 31: one batch empties the ring) are tested before a
     // refill and once there is one per active lane
     if (!INST && qtail != qhead && (refill || qtail - qhead + __popc(idle) >= 32u)) {
@@ -602,12 +610,14 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
           }
         }
       }
-      if (exhausted) break;  // no ray left, no lane active
+      if (wait > 32) break;  // no ray left, no lane active
+      const uint32_t visits = INST ? 0u : __reduce_add_sync(0xFFFFFFFFu, active ? 0u : iters);  // of the rays that ended
+      wait = !INST && visits < kShortVisits * __popc(idle) ? min(SH::kRefillIdle * kShortRefill, 32) : SH::kRefillIdle;
       const int leader = __ffs(idle) - 1;
       uint32_t base = 0;
       if (lane == leader) base = atomicAdd(P.ray_counter, (unsigned)__popc(idle));
       base = __shfl_sync(0xFFFFFFFFu, base, leader);
-      if (base + __popc(idle) >= nrays) exhausted = true;
+      if (base + __popc(idle) >= nrays) wait = 33;
       if (!active) {
         rid = base + __popc(idle & lt_mask);
         if (rid < nrays) {
