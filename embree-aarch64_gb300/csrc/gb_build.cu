@@ -2205,6 +2205,9 @@ __global__ void k_collapse_advance(const uint32_t* __restrict__ tot, uint32_t* _
   if (next == 0 && d + 1 <= (uint32_t)kColMaxLevels) cstate[kColLevels + d + 1] = base;  // end of the last level
 }
 
+// A plane byte as a float, without a conversion: in the mantissa of 2^23.
+__device__ __forceinline__ float byte_f(uint32_t q) { return __uint_as_float(0x4B000000u | q) - 8388608.0f; }
+
 __device__ __forceinline__ uint32_t exp_for(float ext) {
   // smallest power of two 2^(E-127) with 255 * 2^(E-127) >= ext: with ext = m 2^e,
   // 1 <= m < 2, that is e - 7 while m <= 255 / 128 and e - 6 above
@@ -2373,9 +2376,8 @@ __device__ __forceinline__ void collapse_emit_group(
     const uint32_t qhx = min(__float2uint_ru(__fsub_ru(hi.x, ulo.x) * ix), 255u);
     const uint32_t qhy = min(__float2uint_ru(__fsub_ru(hi.y, ulo.y) * iy), 255u);
     const uint32_t qhz = min(__float2uint_ru(__fsub_ru(hi.z, ulo.z) * iz), 255u);
-    // a byte as a float: in the mantissa of 2^23
-    auto f = [](uint32_t q) { return __uint_as_float(0x4B000000u | q) - 8388608.0f; };
-    const float flx = f(qlx), fly = f(qly), flz = f(qlz), fhx = f(qhx), fhy = f(qhy), fhz = f(qhz);
+    const float flx = byte_f(qlx), fly = byte_f(qly), flz = byte_f(qlz), fhx = byte_f(qhx), fhy = byte_f(qhy),
+                fhz = byte_f(qhz);
     // decoded (outward-rounded) box, as traversal sees it
     const float3 dlo = make_float3(__fmaf_rd(flx, sx, ulo.x), __fmaf_rd(fly, sy, ulo.y), __fmaf_rd(flz, sz, ulo.z));
     const float3 dhi = make_float3(__fmaf_ru(fhx, sx, ulo.x), __fmaf_ru(fhy, sy, ulo.y), __fmaf_ru(fhz, sz, ulo.z));
@@ -3639,16 +3641,16 @@ __device__ __forceinline__ void refit_node_group(const float4* tri_box, uint32_t
   if (m != 0) {
     const float ix = __uint_as_float((254u - Ex) << 23), iy = __uint_as_float((254u - Ey) << 23),
                 iz = __uint_as_float((254u - Ez) << 23);
-    const float qlx = fminf(fmaxf(floorf(__fsub_rd(lo.x, ulo.x) * ix), 0.f), 255.f);
-    const float qly = fminf(fmaxf(floorf(__fsub_rd(lo.y, ulo.y) * iy), 0.f), 255.f);
-    const float qlz = fminf(fmaxf(floorf(__fsub_rd(lo.z, ulo.z) * iz), 0.f), 255.f);
-    const float qhx = fminf(fmaxf(ceilf(__fsub_ru(hi.x, ulo.x) * ix), 0.f), 255.f);
-    const float qhy = fminf(fmaxf(ceilf(__fsub_ru(hi.y, ulo.y) * iy), 0.f), 255.f);
-    const float qhz = fminf(fmaxf(ceilf(__fsub_ru(hi.z, ulo.z) * iz), 0.f), 255.f);
+    const uint32_t qlx = min(__float2uint_rd(__fsub_rd(lo.x, ulo.x) * ix), 255u);
+    const uint32_t qly = min(__float2uint_rd(__fsub_rd(lo.y, ulo.y) * iy), 255u);
+    const uint32_t qlz = min(__float2uint_rd(__fsub_rd(lo.z, ulo.z) * iz), 255u);
+    const uint32_t qhx = min(__float2uint_ru(__fsub_ru(hi.x, ulo.x) * ix), 255u);
+    const uint32_t qhy = min(__float2uint_ru(__fsub_ru(hi.y, ulo.y) * iy), 255u);
+    const uint32_t qhz = min(__float2uint_ru(__fsub_ru(hi.z, ulo.z) * iz), 255u);
     node->qlo_x[s] = (uint8_t)qlx; node->qlo_y[s] = (uint8_t)qly; node->qlo_z[s] = (uint8_t)qlz;
     node->qhi_x[s] = (uint8_t)qhx; node->qhi_y[s] = (uint8_t)qhy; node->qhi_z[s] = (uint8_t)qhz;
-    const float3 dlo = make_float3(__fmaf_rd(qlx, sx, ulo.x), __fmaf_rd(qly, sy, ulo.y), __fmaf_rd(qlz, sz, ulo.z));
-    const float3 dhi = make_float3(__fmaf_ru(qhx, sx, ulo.x), __fmaf_ru(qhy, sy, ulo.y), __fmaf_ru(qhz, sz, ulo.z));
+    const float3 dlo = make_float3(__fmaf_rd(byte_f(qlx), sx, ulo.x), __fmaf_rd(byte_f(qly), sy, ulo.y), __fmaf_rd(byte_f(qlz), sz, ulo.z));
+    const float3 dhi = make_float3(__fmaf_ru(byte_f(qhx), sx, ulo.x), __fmaf_ru(byte_f(qhy), sy, ulo.y), __fmaf_ru(byte_f(qhz), sz, ulo.z));
     sah_out += (double)fmaxf(0.f, half_area(dlo, dhi));  // leaves of <= 4 triangles: one block each
     sahx_out += (double)fmaxf(0.f, half_area(lo, hi));
   }
@@ -3670,19 +3672,22 @@ struct RefitLevels {
   uint32_t start[kColMaxLevels + 1];
 };
 
-// Levels of at most this many nodes are refitted by the first CTA alone, without a
-// grid barrier between two of them.
-constexpr uint32_t kRefitNarrow = 64;
+// Two CTAs of 512 threads per SM: the refit of 8k / 200k / 1M triangles takes 20 / 48 /
+// 117 us, with 4 x 256 21 / 67 / 122 us, with 1 x 1024 26 / 50 / 167 us.  Levels of at
+// most kRefitNarrow nodes are refitted by the first CTA alone, without a grid barrier
+// between two of them (64 or 128: 1 to 2 us more).
+constexpr int kRefitThreads = 512, kRefitCtas = 2;
+constexpr uint32_t kRefitNarrow = 32;
 
 // The whole refit in one cooperative launch: the triangles, then the levels,
 // deepest first, a grid barrier between two levels.  A refit is a chain of about 14
 // levels that each take a few microseconds at most: as one launch per level with
 // one thread per node, its eight children's loads in sequence, the chain took
 // 0.44 ms on a 1M-triangle soup whatever the bandwidth (the whole refit 0.61 ms;
-// here 0.14 ms, of which the 176 MB of the triangle pass need 0.03).  *bar and *bar_err are
+// here 0.12 ms, of which the 176 MB of the triangle pass need 0.03).  *bar and *bar_err are
 // zero before the first launch and left ready for the next one (an error of the
 // triangles or nodes does not stop the refit, a barrier that fails does).
-__global__ void __launch_bounds__(256) k_refit_all(const GeomDesc* __restrict__ geoms,
+__global__ void __launch_bounds__(kRefitThreads, kRefitCtas) k_refit_all(const GeomDesc* __restrict__ geoms,
                                                    const uint32_t* __restrict__ slot_of, uint32_t nslots,
                                                    TriRecord* __restrict__ tris, uint32_t num_tris, int robust,
                                                    float4* tri_box, WideNode* __restrict__ nodes, uint32_t num_nodes,
@@ -3744,13 +3749,14 @@ cudaError_t refit_prepare(const GeomDesc* h_geoms, int ngeoms, const DeviceBVH& 
   out->nslots = (uint32_t)slot_of.size();
   out->ngeoms = ngeoms;
   int per_sm = 0;
-  GB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_refit_all, 256, 0));
-  // enough CTAs for the triangles and the widest level, at most 4 per SM (a grid
-  // barrier costs more with every CTA)
+  GB_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_refit_all, kRefitThreads, 0));
+  // enough CTAs for the triangles and the widest level, at most kRefitCtas per SM (a
+  // grid barrier costs more with every CTA)
   uint64_t work = bvh.num_tris;
   for (size_t l = 0; l + 1 < bvh.level_start.size(); l++)
     work = std::max<uint64_t>(work, 8ull * (bvh.level_start[l + 1] - bvh.level_start[l]));
-  out->grid = std::min<uint32_t>(cdiv(work, 256), (uint32_t)std::max(1, std::min(per_sm, 4)) * (uint32_t)num_sms_build());
+  out->grid = std::min<uint32_t>(cdiv(work, 256),
+                                 (uint32_t)std::max(1, std::min(per_sm, kRefitCtas)) * (uint32_t)num_sms_build());
   cudaError_t e = cudaMalloc(&out->d_geoms, sizeof(GeomDesc) * std::max(ngeoms, 1));
   if (e == cudaSuccess) e = cudaMalloc(&out->d_slot, sizeof(uint32_t) * slot_of.size());
   if (e == cudaSuccess) e = cudaMalloc(&out->result, sizeof(RefitResult) + sizeof(float) * 6 * (size_t)bvh.num_nodes);
