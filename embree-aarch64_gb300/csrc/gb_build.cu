@@ -1349,6 +1349,9 @@ __global__ void __launch_bounds__(PLOC_BLOCK) k_ploc_all(const PlocBufs bufs, ui
 
 // Area of the box around clusters j and j + 1; infinite where they are no
 // neighbours (the ends, another segment).
+// The line of p into L2, for a read of the loop's next turn.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ float ploc_adjacent(const float4* clo, const float4* chi, uint32_t n, int j) {
   if (j < 0 || j + 1 >= (int)n) return INFINITY;
   const float4 a = clo[j], b = chi[j], c = clo[j + 1], d = chi[j + 1];
@@ -1437,7 +1440,9 @@ __device__ __forceinline__ bool grid_sums(uint2* __restrict__ words, uint32_t a,
 // round ends at two grid barriers, and 152 CTAs arrive sooner and read fewer sums
 // than 608 of 256 threads.  Rounds of 8k / 300k / 1M / 4M triangles: 23 / 105 / 190 /
 // 527 us, with 4 x 256 threads per SM 27 / 129 / 216 / 563, with 2 x 512 23 / 110 /
-// 196 / 534 (tile per CTA: 732 us at 4M).
+// 196 / 534 (tile per CTA: 732 us at 4M).  What does not fit L2 waits for memory with
+// 32 warps per SM: prefetching each warp's next tile makes it 501 us at 4M (two tiles
+// ahead 508, four 517; collapse costs by full warps of merges 576).
 constexpr int PLOC1_THREADS = 1024, PLOC1_CTAS = 1;
 __global__ void __launch_bounds__(PLOC1_THREADS, PLOC1_CTAS)
     k_ploc_rounds1(const PlocBufs bufs, uint32_t* __restrict__ ploc_state, uint32_t* tile_m, uint32_t* tile_s,
@@ -1459,6 +1464,10 @@ __global__ void __launch_bounds__(PLOC1_THREADS, PLOC1_CTAS)
     // (1) merges of the run's tiles
     for (uint32_t t = t0 + warp; t < t1; t += kWarps) {
       const int i = (int)(32u * t + lane);
+      if (const uint32_t p = 32u * (t + kWarps) + lane; t + kWarps < t1 && p < n) {  // the next tile's
+        prefetch_l2(clo + p);
+        prefetch_l2(chi + p);
+      }
       const float a = ploc_adjacent(clo, chi, n, i);
       const float edge = lane < 2u ? ploc_adjacent(clo, chi, n, lane ? (int)(32u * t) + 32 : (int)(32u * t) - 1) : 0.f;
       float left = __shfl_up_sync(0xFFFFFFFFu, a, 1), right = __shfl_down_sync(0xFFFFFFFFu, a, 1);
@@ -1498,6 +1507,11 @@ __global__ void __launch_bounds__(PLOC1_THREADS, PLOC1_CTAS)
     uint4 v;
     if (!grid_sums<PLOC1_THREADS>(cta_sums, ps, pm, v, bar, err)) break;
     for (uint32_t t = t0 + warp; t < t1; t += kWarps) {
+      if (const uint32_t p = 32u * (t + kWarps) + lane; t + kWarps < t1 && p < n) {
+        prefetch_l2(clo + p);
+        prefetch_l2(chi + p);
+        prefetch_l2(bufs.cidx[par] + p);
+      }
       const uint32_t m = tile_m[t], i = 32u * t + lane, carry = t > t0 ? tile_m[t - 1] >> 31 : before;
       const uint32_t s0 = tile_s[t], m0 = tile_p[t];
       const uint32_t in = min(n - 32u * t, 32u), absorbed = (m << 1) | carry;
@@ -2247,7 +2261,8 @@ struct EmitSmem {
 
 // The wide node of item k, built by the 8 lanes of a lane group (lane & 7 is the
 // child index; all 32 lanes call it, `have` is the group's; g: the group's index in
-// the CTA).  Children are placed in slots greedily, the cheapest (child, free slot)
+// the CTA; k_next: the item the group takes next, or 0xFFFFFFFF: its children's boxes
+// are prefetched, 13 of 578 us at 4M triangles).  Children are placed in slots greedily, the cheapest (child, free slot)
 // pair first with ties to the lower child and then the lower slot, the cost being
 // the child's offset from the node centre along the slot's octant direction (slot s
 // prefers children far along the direction with sign bits s), so that visiting
@@ -2264,7 +2279,7 @@ struct EmitSmem {
 template <int GROUPS>
 __device__ __forceinline__ void collapse_emit_group(
     const BinTree& t, const uint32_t* __restrict__ kids_in, uint32_t k, bool have, uint32_t g, EmitSmem<GROUPS>& sm,
-    const uint32_t* __restrict__ off_int, const uint32_t* __restrict__ off_tri, uint2 off, uint32_t level_base,
+    const uint32_t* __restrict__ off_int, const uint32_t* __restrict__ off_tri, uint2 off, uint32_t k_next, uint32_t level_base,
     uint32_t next_base, uint32_t tri_next, WideNode* __restrict__ nodes, uint32_t* __restrict__ leaf_root,
     uint32_t* __restrict__ next_items, uint32_t node_cap, uint32_t tri_cap, uint32_t* err, double& sah_out,
     double& sahx_out, uint32_t& nleaf_out) {
@@ -2281,6 +2296,7 @@ __device__ __forceinline__ void collapse_emit_group(
   }
   uint32_t cnt = valid ? bt_cnt(t, kid) : 0u;
   const uint32_t oi = have ? off.x + off_int[k] : 0u, ot = have ? off.y + off_tri[k] : 0u;
+  const uint32_t kid_next = k_next != 0xFFFFFFFFu ? kids_in[8 * (size_t)k_next + i] : 0xFFFFFFFFu;
   // union box and quantisation frame
   float3 ulo = valid ? lo : make_float3(INFINITY, INFINITY, INFINITY);
   float3 uhi = valid ? hi : make_float3(-INFINITY, -INFINITY, -INFINITY);
@@ -2358,6 +2374,7 @@ __device__ __forceinline__ void collapse_emit_group(
     }
   }
   const uint32_t slot = valid ? order & 7u : 8u;
+  if (kid_next != 0xFFFFFFFFu) prefetch_l2(t.box + 2 * (size_t)kid_next);
   // this child's planes, its part of the SAH, its place among the slots
   const bool inner = cnt > t.leaf_max;
   uint32_t places = valid ? (inner ? 8u : cnt) << (4u * slot) : 0u;  // 4 bits per slot: triangles, bit 3 an internal child
@@ -2445,7 +2462,7 @@ __global__ void __launch_bounds__(COLLAPSE_THREADS) k_collapse_emit(
   __shared__ EmitSmem<COLLAPSE_THREADS / 8> sm;
   for (uint32_t k0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 3; k0 < nitems; k0 += (gridDim.x * blockDim.x) >> 3) {
     const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
-    collapse_emit_group(t, kids_in, k, k < nitems, threadIdx.x >> 3, sm, off_int, off_tri, make_uint2(0u, 0u), level_base, next_base, tri_next,
+    collapse_emit_group(t, kids_in, k, k < nitems, threadIdx.x >> 3, sm, off_int, off_tri, make_uint2(0u, 0u), 0xFFFFFFFFu, level_base, next_base, tri_next,
                         nodes, leaf_root, next_items, node_cap, tri_cap, err, sah, sahx, nleaf);
   }
   nleaf = __reduce_add_sync(0xFFFFFFFFu, nleaf);
@@ -2540,8 +2557,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_collapse_all(
     // (3) the wide nodes of this CTA's items, one per 8-lane group
     for (uint32_t k0 = first + ((threadIdx.x & ~31u) >> 3); k0 < last; k0 += blockDim.x >> 3) {
       const uint32_t k = k0 + ((threadIdx.x & 31u) >> 3);
-      collapse_emit_group(t, kids, k, k < last, threadIdx.x >> 3, sm, nint, ntri, make_uint2(sums.x, sums.y), base, base + nitems, tri_next, nodes,
-                          leaf_root, next_items, node_cap, tri_cap, err, sah, sahx, nleaf);
+      const uint32_t k_next = k + (blockDim.x >> 3);
+      collapse_emit_group(t, kids, k, k < last, threadIdx.x >> 3, sm, nint, ntri, make_uint2(sums.x, sums.y),
+                          k_next < last ? k_next : 0xFFFFFFFFu, base, base + nitems, tri_next, nodes, leaf_root,
+                          next_items, node_cap, tri_cap, err, sah, sahx, nleaf);
     }
     // (4) the next level, alike in every CTA
     if (blockIdx.x == 0 && threadIdx.x == 0 && depth < (uint32_t)kColMaxLevels) cstate[kColLevels + depth] = base;
