@@ -16,7 +16,7 @@ struct TraceShapeDesc {
 inline constexpr TraceShapeDesc kTraceShapes[] = {
     {128, 9, 8, 4},   // default
     {128, 8, 8, 4},   // 64 registers a thread
-    {128, 9, 16, 4},  // deeper shared stack
+    {128, 9, 12, 4},  // deeper shared stack (16 entries leave 28 KB of L1: twice the time)
     {128, 9, 4, 4},   // shallower shared stack
     {64, 18, 8, 4},   // two-warp CTAs
     {256, 4, 8, 4},   // eight-warp CTAs, 64 registers
