@@ -39,7 +39,7 @@ import numpy as np  # noqa: E402
 METRIC = "Mrays/s closest/shadow, learned vs plain GPU, exact hits; build Mtris/s"
 RAY_BYTES_CLOSEST = 84   # read 48 B RTCRay, write 4 B tfar + 32 B RTCHit
 RAY_BYTES_SHADOW = 52    # read 48 B RTCRay, write 4 B tfar
-NODE_BYTES = 80
+NODE_BYTES = 80          # the record of a node; the traversal's nodes are padded to 96 B
 TRI_BYTES = 48
 
 
@@ -299,7 +299,11 @@ def run_reference(args, rank, world):
 # GPU arm
 # ---------------------------------------------------------------------------
 
-MLP_FLOPS_PER_RAY = 2 * (32 * 64 + 64 * 64 + 64 * 64 + 64 * 4096)  # forward pass of the proposer
+
+
+def mlp_flops_per_ray(treelets):
+    """Forward pass of the proposer: its outputs come in chunks of 128 treelets."""
+    return 2 * (32 * 64 + 64 * 64 + 64 * 64 + 64 * 128 * ((treelets + 127) // 128))
 
 
 def run_learned(api, dev, torch, stream, scale, steps, warmup, cpu_seconds):
@@ -411,7 +415,7 @@ def run_learned(api, dev, torch, stream, scale, steps, warmup, cpu_seconds):
                      "learned_Mrays_per_s": n / (ms_learn * 1e-3) / 1e6, "speedup": ms_plain / ms_learn,
                      "mismatches": mism, "answered_by_proposal": int(q["proposal_hits"]),
                      "hits_or_occluded": answered, "inference_ms": inf_ms,
-                     "mlp_TFLOPs": MLP_FLOPS_PER_RAY * n / (inf_ms * 1e-3) / 1e12}
+                     "mlp_TFLOPs": mlp_flops_per_ray(prop.stats()["num_treelets"]) * n / (inf_ms * 1e-3) / 1e12}
         total_plain += ms_plain
         total_learned += ms_learn
         del pristine, w_plain, w_learn, treelets
