@@ -418,14 +418,16 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
   // j ^ o (one shared-memory byte load per node instead of a three-stage swap
   // network: 1.4 % faster; the reversed order lets one count of leading zeros
   // find the next child: 0.5 %)
-  __shared__ uint8_t s_perm[8][256];
-  for (int i = threadIdx.x; i < 8 * 256; i += SH::kThreads) {
-    const uint32_t o = i >> 8;
-    uint32_t v = i & 255;  // bit j ^ o of the slot mask moves to bit j: swaps of 1, 2 and 4 bits
-    if (o & 1u) v = ((v & 0x55u) << 1) | ((v >> 1) & 0x55u);
-    if (o & 2u) v = ((v & 0x33u) << 2) | ((v >> 2) & 0x33u);
-    if (o & 4u) v = ((v & 0x0Fu) << 4) | (v >> 4);
-    s_perm[o][i & 255] = (uint8_t)(__brev(v) >> 24);
+  alignas(4) __shared__ uint8_t s_perm[8][256];
+  // four entries at a time (one by one, the filling took 1.5 us of a 1,000-ray query's 28)
+  for (int i = threadIdx.x; i < 8 * 64; i += SH::kThreads) {
+    const uint32_t o = i >> 6;
+    // bit j ^ o of the slot mask moves to bit j: swaps of 1, 2 and 4 bits of each byte
+    uint32_t v = 0x03020100u + 0x04040404u * (i & 63u);
+    if (o & 1u) v = ((v & 0x55555555u) << 1) | ((v >> 1) & 0x55555555u);
+    if (o & 2u) v = ((v & 0x33333333u) << 2) | ((v >> 2) & 0x33333333u);
+    if (o & 4u) v = ((v & 0x0F0F0F0Fu) << 4) | ((v >> 4) & 0x0F0F0F0Fu);
+    reinterpret_cast<uint32_t*>(s_perm)[i] = __byte_perm(__brev(v), 0u, 0x0123u);
   }
   s_tri[threadIdx.x] = kInvalidID;  // no result to write yet
   __shared__ uint32_t s_batch[kWarps];  // batched queries: a batch that a ray of this warp was in
