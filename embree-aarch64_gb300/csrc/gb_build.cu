@@ -860,17 +860,10 @@ __device__ __forceinline__ void dp_child_costs(const float4* cost, uint32_t c, u
   out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w; out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
 }
 
-// cost(n, 1..8) and the choices of binary node n with children l and r (cnt_l,
-// cnt_r triangles; a child of one triangle is a primitive, whose area Al / Ar
-// the caller passes); A is n's box area.  The PLOC kernels call it as they
-// create each node, so the table is complete when the clustering ends
-// (children are always created before their parent).
-__device__ __forceinline__ void dp_node(float4* cost, uint4* link, uint32_t n, uint32_t l, uint32_t r, float A,
-                                        uint32_t cnt_l, uint32_t cnt_r, float Al, float Ar, uint32_t leaf_max) {
-  const uint32_t cnt = cnt_l + cnt_r;
-  float cl[8], cr[8];
-  dp_child_costs(cost, l, cnt_l, Al, cl);
-  dp_child_costs(cost, r, cnt_r, Ar, cr);
+// cost(n, 1..8) into c and the tables, and the choices of n, from its children's costs.
+__device__ __forceinline__ void dp_combine(float4* cost, uint4* link, uint32_t n, uint32_t l, uint32_t r, float A,
+                                           uint32_t cnt, const float (&cl)[8], const float (&cr)[8], uint32_t leaf_max,
+                                           float (&c)[8]) {
   float D[9];
   uint32_t K[9];
 #pragma unroll
@@ -888,7 +881,6 @@ __device__ __forceinline__ void dp_node(float4* cost, uint4* link, uint32_t n, u
   }
   const float c_int = A + D[8];
   const float c_leaf = cnt <= leaf_max ? A * (float)((cnt + 3) / 4) : INFINITY;
-  float c[8];
   c[0] = fminf(c_leaf, c_int);
   uint32_t b[8];
   b[0] = K[8];
@@ -902,6 +894,18 @@ __device__ __forceinline__ void dp_node(float4* cost, uint4* link, uint32_t n, u
            make_uint4(l, r, b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24), b[4] | (b[5] << 8) | (b[6] << 16) | (b[7] << 24)));
 }
 
+// cost(n, 1..8) and the choices of binary node n with children l and r (cnt_l,
+// cnt_r triangles; a child of one triangle is a primitive, whose area Al / Ar
+// the caller passes); A is n's box area.  The PLOC kernels call it as they
+// create each node, so the table is complete when the clustering ends
+// (children are always created before their parent).
+__device__ __forceinline__ void dp_node(float4* cost, uint4* link, uint32_t n, uint32_t l, uint32_t r, float A,
+                                        uint32_t cnt_l, uint32_t cnt_r, float Al, float Ar, uint32_t leaf_max) {
+  float cl[8], cr[8], c[8];
+  dp_child_costs(cost, l, cnt_l, Al, cl);
+  dp_child_costs(cost, r, cnt_r, Ar, cr);
+  dp_combine(cost, link, n, l, r, A, cnt_l + cnt_r, cl, cr, leaf_max, c);
+}
 
 // Grid barrier of the cooperative build kernels (all CTAs resident).
 struct GridBarrier {
@@ -1724,8 +1728,9 @@ __global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_small(const float4*
 // adjacent areas (k_ploc_rounds1).  A round of one CTA is a chain of steps between
 // barriers, so the new nodes' collapse costs -- two dependent L2 reads and 28
 // sums, the longest step -- are left to the next round, which reads them while it
-// works on its own areas and merges.  The last 4,096 clusters of the 4M soup:
-// 174 us with the costs inside the round, 90 us so.
+// works on its own areas and merges, and the last 32 clusters to one warp
+// (ploc_last).  The last 4,096 clusters of the 4M soup: 174 us with the costs inside
+// the round, 96 us so, 88 us with the last warp; 4,096 of 8k triangles 44 and 35 us.
 struct PlocTask {       // costs to compute: node task_base + index
   uint32_t l, r;        // children
   float A, Al, Ar;      // areas (Al, Ar: of primitive children)
@@ -1733,6 +1738,85 @@ struct PlocTask {       // costs to compute: node task_base + index
 };
 constexpr size_t kPlocFinishSmem = (size_t)PLOC_SMALL * (2 * sizeof(float3) + 3 * sizeof(uint32_t)) +
                                    (PLOC_SMALL + 2) * sizeof(float) + (PLOC_SMALL / 2) * sizeof(PlocTask);
+
+// The last 32 clusters, by one warp: a cluster per lane with its collapse costs, a
+// round in registers and shuffles instead of four CTA barriers (8 us less for the ten
+// rounds or so).
+struct PlocLast {
+  uint32_t n, node_next, iters;
+  uint8_t src[32];  // lane of each survivor
+};
+__device__ __noinline__ void ploc_last(float3* s_lo, float3* s_hi, uint32_t* s_idx, uint32_t* s_seg, uint32_t* s_cnt,
+                                       PlocLast& st, float4* __restrict__ bnbox, uint32_t* __restrict__ bncnt,
+                                       uint32_t node_cap, uint32_t* err, float4* __restrict__ dp_cost,
+                                       uint4* __restrict__ dp_link, uint32_t leaf_max) {
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  uint32_t n = st.n, node_next = st.node_next, iters = st.iters;
+  float3 lo = s_lo[lane], hi = s_hi[lane];  // of lanes past n: not used
+  uint32_t id = s_idx[lane], seg = s_seg[lane], cnt = s_cnt[lane];
+  float c[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (dp_cost && lane < n) dp_child_costs(dp_cost, id, cnt, half_area(lo, hi), c);
+  while (n > 1) {
+    iters++;
+    const float3 rlo = make_float3(__shfl_down_sync(0xFFFFFFFFu, lo.x, 1), __shfl_down_sync(0xFFFFFFFFu, lo.y, 1),
+                                   __shfl_down_sync(0xFFFFFFFFu, lo.z, 1));
+    const float3 rhi = make_float3(__shfl_down_sync(0xFFFFFFFFu, hi.x, 1), __shfl_down_sync(0xFFFFFFFFu, hi.y, 1),
+                                   __shfl_down_sync(0xFFFFFFFFu, hi.z, 1));
+    const uint32_t rid = __shfl_down_sync(0xFFFFFFFFu, id, 1), rcnt = __shfl_down_sync(0xFFFFFFFFu, cnt, 1);
+    const uint32_t rseg = __shfl_down_sync(0xFFFFFFFFu, seg, 1);
+    const float3 ulo = f3min(lo, rlo), uhi = f3max(hi, rhi);
+    const float a = lane + 1u < n && seg == rseg ? half_area(ulo, uhi) : INFINITY;
+    float left = __shfl_up_sync(0xFFFFFFFFu, a, 1), right = __shfl_down_sync(0xFFFFFFFFu, a, 1);
+    if (lane == 0u) left = INFINITY;
+    if (lane == 31u) right = INFINITY;
+    const bool merge = a != INFINITY && a < left && a <= right;
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, merge);
+    if (m == 0u) break;
+    if (node_next + __popc(m) > node_cap) {
+      if (lane == 0u) atomicOr(err, kErrBuild);
+      break;
+    }
+    float cr[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) cr[i] = __shfl_down_sync(0xFFFFFFFFu, c[i], 1);
+    if (merge) {
+      const uint32_t nid = node_next + __popc(m & lt);
+      bnbox[2 * (size_t)nid] = make_float4(ulo.x, ulo.y, ulo.z, __uint_as_float(id));
+      bnbox[2 * (size_t)nid + 1] = make_float4(uhi.x, uhi.y, uhi.z, __uint_as_float(rid));
+      lo = ulo;
+      hi = uhi;
+      cnt += rcnt;
+      bncnt[nid] = cnt;
+      if (dp_cost) {
+        float cn[8];
+        dp_combine(dp_cost, dp_link, nid, id, rid, a, cnt, c, cr, leaf_max, cn);
+#pragma unroll
+        for (int i = 0; i < 8; i++) c[i] = cn[i];
+      }
+      id = nid;
+    }
+    // the survivors move up
+    const uint32_t alive = (n == 32u ? 0xFFFFFFFFu : (1u << n) - 1u) & ~(m << 1);
+    if (alive >> lane & 1u) st.src[__popc(alive & lt)] = (uint8_t)lane;
+    __syncwarp();
+    node_next += __popc(m);
+    n = __popc(alive);
+    const int src = lane < n ? st.src[lane] : 31;
+    lo = make_float3(__shfl_sync(0xFFFFFFFFu, lo.x, src), __shfl_sync(0xFFFFFFFFu, lo.y, src), __shfl_sync(0xFFFFFFFFu, lo.z, src));
+    hi = make_float3(__shfl_sync(0xFFFFFFFFu, hi.x, src), __shfl_sync(0xFFFFFFFFu, hi.y, src), __shfl_sync(0xFFFFFFFFu, hi.z, src));
+    id = __shfl_sync(0xFFFFFFFFu, id, src);
+    seg = __shfl_sync(0xFFFFFFFFu, seg, src);
+    cnt = __shfl_sync(0xFFFFFFFFu, cnt, src);
+#pragma unroll
+    for (int i = 0; i < 8; i++) c[i] = __shfl_sync(0xFFFFFFFFu, c[i], src);
+    __syncwarp();  // st.src is written again
+  }
+  if (lane < n) {
+    s_idx[lane] = id;
+    s_seg[lane] = seg;
+  }
+  if (lane == 0u) st.n = n, st.node_next = node_next, st.iters = iters;
+}
 
 __global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_finish1(const PlocBufs bufs, uint32_t* __restrict__ ploc_state,
                                                                      float4* __restrict__ bnbox,
@@ -1776,7 +1860,8 @@ __global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_finish1(const PlocB
   // every round merges at least the closest pair of each segment that still
   // has two clusters, so n0 - 1 rounds always suffice; the bound only guards
   // against a logic error.  A round without merges ends the clustering.
-  while (n > 1 && !failed) {
+  bool stalled = false;  // a round merged nothing
+  while (n > 32 && !failed) {
     if (iters >= PLOC_SMALL) {
       if (threadIdx.x == 0) atomicOr(err, kErrBuild);
       break;
@@ -1883,9 +1968,22 @@ __global__ void __launch_bounds__(PLOC_SMALL_THREADS) k_ploc_finish1(const PlocB
     n = total & 0xFFFFu;
     if (!dp_cost) tasks = 0;
     __syncthreads();
-    if ((total >> 16) == 0) break;
+    if ((total >> 16) == 0) {
+      stalled = true;
+      break;
+    }
   }
   for (uint32_t k = threadIdx.x; k < tasks; k += blockDim.x) pay(k);
+  __shared__ PlocLast s_last;
+  if (threadIdx.x == 0) s_last.n = n, s_last.node_next = node_next, s_last.iters = iters;
+  __syncthreads();
+  if (n > 1 && n <= 32 && !failed && !stalled) {
+    if (warp == 0) ploc_last(s_lo, s_hi, s_idx, s_seg, s_cnt, s_last, bnbox, bncnt, node_cap, err, dp_cost, dp_link, leaf_max);
+    __syncthreads();
+    n = s_last.n;
+    node_next = s_last.node_next;
+    iters = s_last.iters;
+  }
   // one root per segment (nseg == 1: the single tree's root)
   for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
     const uint32_t seg = nseg > 1 ? s_seg[k] : 0u;

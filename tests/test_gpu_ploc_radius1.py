@@ -43,7 +43,7 @@ def _commits(rtc, cfg, meshes, batched):
 
 
 @pytest.mark.parametrize("mesh", [_random, _equal, _plane], ids=["random", "equal", "plane"])
-@pytest.mark.parametrize("n", [1, 2, 33, 257, 4095, 4097, 8225, 60_000])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 32, 33, 257, 4095, 4097, 8225, 60_000])
 def test_replayed_tree_equals_host_driven(rtc, mesh, n):
     ref = _commits(rtc, b"gpu.graph_rebuild=0", [mesh(n)], False)
     got = _commits(rtc, b"", [mesh(n)], False)
