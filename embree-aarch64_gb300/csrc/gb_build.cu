@@ -231,15 +231,18 @@ __device__ __forceinline__ uint32_t spread10(uint32_t x) {
 // Morton builder (kernels/builders/bvh_builder_morton.h:62-86, LATTICE_BITS_PER_DIM
 // 10), so valid keys fit in 30 bits (42 with the slot) and the sort needs 4 (6)
 // digit passes instead of 8; invalid primitives get bit 30 (42) set, above every
-// valid key, so they sort after all valid ones.  key32: the 30-bit keys of an
-// unsegmented build are written as 32-bit words (the sort then moves 4-byte keys).
-constexpr uint32_t kMaxSegments = 4096;
+// valid key, so they sort after all valid ones.  With at most kFewSegments slots all
+// keys fit in 40 bits, the invalid ones as 40 set bits (a slot that none has), and the
+// sort needs 5 passes (1.8M triangles of 128 scenes: 139 us, with 6 160).  key32: the
+// 30-bit keys of an unsegmented build are written as 32-bit words (the sort then moves
+// 4-byte keys).  nseg: geometries of a segmented build, else 0.
+constexpr uint32_t kMaxSegments = 4096, kFewSegments = 1023;
 
 // Grid-stride; the AND / OR of all keys (constant digits are not sorted) is
 // reduced per thread, per warp and per CTA: two global atomics per CTA.
 __global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ pbox,
                                                 uint32_t n, BoundsAcc* acc, uint64_t* __restrict__ keys,
-                                                uint32_t* __restrict__ vals, int cube, int segmented, int bits30,
+                                                uint32_t* __restrict__ vals, int cube, uint32_t nseg, int bits30,
                                                 int key32) {
   __shared__ unsigned long long s_and, s_or;
   if (threadIdx.x == 0) {
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ pbox,
   __syncthreads();
   unsigned long long ka = ~0ull, ko = 0ull;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    uint64_t key = bits30 ? (1ull << (segmented ? 42 : 30)) : ~0ull;
+    uint64_t key = !bits30 ? ~0ull : nseg == 0 ? 1ull << 30 : nseg <= kFewSegments ? (1ull << 40) - 1ull : 1ull << 42;
     {
       const float4 a = pbox[2 * (size_t)i], b = pbox[2 * (size_t)i + 1];
       if (a.x <= b.x) {
@@ -274,7 +277,7 @@ __global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ pbox,
             x = fminf(fmaxf(x * 1024.0f, 0.0f), 1023.0f);
             c30 |= spread10((uint32_t)x) << (2 - d);
           }
-          key = segmented ? ((uint64_t)(__float_as_uint(a.w) & (kMaxSegments - 1)) << 30) | c30 : c30;
+          key = nseg ? ((uint64_t)(__float_as_uint(a.w) & (kMaxSegments - 1)) << 30) | c30 : c30;
         } else {
 #pragma unroll
           for (int d = 0; d < 3; d++) {
@@ -283,7 +286,7 @@ __global__ void __launch_bounds__(256) k_morton(const float4* __restrict__ pbox,
             x = fminf(fmaxf(x * 2097152.0f, 0.0f), 2097151.0f);
             code |= spread21((uint32_t)x) << (2 - d);
           }
-          key = segmented ? ((uint64_t)(__float_as_uint(a.w) & (kMaxSegments - 1)) << 51) | (code >> 12) : code;
+          key = nseg ? ((uint64_t)(__float_as_uint(a.w) & (kMaxSegments - 1)) << 51) | (code >> 12) : code;
         }
       }
       if (key32) reinterpret_cast<uint32_t*>(keys)[i] = (uint32_t)key;
@@ -2947,7 +2950,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   if (segmented && (uint32_t)ngeoms > kMaxSegments) return cudaErrorInvalidValue;
   const bool key32 = opt.morton_bits == 30 && !segmented;  // 30-bit keys sorted as 32-bit words
   k_morton<<<grid_stride_blocks(total), 256, 0, st>>>(pbox, total, acc, keys_a, vals_a, opt.morton_cube,
-                                                      segmented ? 1 : 0, opt.morton_bits == 30 ? 1 : 0,
+                                                      segmented ? nseg : 0u, opt.morton_bits == 30 ? 1 : 0,
                                                       key32 ? 1 : 0);
   note_launches(1);
   GB_CHECK(cudaGetLastError());
@@ -3389,15 +3392,18 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
                                                     g.opt.robust ? 1 : 0);
   const bool key32 = g.opt.morton_bits == 30 && !g.opt.segmented;  // 30-bit keys sorted as 32-bit words
   k_morton<<<grid_stride_blocks(T), 256, 0, st>>>(g.pbox, T, acc, g.keys_a, g.vals_a, g.opt.morton_cube,
-                                                  g.opt.segmented ? 1 : 0, g.opt.morton_bits == 30 ? 1 : 0,
+                                                  g.opt.segmented ? g.nseg : 0u, g.opt.morton_bits == 30 ? 1 : 0,
                                                   key32 ? 1 : 0);
   note_launches(3);
   stamp(1);
   // all digits of the key width (the ordinary build skips constant ones: the same order)
   uint64_t *ka = g.keys_a, *kb = g.keys_b;
   uint32_t *va = g.vals_a, *vb = g.vals_b;
-  // the digits the key width can use: 63-bit keys 8, 30-bit keys 4 (6 with the slot)
-  const uint32_t digits = g.opt.morton_bits == 30 ? (g.opt.segmented ? 0x3Fu : 0x0Fu) : 0xFFu;
+  // the digits the key width can use: 63-bit keys 8, 30-bit keys 4 (5 or 6 with the slot)
+  const uint32_t digits = g.opt.morton_bits != 30 ? 0xFFu
+                          : !g.opt.segmented    ? 0x0Fu
+                          : g.nseg <= kFewSegments ? 0x1Fu
+                                                   : 0x3Fu;
   if (key32) {
     uint32_t *ka32 = reinterpret_cast<uint32_t*>(ka), *kb32 = reinterpret_cast<uint32_t*>(kb);
     GB_CHECK(onesweep_sort(ka32, va, kb32, vb, T, digits, g.hist, &acc->pad, st));
