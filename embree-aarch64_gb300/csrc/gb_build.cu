@@ -2782,7 +2782,7 @@ static void scan_excl2(uint32_t* a, uint32_t* b, uint32_t n, uint32_t* ta, uint3
   note_launches(1);
 }
 
-// Scratch words of onesweep_sort for n keys and `passes` digit passes.
+// Scratch words of onesweep_sort for exactly n keys and `passes` digit passes.
 static inline size_t onesweep_scratch_words(uint32_t n, int passes) {
   return kOsStatus + (size_t)passes * cdiv(n, os_tile(n)) * 256u;
 }
@@ -3624,7 +3624,8 @@ cudaError_t sort_pairs_passes(uint64_t* keys, uint32_t* vals, uint64_t* kb, uint
   return onesweep_sort(ka, va, kb, vb, n, (1u << passes) - 1u, hist, nullptr, st);
 }
 
-// onesweep scratch for all 8 digits of n keys
+// onesweep scratch for all 8 digits of exactly n keys (fewer keys in smaller tiles can
+// need more)
 uint32_t sort_hist_entries(uint32_t n) { return (uint32_t)onesweep_scratch_words(n, 8); }
 
 cudaError_t sort_pairs(uint64_t* keys, uint32_t* vals, uint32_t n, cudaStream_t st) {
