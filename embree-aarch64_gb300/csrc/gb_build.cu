@@ -1010,11 +1010,17 @@ struct PlocBufs {
 // The clusters alternate between two buffers, one round reading A and writing
 // B, the next the reverse; kPlocParity counts (mod 2) the rounds that ran, so
 // the current clusters are in B when it is 1 whatever no-op rounds followed.
-// bar, the cooperative rounds' barrier (or null), is zeroed too.
-__global__ void k_ploc_state_init(const BoundsAcc* __restrict__ acc, uint32_t* __restrict__ ploc_state, GridBarrier* bar) {
+// bar, the cooperative rounds' barrier (or null), is zeroed too.  expect: the valid
+// primitives that every array from here on is sized for.  A replayed build whose
+// input has another number of them clusters nothing: without clusters there are no
+// roots, no levels and no leaves, no kernel leaves its arrays (with more primitives
+// than planned the rounds would index past theirs) or takes a merged node for a
+// primitive (ids below `expect`), and k_graph_build_check reports the count.
+__global__ void k_ploc_state_init(const BoundsAcc* __restrict__ acc, uint32_t expect, uint32_t* __restrict__ ploc_state,
+                                  GridBarrier* bar) {
   if (threadIdx.x == 0) {
     if (bar) bar->count = 0;
-    const uint32_t n = acc->nvalid;
+    const uint32_t n = acc->nvalid == expect ? expect : 0u;
     ploc_state[kPlocN] = n;
     ploc_state[kPlocNext] = n;  // binary leaves are the primitives 0..n-1
     ploc_state[kPlocRounds] = 0;
@@ -3046,7 +3052,7 @@ cudaError_t build_bvh(const GeomDesc* h_geoms, int ngeoms, cudaStream_t st, cons
   GB_CHECK(arena.alloc(&ploc_state, kPlocStateWords));
   uint32_t* h_tot = nullptr;
   GB_CHECK(arena.host(&h_tot, kPlocStateWords));
-  k_ploc_state_init<<<1, 32, 0, st>>>(acc, ploc_state, nullptr);
+  k_ploc_state_init<<<1, 32, 0, st>>>(acc, N, ploc_state, nullptr);
   note_launches(1);
   const int radius = opt.ploc_radius == 1 || opt.ploc_radius == 2 || opt.ploc_radius == 4 || opt.ploc_radius == 8
                          ? opt.ploc_radius
@@ -3421,7 +3427,7 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
   k_ploc_init<<<cdiv(N, 256), 256, 0, st>>>(g.pbox, va, N, &acc->nvalid, g.bnbox, g.cidx[0],
                                             g.clo[0], g.chi[0], g.opt.segmented ? 1 : 0);
   stamp(3);
-  k_ploc_state_init<<<1, 32, 0, st>>>(acc, g.ploc_state, reinterpret_cast<GridBarrier*>(g.ploc_bar));
+  k_ploc_state_init<<<1, 32, 0, st>>>(acc, N, g.ploc_state, reinterpret_cast<GridBarrier*>(g.ploc_bar));
   note_launches(2);
   const uint32_t nbin_cap = 2 * N;
   const PlocBufs pb{{g.clo[0], g.clo[1]}, {g.chi[0], g.chi[1]}, {g.cidx[0], g.cidx[1]}};
