@@ -3802,11 +3802,14 @@ struct RefitLevels {
   uint32_t start[kColMaxLevels + 1];
 };
 
-// Two CTAs of 512 threads per SM: the refit of 8k / 200k / 1M triangles takes 20 / 48 /
-// 117 us, with 4 x 256 21 / 67 / 122 us, with 1 x 1024 26 / 50 / 167 us.  Levels of at
-// most kRefitNarrow nodes are refitted by the first CTA alone, without a grid barrier
-// between two of them (64 or 128: 1 to 2 us more).
-constexpr int kRefitThreads = 512, kRefitCtas = 2;
+// Two CTAs of 256 threads per SM: the refit of a soup of 8k / 60k / 200k / 500k / 1M
+// triangles takes 25 / 36 / 48 / 71 / 117 us, with 2 x 512 28 / 36 / 55 / 75 / 109, with
+// 3 x 256 25 / 36 / 55 / 78 / 115, with 4 x 256 25 / 36 / 64 / 87 / 123, with 1 x 512
+// 28 / 36 / 48 / 72 / 117 and with 1 x 1024 36 / 47 / 58 / 79 / 113 us: a chain of levels
+// waits for all CTAs and warps at each barrier, and only the largest trees have work
+// for more of them.  Levels of at most kRefitNarrow nodes are refitted by the first CTA
+// alone, without a grid barrier between two of them (64 or 128: 1 to 2 us more).
+constexpr int kRefitThreads = 256, kRefitCtas = 2;
 constexpr uint32_t kRefitNarrow = 32;
 
 // The whole refit in one cooperative launch: the triangles, then the levels,
@@ -3885,7 +3888,7 @@ cudaError_t refit_prepare(const GeomDesc* h_geoms, int ngeoms, const DeviceBVH& 
   uint64_t work = bvh.num_tris;
   for (size_t l = 0; l + 1 < bvh.level_start.size(); l++)
     work = std::max<uint64_t>(work, 8ull * (bvh.level_start[l + 1] - bvh.level_start[l]));
-  out->grid = std::min<uint32_t>(cdiv(work, 256),
+  out->grid = std::min<uint32_t>(cdiv(work, kRefitThreads),
                                  (uint32_t)std::max(1, std::min(per_sm, kRefitCtas)) * (uint32_t)num_sms_build());
   cudaError_t e = cudaMalloc(&out->d_geoms, sizeof(GeomDesc) * std::max(ngeoms, 1));
   if (e == cudaSuccess) e = cudaMalloc(&out->d_slot, sizeof(uint32_t) * slot_of.size());
@@ -3914,7 +3917,7 @@ cudaError_t refit_enqueue(const DeviceBVH& bvh, const RefitScratch& s, cudaStrea
     std::copy(bvh.level_start.begin(), bvh.level_start.end(), lv.start);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(s.grid);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(kRefitThreads);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
