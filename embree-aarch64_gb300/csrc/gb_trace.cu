@@ -12,17 +12,19 @@
 
 namespace gb {
 
-constexpr uint32_t kFewInstRays = 1u << 19;
+constexpr uint32_t kFewInstRays = 3u << 18;
 using FewRaysShape = Shape<128, 5, 8, 4>;
 
 template <bool ANYHIT, bool COUNT, bool ALIGNED, bool ROBUST, bool SEEDED = false, bool INST = false,
           bool EXCL = false>
 static cudaError_t launch_one(const TraceParams& P, cudaStream_t st) {
   // Scenes with instances: few rays leave lanes without work whatever the occupancy, and
-  // five CTAs per SM with 102 registers trace them sooner than eight with 64 (30k / 100k /
-  // 300k rays on 125 or 10 instances 147 / 160 / 220 us against 153 / 165 / 226); with
-  // more rays than lanes several times over the eight are faster (1M rays 780 against
-  // 867 us).
+  // five CTAs per SM with 92 registers trace them sooner than eight with 63 (kernel,
+  // 125 instances of 50k triangles: 300k / 524k / 700k / 1M rays 321 / 427 / 519 / 709
+  // us against 365 / 464 / 519 / 670; 60 of 20k: 420k / 620k / 850k 229 / 286 / 361
+  // against 252 / 301 / 355; 30 of 10k: 100k / 524k / 700k / 1M 125 / 163 / 180 / 230
+  // against 132 / 191 / 211 / 244).  The two cross between 700k and 850k rays, or above
+  // where the instances are few and small.
   if constexpr (INST && !COUNT)
     if (P.nrays <= kFewInstRays) return launch_shaped<ANYHIT, COUNT, ALIGNED, ROBUST, SEEDED, INST, EXCL, FewRaysShape>(P, st);
   return launch_shaped<ANYHIT, COUNT, ALIGNED, ROBUST, SEEDED, INST, EXCL, DefaultShape>(P, st);
