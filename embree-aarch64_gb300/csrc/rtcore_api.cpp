@@ -1064,7 +1064,7 @@ void run_query(Scene* scene, void* rays, unsigned M, size_t stride, bool anyhit,
   P.ray_counter = c.dscratch;
   P.err = c.dscratch + 1;
   P.counters = reinterpret_cast<gb::TraceCounters*>(c.dscratch + 2);
-  P.max_iters = 4 * bvh.num_nodes + 64;  // node visits, triangle phases and pops per ray
+  P.max_iters = 4 * bvh.num_nodes + 64;  // node visits per ray
   if (scene->ninsts) {
     P.insts = scene->d_insts;
     P.ninsts = scene->ninsts;
@@ -1074,6 +1074,11 @@ void run_query(Scene* scene, void* rays, unsigned M, size_t stride, bool anyhit,
   P.num_tris = bvh.num_tris;
   P.robust = bvh.robust;
   P.shape = scene->trace_shape.load(std::memory_order_relaxed);
+  // device rays and host rays traced in place: the kernel itself reports its state
+  // and leaves the scratch zero, so the call is one launch between two events (e1, e2),
+  // and its time the kernel's unless something is enqueued before it (from e0)
+  const bool reports = on_device || direct;
+  const bool timed_from_e0 = !reports || batch || !c.scratch_zero;
   // batched: the batch boundaries on the device, validated on the host
   std::unique_ptr<uint32_t, void (*)(uint32_t*)> d_start(nullptr, [](uint32_t* p) { if (p) cudaFree(p); });
   if (batch) {
@@ -1087,15 +1092,13 @@ void run_query(Scene* scene, void* rays, unsigned M, size_t stride, bool anyhit,
     uint32_t* p = nullptr;
     cuda_ok(cudaMalloc((void**)&p, hs.size() * sizeof(uint32_t)), "cudaMalloc batches");
     d_start.reset(p);
+    cuda_ok(cudaEventRecord(c.e0, st), "event");
     cuda_ok(cudaMemcpyAsync(p, hs.data(), hs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st), "batches");
     P.batch_start = p;
     P.batch_root = scene->d_roots;
     P.nbatches = batch->nbatches;
   }
-  // device rays and host rays traced in place: the kernel itself reports its state
-  // and leaves the scratch zero, so the call is one launch between two events
-  const bool reports = on_device || direct;
-  if (!reports) cuda_ok(cudaEventRecord(c.e0, st), "event");
+  if (timed_from_e0 && !batch) cuda_ok(cudaEventRecord(c.e0, st), "event");
   unsigned launches = 0;
   if (!reports || !c.scratch_zero) {
     cuda_ok(cudaMemsetAsync(c.dscratch, 0, 64, st), "memset");
@@ -1204,8 +1207,8 @@ void run_query(Scene* scene, void* rays, unsigned M, size_t stride, bool anyhit,
   c.scratch_zero = reports;
   float k_ms = 0, t_ms = 0;
   cudaEventElapsedTime(&k_ms, c.e1, c.e2);
-  if (reports) t_ms = k_ms;
-  else cudaEventElapsedTime(&t_ms, c.e0, c.e3);
+  if (timed_from_e0) cudaEventElapsedTime(&t_ms, c.e0, reports ? c.e2 : c.e3);
+  else t_ms = k_ms;
   c.last.kernel_ms = k_ms;
   c.last.total_ms = t_ms;
   const gb::TraceCounters* tc = reinterpret_cast<const gb::TraceCounters*>(c.hscratch + 2);

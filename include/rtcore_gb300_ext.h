@@ -30,7 +30,7 @@ typedef struct RTCGBBuildStats {
 
 typedef struct RTCGBQueryStats {
   double kernel_ms;              /* traversal kernel time of the last query */
-  double total_ms;               /* whole call incl. host<->device copies */
+  double total_ms;               /* device time of the whole call: its copies, set-up and kernels */
   unsigned long long rays;       /* rays traversed (counting mode only) */
   unsigned long long nodes;      /* wide nodes visited (counting mode only) */
   unsigned long long tris;       /* triangle tests (counting mode only) */
