@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
   __shared__ uint2 s_stack[kSharedStack][SH::kThreads];
   // per lane: distance, u, v and triangle of its ray's nearest hit so far
   // (any hit: the distance becomes -inf at a hit); SEEDED: the triangle of the
-  // last hit found in a proposed subtree
+  // last hit found in a proposed subtree (any hit: 0 once there is one)
   __shared__ float s_t[SH::kThreads], s_u[ANYHIT ? 1 : SH::kThreads], s_v[ANYHIT ? 1 : SH::kThreads];
   __shared__ uint32_t s_tri[SH::kThreads], s_seed[SEEDED ? SH::kThreads : 1];
   // per lane: ray direction and tnear, which only triangle tests read
@@ -541,9 +541,12 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
       }
     }
     if (ANYHIT) {
+      // Lanes with hits of one ray write in no order.  All of a ray's proposed subtrees
+      // come before the rest, so its first hit is a proposal's if any of them is: a word
+      // for that, which all its writers set alike, counts as testing in place would.
       if (hit) {
         commit(w0 + own, hit_ti, A, B, C, D);
-        if (SEEDED && (e.y & 256u)) s_seed[w0 + own] = hit_ti;
+        if (SEEDED && (e.y & 256u)) s_seed[w0 + own] = 0u;
       }
       __syncwarp();
     } else {
@@ -587,7 +590,7 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
         const uint32_t hit_tri = s_tri[threadIdx.x];
         if (hit_tri != kInvalidID) {
           s_tri[threadIdx.x] = kInvalidID;
-          if (SEEDED && hit_tri == s_seed[threadIdx.x]) n_prop++;
+          if (SEEDED && (ANYHIT ? s_seed[threadIdx.x] == 0u : hit_tri == s_seed[threadIdx.x])) n_prop++;
           char* rec = P.rays + (uint64_t)rid * P.stride;
           if (ANYHIT) {
             *reinterpret_cast<float*>(rec + 32) = -INFINITY;
