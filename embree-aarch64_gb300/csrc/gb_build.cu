@@ -3307,8 +3307,6 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
   g->nseg = opt.segmented ? (uint32_t)ngeoms : 1u;
   g->nbin = 2 * N - plan.roots;
   g->maxw = N;
-  g->maxb = cdiv(N, PLOC_BLOCK);
-  g->rs_blocks = cdiv(g->total, os_tile(g->total));
   g->radius = (opt.ploc_radius == 1 || opt.ploc_radius == 2 || opt.ploc_radius == 4 || opt.ploc_radius == 8)
                   ? (uint32_t)opt.ploc_radius
                   : (uint32_t)PLOC_R_MAX;
@@ -3348,8 +3346,7 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
       (e = alloc(&g->chi[0], N)) || (e = alloc(&g->chi[1], N)) || (e = alloc(&g->cidx[0], N)) ||
       (e = alloc(&g->cidx[1], N)) || (e = alloc(&g->nn, N)) || (e = alloc(&g->bsurv, cdiv(N, 32))) ||
       (e = alloc(&g->bmerge, cdiv(N, 32))) ||
-      (e = alloc(&g->scan_sums, 2 * (size_t)scan_scratch(std::max(g->maxb, maxw)))) ||
-      (e = alloc(&g->d_tot, 4)) || (e = alloc(&g->d_root, g->nseg)) || (e = alloc(&g->d_iters, 1)) ||
+      (e = alloc(&g->d_root, g->nseg)) || (e = alloc(&g->d_iters, 1)) ||
       (e = alloc(&g->ploc_state, kPlocStateWords)) || (e = alloc(&g->cost, 2 * (size_t)(2 * N))) ||
       (e = alloc(&g->link, 2 * (size_t)N)) || (e = alloc(&g->nodes, maxw)) || (e = alloc(&g->tris, N)) ||
       (e = alloc(&g->items[0], maxw)) || (e = alloc(&g->items[1], maxw)) || (e = alloc(&g->kids, 8 * (size_t)maxw)) ||
@@ -3365,9 +3362,6 @@ cudaError_t graph_build_prepare(const GeomDesc* h_geoms, int ngeoms, const Build
   }
   g->acc = acc;
   e = cudaMemcpy(g->d_geoms, h_geoms, sizeof(GeomDesc) * ngeoms, cudaMemcpyHostToDevice);
-  // the scans' look-back state starts at zero and every scan leaves it so
-  if (e == cudaSuccess)
-    e = cudaMemset(g->scan_sums, 0, sizeof(uint32_t) * 2 * scan_scratch(std::max(g->maxb, maxw)));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_os_scatter<uint64_t, RS_ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)os_scatter_smem<uint64_t, RS_ITEMS>());

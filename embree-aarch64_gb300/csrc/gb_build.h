@@ -67,7 +67,7 @@ struct GraphBuild {
   GraphBuildPlan plan;
   BuildOptions opt;
   int ngeoms = 0;
-  uint32_t total = 0, nseg = 1, nbin = 0, maxw = 0, maxb = 0, rs_blocks = 0, radius = 1;
+  uint32_t total = 0, nseg = 1, nbin = 0, maxw = 0, radius = 1;
   std::vector<void*> allocs;  // every device allocation (released by graph_build_release)
   GeomDesc* d_geoms = nullptr;
   float4* pbox = nullptr;     // primitive boxes, two words each
@@ -76,7 +76,7 @@ struct GraphBuild {
   uint32_t *vals_a = nullptr, *vals_b = nullptr, *hist = nullptr;
   float4 *bnbox = nullptr, *clo[2] = {nullptr, nullptr}, *chi[2] = {nullptr, nullptr};
   uint32_t *bncnt = nullptr, *cidx[2] = {nullptr, nullptr}, *nn = nullptr, *bsurv = nullptr, *bmerge = nullptr;
-  uint32_t *scan_sums = nullptr, *d_tot = nullptr, *d_root = nullptr, *d_iters = nullptr, *ploc_state = nullptr;
+  uint32_t *d_root = nullptr, *d_iters = nullptr, *ploc_state = nullptr;
   float4* cost = nullptr;
   uint4* link = nullptr;
   WideNode* nodes = nullptr;
