@@ -842,14 +842,25 @@ __global__ void __launch_bounds__(SH::kThreads, min_ctas<ANYHIT, COUNT, ROBUST, 
       atomicAdd(&P.counters->rays, n_rays);
     }
   }
+  // The CTA that ends last reports the state and zeroes it.  A CTA's ticket releases what
+  // its threads added to the state; only the last one acquires, and its lanes take one
+  // word each.  (Two full fences in every CTA and ten exchanges one after the other made
+  // queries of 20k to 300k rays 3 to 9 us longer: 150k shadow rays on a 36k / 300k soup
+  // 80 / 195 us of kernel time so, 75 / 188 now.)
   if (P.done) {
     __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      if (atomicAdd(P.done, 1u) == gridDim.x - 1) {
-        __threadfence();
-        for (int i = 0; i < kStateWords; i++) P.host_state[i] = atomicExch(P.ray_counter + i, 0u);
-        *P.done = 0u;
+    if (warp == 0) {
+      uint32_t last = 0;
+      if (lane == 0) {
+        uint32_t ticket;
+        asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(P.done) : "memory");
+        last = ticket == gridDim.x - 1 ? 1u : 0u;
+        if (last) __threadfence();
+      }
+      if (__shfl_sync(0xFFFFFFFFu, last, 0)) {
+        __syncwarp();
+        if (lane < kStateWords) P.host_state[lane] = atomicExch(P.ray_counter + lane, 0u);
+        if (lane == 0) *P.done = 0u;
       }
     }
   }
