@@ -4,14 +4,16 @@
 // kernels/builders/bvh_builder_sah.h:222-319) with a GPU pipeline:
 //   1. primrefs: per-triangle validity + AABB, scene and centroid bounds
 //      (validity rule of kernels/common/scene_triangle_mesh.h:127-147)
-//   2. 63-bit Morton codes of the centroids (21 bits per axis)
+//   2. Morton codes of the centroids, 30 bits (10 per axis) or 63
 //   3. stable LSD radix sort of (code, primref index), 8-bit digits; passes
 //      whose digit is constant over all keys are skipped.  Stable sorting by
 //      key with the index as value gives exactly std::stable_sort's order.
 //   4. PLOC agglomerative clustering (nearest neighbour by merged-box surface
-//      area within a window of +-16 clusters, mutual pairs merge) -> binary tree
-//   5. top-down collapse into 8-wide nodes (largest-area child opened first),
-//      child boxes quantised to 8 bits per plane, children placed in slots
+//      area among the clusters on either side, mutual pairs merge; with
+//      gpu.ploc_radius within up to +-16) -> binary tree
+//   5. top-down collapse into 8-wide nodes of the least surface-area cost for that
+//      binary tree (gpu.collapse=greedy: largest-area child opened first), child
+//      boxes quantised to 8 bits per plane, children placed in slots
 //      so that the ray's direction octant gives a near-to-far visiting order,
 //      leaves of <= 4 triangles written as v0/e1/e2 records.
 // Everything is deterministic: the same input gives the same bytes.
@@ -342,7 +344,7 @@ cudaError_t copy_device(void* dst, const void* src, size_t bytes, cudaStream_t s
 //
 // One pass over the keys counts every digit (8 bits each) at once; its last CTA
 // turns the counts into each digit's bucket bases.  Then one scatter kernel per
-// digit pass: CTAs take 4096-key tiles in ticket order, publish their digit counts
+// digit pass: CTAs take tiles of 1,024 or 4,096 keys in ticket order, publish their digit counts
 // and find the counts of all tiles before them by decoupled look-back (Merrill &
 // Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016), rank
 // their keys stably and scatter them.  No scan kernels and no host reads.  The
@@ -445,8 +447,8 @@ __global__ void __launch_bounds__(256) k_os_hist(const K* __restrict__ keys, uin
 
 // One digit pass: tile `ticket` of kin/vin is ranked by digit (bits shift..shift+7)
 // and scattered stably to kout/vout.  status: this pass's ntiles x 256 table.
-// Warp w ranks keys base + w*512 .. +511 (16 rows of 32) by match_any into
-// per-warp digit counts; the tile's digit counts are published for the look-back;
+// Warp w ranks the keys from base + w * 32 * ITEMS on (ITEMS rows of 32) by votes
+// into per-warp digit counts; the tile's digit counts are published for the look-back;
 // the keys are placed in shared memory in (digit, original order) order and written
 // out in runs, consecutive threads to consecutive positions of a digit's bucket.
 constexpr int RS_WARPS = RS_THREADS / 32;
@@ -1360,11 +1362,11 @@ __global__ void __launch_bounds__(PLOC_BLOCK) k_ploc_all(const PlocBufs bufs, ui
   }
 }
 
-// Area of the box around clusters j and j + 1; infinite where they are no
-// neighbours (the ends, another segment).
 // The line of p into L2, for a read of the loop's next turn.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// Area of the box around clusters j and j + 1; infinite where they are no
+// neighbours (the ends, another segment).
 __device__ __forceinline__ float ploc_adjacent(const float4* clo, const float4* chi, uint32_t n, int j) {
   if (j < 0 || j + 1 >= (int)n) return INFINITY;
   const float4 a = clo[j], b = chi[j], c = clo[j + 1], d = chi[j + 1];
@@ -2842,9 +2844,6 @@ static cudaError_t onesweep_sort(K*& ka, uint32_t*& va, K*& kb, uint32_t*& vb, u
   return cudaGetLastError();
 }
 
-// Stream-ordered scratch of one build: device allocations, pinned host
-// buffers and events are released when the arena goes out of scope, on every
-// return path (free() releases a buffer early to lower the peak).
 // The one-CTA finish of the clustering, by search radius.
 static cudaError_t ploc_finish_prepare() {
   GB_CHECK(cudaFuncSetAttribute(k_ploc_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlocSmallSmem));
@@ -2866,6 +2865,9 @@ static cudaError_t ploc_finish(const PlocBufs& pb, uint32_t* ploc_state, float4*
   return cudaGetLastError();
 }
 
+// Stream-ordered scratch of one build: device allocations, pinned host
+// buffers and events are released when the arena goes out of scope, on every
+// return path (free() releases a buffer early to lower the peak).
 struct BuildArena {
   cudaStream_t st;
   std::vector<void*> dev, pinned;
@@ -3463,12 +3465,10 @@ cudaError_t graph_build_enqueue(const GraphBuild& g, cudaStream_t st) {
                          (int)g.radius, dp_cost, dp_link, leaf_max, st));
   }
   stamp(5);
-  // collapse decisions and levels
+  // all collapse levels in one cooperative launch
   BinTree bt{g.bnbox, g.bncnt, N, leaf_max, (uint32_t)(g.opt.robust != 0), dp_link};
   GB_CHECK(cudaMemsetAsync(g.leaf_root, 0xFF, sizeof(uint32_t) * N, st));
-  // collapse levels in a loop the device ends
   stamp(6);
-  // all collapse levels in one cooperative launch
   k_collapse_roots<<<1, 1024, 0, st>>>(g.d_root, g.nseg, g.nbin, g.items[0], g.seg_index, g.cstate, g.d_sah, g.d_leaves,
                                        reinterpret_cast<GridBarrier*>(g.col_bar));
   {

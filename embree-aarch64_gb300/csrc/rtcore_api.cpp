@@ -715,7 +715,8 @@ struct Scene : RefCounted {
         return;
       }
     }
-    // estimated device bytes of the build (scratch + result)
+    // estimated device bytes of the build: scratch and result, or the result and what a
+    // refitted scene keeps of its refits (32 B a triangle, 24 B a node)
     device->memory((ssize_t)(total * 256 + 4096), false);
     gb::free_bvh(&bvh);
     gb::refit_release(&refit);
